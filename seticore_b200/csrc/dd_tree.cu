@@ -30,7 +30,7 @@
 // offset whose last channel leaves [0, N) (dedoppler.cu:40-46), which for negative
 // drift blocks near the low edge skips every offset.  Lanes whose whole strip is
 // eligible run the generated code; edge strips run it too but fold only their fully eligible
-// channels, and sum the paths of the few partially eligible ones one by one (edge_strip).
+// channels, and sum the paths of the few partially eligible ones with the lanes of the warp (edge_unit).
 //
 // The element type E of the input is float (the plain form) or a 16-bit type (the
 // precision form's normalised spectra, converted to float as they are staged); sums are
@@ -242,68 +242,65 @@ __device__ __forceinline__ void strip_part(int part, const Row (&row)[R], float*
   }
 }
 
-// A strip at the band's edges (not every path of every channel eligible; dedoppler.cu:40-46:
-// path (db, off) counts for channel c iff c + e >= 0 and c + e + off < N, e = (Tr-1)*db).
-// Channels whose offsets [lo, hi) are all eligible take the generated code with a range fold
-// (its other channels read staged zeros or neighbours and are not folded); the few channels
-// with some offsets eligible (fewer than hi - lo) sum those paths one by one in the tree's
-// pairing; channels with none are skipped.  Out of line, so that its second instance of the
-// generated code and its per-path loop do not raise the register needs of the interior path:
-// the staged rows are rebuilt from the lane's tile address and the rows' window offsets.
-template <int R, int PART, int U, int ITERS, int RELOAD>
-__device__ __noinline__ void edge_strip(int part, int lo, int hi, unsigned tbase, const int* win, int ks,
-                                        float* mrow, long long cs, long long e, long long base_off, long long N) {
-  constexpr int S = U * ITERS;
+// The sum of one path of R staged rows, in the tree's pairing: row(t) is the row's shared address
+// at the path's start channel.
+template <int R, typename Row, typename RowAt>
+__device__ __forceinline__ float staged_path_sum(int off, RowAt row_at) {
   constexpr int LEVELS = (R >= 32) ? 5 : (R >= 16) ? 4 : (R >= 8) ? 3 : (R >= 4) ? 2 : 1;
   static_assert((1 << LEVELS) == R, "rows are a power of two");
-  SharedRow row[R];
+  float v[R];
 #pragma unroll
-  for (int t = 0; t < R; ++t) row[t].a = tbase + 4u * (unsigned)(win[t] + ks * t);
-  // channel c: all offsets eligible iff -e <= c <= N - 1 - e - base_off - (hi - 1)
-  const long long first = -e - cs;
-  const long long last_all = N - 1 - e - base_off - (hi - 1) - cs;
-  const int f_lo = (int)max(0ll, first), f_hi = (int)min((long long)S - 1, last_all);
-  if (f_lo <= f_hi) strip_part<R, PART, U, ITERS, RELOAD>(part, row, mrow, FoldRange{f_lo, f_hi});
-  // partially eligible: offsets [lo, lim) with lim = N - c - e - base_off in (lo, hi)
-  const long long p_lo = max(max(0ll, first), last_all + 1);
-  const long long p_hi = min((long long)S - 1, N - 1 - e - base_off - lo - cs);
-  for (long long s = p_lo; s <= p_hi; ++s) {
-    if (cs + s >= N) break;
-    const long long lim = N - (cs + s) - e - base_off;
-    const int rhi = (int)min((long long)hi, lim);
-    for (int r = lo; r < rhi; ++r) {
-      const float v = path_sum_pow2(LEVELS, r, [&](int t, int pos) { return row[t][(int)s + pos]; });
-      fold_max(mrow + s, fmaxf(v, 0.0f));
-    }
+  for (int t = 0; t < R; ++t) {
+    // path_pos(off, R, t), unrolled: the bits of t are constants here
+    int pos = 0;
+#pragma unroll
+    for (int m = 0; m < LEVELS; ++m)
+      if (t & (1 << m)) pos += ((off >> (LEVELS - 1 - m)) + 1) >> 1;
+    v[t] = Row{row_at(t)}[pos];
   }
+#pragma unroll
+  for (int h = 1; h < R; h *= 2)
+#pragma unroll
+    for (int t = 0; t + h < R; t += 2 * h) v[t] = v[t] + v[t + h];
+  return v[0];
 }
 
-// The same for one drift block of a paired-FP16 tile (H: its half), in float arithmetic from
-// the FP16 leaves: the edge strips of the 16-bit forms' paired tree.  Its error is within the
-// paired tree's bound (the float sums of FP16 leaves are closer to the exact sums).
-template <int R, int PART, int U, int ITERS, int RELOAD, int H>
-__device__ __noinline__ void edge_strip_half(int part, int lo, int hi, unsigned tbase, const int* win, int ks,
-                                             float* mrow, long long cs, long long e, long long base_off, long long N) {
+// A warp's unit at the band's edges (some lane's strip has paths that leave [0, N);
+// dedoppler.cu:40-46: path (db, off) counts for channel c iff c + e >= 0 and c + e + off < N,
+// e = (Tr-1)*db).  Channels whose offsets [lo, hi) are all eligible take the generated code with
+// a range fold (its other channels read staged zeros or neighbours and are not folded).  The
+// fewer than hi - lo channels with some offsets eligible lie side by side in the tile, and the
+// warp's lanes share their paths, one path sum at a time each: one lane alone needed 16-row
+// sums for up to 120 paths, which whole rounds of CTAs waited for (16 rows, 54 drift blocks:
+// 32768 channels 45 -> 27 us, 2^20 channels 258 -> 244 us, eight of them 1887 -> 1785 us).  Channels with no eligible path are skipped.  Out of line, so that its second
+// instance of the generated code does not raise the register needs of the interior path.
+// tbase: the tile's shared address; Row: the staged element (float, or one half of a pair).
+template <typename Row, int R, int PART, int U, int ITERS, int RELOAD>
+__device__ __noinline__ void edge_unit(int part, int lo, int hi, unsigned tbase, const int* win, int ks, float* top,
+                                       long long x0, long long e, long long base_off, long long N) {
   constexpr int S = U * ITERS;
-  constexpr int LEVELS = (R >= 32) ? 5 : (R >= 16) ? 4 : (R >= 8) ? 3 : (R >= 4) ? 2 : 1;
-  static_assert((1 << LEVELS) == R, "rows are a power of two");
-  SharedRowHalf<H> row[R];
+  const int lane = threadIdx.x & 31;
+  // all offsets of channel c eligible iff first <= c <= last_all
+  const long long first = -e;
+  const long long last_all = N - 1 - e - base_off - (hi - 1);
+  const long long cs = x0 + (long long)lane * S;
+  const int f_lo = (int)min(max(0ll, first - cs), (long long)S), f_hi = (int)max(min((long long)S - 1, last_all - cs), -1ll);
+  if (f_lo <= f_hi) {
+    Row row[R];
 #pragma unroll
-  for (int t = 0; t < R; ++t) row[t].a = tbase + 4u * (unsigned)(win[t] + ks * t);
-  const long long first = -e - cs;
-  const long long last_all = N - 1 - e - base_off - (hi - 1) - cs;
-  const int f_lo = (int)max(0ll, first), f_hi = (int)min((long long)S - 1, last_all);
-  if (f_lo <= f_hi) strip_part<R, PART, U, ITERS, RELOAD>(part, row, mrow, FoldRange{f_lo, f_hi});
-  const long long p_lo = max(max(0ll, first), last_all + 1);
-  const long long p_hi = min((long long)S - 1, N - 1 - e - base_off - lo - cs);
-  for (long long s = p_lo; s <= p_hi; ++s) {
-    if (cs + s >= N) break;
-    const long long lim = N - (cs + s) - e - base_off;
-    const int rhi = (int)min((long long)hi, lim);
-    for (int r = lo; r < rhi; ++r) {
-      const float v = path_sum_pow2(LEVELS, r, [&](int t, int pos) { return row[t][(int)s + pos]; });
-      fold_max(mrow + s, fmaxf(v, 0.0f));
-    }
+    for (int t = 0; t < R; ++t) row[t].a = tbase + 4u * (unsigned)(lane * S + win[t] + ks * t);
+    strip_part<R, PART, U, ITERS, RELOAD>(part, row, top + lane * S, FoldRange{f_lo, f_hi});
+  }
+  // partially eligible: offsets [lo, lim) with lim = N - c - e - base_off in (lo, hi)
+  const long long p_lo = max(max(x0, first), last_all + 1);
+  const long long p_hi = min(min(x0 + kWarp * S - 1, N - 1), N - 1 - e - base_off - lo);
+  const int n = p_hi >= p_lo ? (int)(p_hi - p_lo + 1) * PART : 0;
+  for (int i = lane; i < n; i += kWarp) {
+    const int c = (int)(p_lo - x0) + i / PART;  // channel of the tile
+    const int r = lo + i % PART;
+    if (x0 + c + e + base_off + r >= N) continue;
+    const float v = staged_path_sum<R, Row>(r, [&](int t) { return tbase + 4u * (unsigned)(c + win[t] + ks * t); });
+    fold_max(top + c, fmaxf(v, 0.0f));
   }
 }
 
@@ -645,7 +642,8 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
     if constexpr (PAIR) {
       // Units of two drift blocks (k, k + 1) and an offset part, part-major; an odd chunk's
       // last pair folds only its first drift block.
-      const unsigned tb0 = static_cast<unsigned>(__cvta_generic_to_shared(tile)) + 4u * (unsigned)(lane * S);
+      const unsigned tile_a = static_cast<unsigned>(__cvta_generic_to_shared(tile));
+      const unsigned tb0 = tile_a + 4u * (unsigned)(lane * S);
       const int np = (nj + 1) / 2;
       for (int u = warp; u < np * NPARTS; u += nwarps) {
         const int part = u / np;
@@ -662,13 +660,16 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
         const long long b1 = b0 + p.off_step;
         const bool in0 = (cs + e0 >= 0) && (cs + S - 1 + e0 + b0 + hi - 1 <= p.N - 1);
         const bool in1 = !hi_ok || ((cs + e1 >= 0) && (cs + S - 1 + e1 + b1 + hi - 1 <= p.N - 1));
-        if (in0 && in1) {
+        // One lane at the edge sends the warp's whole unit down the edge path, whose float sums
+        // of the FP16 leaves are within the paired tree's bound (closer to the exact sums).
+        if (__all_sync(0xffffffffu, in0 && in1)) {
           strip_part_h2<R, PART, kU, ITERS, RELOAD>(part, row, mrow, FoldPair{hi_ok});
         } else {
           constexpr int FR = R == 16 ? 12 : 0;  // the float code's reread threshold
-          edge_strip_half<R, PART, kU, ITERS, FR, 0>(part, lo, hi, tb0, &geo_win[0][0], ks, mrow, cs, e0, b0, p.N);
+          edge_unit<SharedRowHalf<0>, R, PART, kU, ITERS, FR>(part, lo, hi, tile_a, &geo_win[0][0], ks, topS, x0, e0, b0, p.N);
           if (hi_ok)
-            edge_strip_half<R, PART, kU, ITERS, FR, 1>(part, lo, hi, tb0, &geo_win[0][0], ks, mrow, cs, e1, b1, p.N);
+            edge_unit<SharedRowHalf<1>, R, PART, kU, ITERS, FR>(part, lo, hi, tile_a, &geo_win[0][0], ks, topS, x0, e1, b1,
+                                                                p.N);
         }
       }
     }
@@ -718,12 +719,12 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
       const long long e = (long long)p.elig_T1 * (p.db_first + (long long)(k0 + k) * p.db_step);
       const long long base_off = p.off_base + (long long)(k0 + k) * p.off_step;
       const bool interior = (cs + e >= 0) && (cs + S - 1 + e + base_off + hi - 1 <= p.N - 1);
-      if (interior) {
+      if (__all_sync(0xffffffffu, interior)) {
         strip_part<R, PART, kU, ITERS, RELOAD>(part, row, mrow, FoldAll{});
       } else {
-        edge_strip<R, PART, kU, ITERS, RELOAD>(
-            part, lo, hi, static_cast<unsigned>(__cvta_generic_to_shared(tile)) + 4u * (unsigned)(lane * S),
-            &geo_win[g][0], ks, mrow, cs, e, base_off, p.N);
+        edge_unit<SharedRow, R, PART, kU, ITERS, RELOAD>(part, lo, hi,
+                                                         static_cast<unsigned>(__cvta_generic_to_shared(tile)),
+                                                         &geo_win[g][0], ks, topS, x0, e, base_off, p.N);
       }
     }
 
@@ -767,44 +768,124 @@ cudaError_t launch_tree(TreeBatch& b, int num_sms, size_t smem_budget, cudaStrea
   if ((err = cudaFuncGetAttributes(&fa, kern)) != cudaSuccess) return err;
   const int max_dyn = optin - (int)fa.sharedSizeBytes;  // static + dynamic must fit the opt-in limit
   if (smem_budget > (size_t)max_dyn) smem_budget = (size_t)max_dyn;
+  // The attribute is raised to the device's opt-in maximum, the same value from every
+  // caller: host threads launching with different budgets cannot lower it under each other.
+  err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn);
+  if (err != cudaSuccess) return err;
   size_t smem = 0;
   int max_warps = 1;
   long long n_items = 0;
+  // Lays the groups' items out in order, group k in chunks of jobs_per_chunk jobs.
+  auto lay_out = [&]() {
+    smem = 0;
+    max_warps = 1;
+    n_items = 0;
+    for (int k = 0; k < b.count; ++k) {
+      TreeGroup& p = b.g[k];
+      const bool shared_rows = (p.job_row_stride == 0);
+      const int jpc = p.jobs_per_chunk;
+      p.n_chunks = (p.n_jobs + jpc - 1) / jpc;
+      const long long x_end = p.x_end > 0 ? p.x_end : (p.x_end < 0 ? p.x_begin : p.N);
+      p.tile_first = p.x_begin / W;
+      p.n_tiles = (int)std::max<long long>(0, (x_end + W - 1) / W - p.tile_first);
+      p.item_begin = (int)n_items;
+      n_items += (long long)p.n_tiles * p.n_chunks;
+      const size_t sm = tree_smem_bytes<E, R, NPARTS, S, EMIT, MAXW>(jpc, p.d_step, shared_rows);
+      if (sm > smem) smem = sm;
+      const int w = (PAIR ? (jpc + 1) / 2 : jpc) * NPARTS;  // warp units of a chunk
+      if (w > max_warps) max_warps = w;
+    }
+  };
   for (int k = 0; k < b.count; ++k) {
     TreeGroup& p = b.g[k];
+    if (p.x_begin < 0 || p.x_begin % W != 0) return cudaErrorInvalidValue;
     const bool shared_rows = (p.job_row_stride == 0);
     // Largest chunk of jobs whose staged windows fit the shared-memory budget.
     int jpc = shared_rows ? p.n_jobs : (p.n_jobs < kMaxSeg ? p.n_jobs : kMaxSeg);
     while (jpc > 1 && tree_smem_bytes<E, R, NPARTS, S, EMIT, MAXW>(jpc, p.d_step, shared_rows) > smem_budget)
       jpc = shared_rows ? (jpc + 1) / 2 : jpc - 1;
     p.jobs_per_chunk = jpc;
-    p.n_chunks = (p.n_jobs + jpc - 1) / jpc;
-    const long long x_end = p.x_end > 0 ? p.x_end : (p.x_end < 0 ? p.x_begin : p.N);
-    if (p.x_begin < 0 || p.x_begin % W != 0) return cudaErrorInvalidValue;
-    p.tile_first = p.x_begin / W;
-    p.n_tiles = (int)std::max<long long>(0, (x_end + W - 1) / W - p.tile_first);
-    p.item_begin = (int)n_items;
-    n_items += (long long)p.n_tiles * p.n_chunks;
-    const size_t sm = tree_smem_bytes<E, R, NPARTS, S, EMIT, MAXW>(jpc, p.d_step, shared_rows);
-    if (sm > smem) smem = sm;
-    const int w = (PAIR ? (jpc + 1) / 2 : jpc) * NPARTS;  // warp units of a chunk
-    if (w > max_warps) max_warps = w;
+  }
+  lay_out();
+  if (smem > (size_t)max_dyn) return cudaErrorInvalidValue;  // one job alone does not fit
+  // CTAs that run at once, with the largest chunks.
+  auto resident = [&]() {
+    const int warps = max_warps > MAXW ? MAXW : max_warps;
+    int per_sm = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * kWarp, smem) != cudaSuccess || per_sm < 1)
+      per_sm = 1;
+    return (long long)per_sm * num_sms;
+  };
+  long long slots = resident();
+  // The items that do not fill a whole round of resident CTAs -- all of them for a small search,
+  // the last round of a larger one -- are cut into smaller chunks of jobs, so that the idle SMs
+  // share their drift blocks.  A chunk's time is its staging, about 0.4 of a 16-row unit's strip
+  // (kStage, in strips of this row count), and one strip per round of its units over the CTA's
+  // warps; the cut with the smallest estimate is taken.  16 rows, 54 drift blocks: 32768
+  // channels (32 tiles) 148 -> 45 us, 2^20 channels (993 tiles on 296 slots) 324 -> 258 us;
+  // beyond a dozen rounds the last one is small change and whole chunks stage least (8 searches
+  // of 2^20 channels, 27 rounds: 1887 us either way).
+  if constexpr (!EMIT) {
+    bool shared = n_items > 0 && n_items < 12 * slots;
+    for (int k = 0; k < b.count; ++k) shared = shared && b.g[k].job_row_stride == 0;
+    if (shared) {
+      constexpr int kLevels = R >= 32 ? 5 : R >= 16 ? 4 : R >= 8 ? 3 : R >= 4 ? 2 : 1;
+      constexpr double kStage = 0.4 * 64.0 / (R * kLevels / NPARTS);
+      const long long rem = n_items % slots;
+      // Tail groups: whole groups inside the last round, and the split rest of the one that
+      // reaches into it.
+      int first_tail = b.count;
+      long long left = rem;
+      while (left > 0 && first_tail > 0) {
+        TreeGroup& p = b.g[first_tail - 1];
+        const long long items = (long long)p.n_tiles * p.n_chunks;
+        if (items <= left) {
+          left -= items;
+          --first_tail;
+          continue;
+        }
+        const int tiles = (int)(left / p.n_chunks);  // its last tiles lie in the last round
+        if (tiles > 0 && b.count < kMaxBatch) {
+          for (int k = b.count; k > first_tail; --k) b.g[k] = b.g[k - 1];
+          ++b.count;
+          TreeGroup& q = b.g[first_tail];
+          q = b.g[first_tail - 1];
+          const int cut = (p.tile_first + p.n_tiles - tiles) * W;
+          b.g[first_tail - 1].x_end = cut;
+          q.x_begin = cut;
+          if (q.x_end == 0) q.x_end = q.N;
+          q.n_tiles = tiles;
+        }
+        left = 0;
+      }
+      int best = 0, max_jobs = 0;
+      double best_time = 0.0;
+      for (int k = first_tail; k < b.count; ++k) max_jobs = std::max(max_jobs, b.g[k].jobs_per_chunk);
+      for (int j = max_jobs; j >= 1; --j) {
+        long long items = 0;
+        for (int k = first_tail; k < b.count; ++k) {
+          const int jk = std::min(j, b.g[k].jobs_per_chunk);
+          items += (long long)b.g[k].n_tiles * ((b.g[k].n_jobs + jk - 1) / jk);
+        }
+        const int units = (PAIR ? (j + 1) / 2 : j) * NPARTS;
+        const double t = (double)((items + slots - 1) / slots) * (kStage + (units + MAXW - 1) / MAXW);
+        if (best == 0 || t < best_time) {
+          best = j;
+          best_time = t;
+        }
+      }
+      for (int k = first_tail; k < b.count; ++k)
+        b.g[k].jobs_per_chunk = std::min(best, b.g[k].jobs_per_chunk);
+      lay_out();
+      slots = resident();
+    }
   }
   if (n_items == 0) return cudaSuccess;
   if (n_items > (1ll << 30)) return cudaErrorInvalidValue;
   b.n_items = (int)n_items;
   b.stage_wait_tries = stage_wait_tries();
-  // The attribute is raised to the device's opt-in maximum, the same value from every
-  // caller: host threads launching with different budgets cannot lower it under each other.
-  if (smem > (size_t)max_dyn) return cudaErrorInvalidValue;  // one job alone does not fit
-  err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn);
-  if (err != cudaSuccess) return err;
   // Enough warps for every (job, offset part) unit of a chunk, at most MAXW.
   const int warps = max_warps > MAXW ? MAXW : max_warps;
-  int per_sm = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * kWarp, smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  const long long slots = (long long)per_sm * num_sms;
   const int grid = (int)(n_items < slots ? n_items : slots);
   kern<<<grid, warps * kWarp, smem, stream>>>(b);
   return cudaGetLastError();
