@@ -9,8 +9,8 @@
 //   column sums (dd_tree.cu; for Tr > 32 the level path of dd_levels.cu, one search at a
 //   time) -> order statistics + variance (dd_stats.cu) -> window de-duplication + drift
 //   recovery (dd_hits.cu)
-// then copies the headers and the first candidates of every search to pinned host memory
-// in two copies and synchronises once.  Only hit lists cross to the host, not the
+// whose last kernel leaves the header and the first candidates of each search in pinned host
+// memory, and synchronises once.  Only hit lists cross to the host, not the
 // reference's four N-length arrays per search.
 #include <algorithm>
 #include <climits>
@@ -112,6 +112,7 @@ struct sc_dd {
   scb::LevelSide side;
   int level_pairs = 1;  // pairs of level buffers in scratch_a
   void* host = nullptr;  // pinned: slots * (header + kHostCands candidates)
+  // addIncoherentPower's paths and sums, in pinned host memory that its kernel reads and writes.
   int* inc_index = nullptr;
   int* inc_steps = nullptr;
   float* inc_vals = nullptr;
@@ -233,6 +234,15 @@ int ensure_prec(sc_dd* d, int slots) {
   return SC_DD_OK;
 }
 
+void free_inc(sc_dd* d) {
+  if (d->inc_index) cudaFreeHost(d->inc_index);
+  if (d->inc_steps) cudaFreeHost(d->inc_steps);
+  if (d->inc_vals) cudaFreeHost(d->inc_vals);
+  d->inc_index = d->inc_steps = nullptr;
+  d->inc_vals = nullptr;
+  d->inc_cap = 0;
+}
+
 void free_all(sc_dd* d) {
   drop_graphs(d);
   if (d->cap_stream) cudaStreamDestroy(d->cap_stream);
@@ -249,9 +259,7 @@ void free_all(sc_dd* d) {
   }
   if (d->side.fork) cudaEventDestroy(d->side.fork);
   d->side = scb::LevelSide{};
-  dfree(d, &d->inc_index, sizeof(int) * d->inc_cap);
-  dfree(d, &d->inc_steps, sizeof(int) * d->inc_cap);
-  dfree(d, &d->inc_vals, sizeof(float) * d->inc_cap);
+  free_inc(d);
   for (cudaEvent_t& e : d->ev)
     if (e) cudaEventDestroy(e);
 }
@@ -290,16 +298,15 @@ int ensure_slots(sc_dd* d, int slots, int cand_cap) {
 
 int ensure_inc(sc_dd* d, int n) {
   if (n <= d->inc_cap) return SC_DD_OK;
-  dfree(d, &d->inc_index, sizeof(int) * d->inc_cap);
-  dfree(d, &d->inc_steps, sizeof(int) * d->inc_cap);
-  dfree(d, &d->inc_vals, sizeof(float) * d->inc_cap);
-  d->inc_cap = 0;
+  free_inc(d);
   const int cap = std::max(n, 4096);
   cudaError_t e;
-  if ((e = dalloc(d, &d->inc_index, sizeof(int) * cap)) != cudaSuccess ||
-      (e = dalloc(d, &d->inc_steps, sizeof(int) * cap)) != cudaSuccess ||
-      (e = dalloc(d, &d->inc_vals, sizeof(float) * cap)) != cudaSuccess)
+  if ((e = cudaMallocHost(&d->inc_index, sizeof(int) * cap)) != cudaSuccess ||
+      (e = cudaMallocHost(&d->inc_steps, sizeof(int) * cap)) != cudaSuccess ||
+      (e = cudaMallocHost(&d->inc_vals, sizeof(float) * cap)) != cudaSuccess) {
+    free_inc(d);
     return cuda_fail(e, "incoherent staging allocation");
+  }
   d->inc_cap = cap;
   return SC_DD_OK;
 }
@@ -347,7 +354,12 @@ int queue_batch(sc_dd* dd, int n, const float* const* inputs, const long long* s
       q.flag_count = dd->flag_counts + k;
       q.norm_moments = dd->norm_moments + (size_t)scb::kNormMomentsDoubles * k;
       q.norm_ticket = dd->norm_tickets + k;
+      q.report.flag_out = dd->host_flag_counts + k;
+      q.report.norm_out = k == 0 && first_batch ? dd->host_norm : nullptr;
     }
+    q.report.hdr = dd->host_hdrs() + k;
+    q.report.cands = dd->host_cands() + (size_t)kHostCands * k;
+    q.report.head = std::min(kHostCands, dd->cand_cap);
   }
   EventHooks eh{dd, first_batch};
   scb::ExecHooks hooks;
@@ -457,21 +469,10 @@ int run_searches(sc_dd* dd, int count, const float* const* inputs, const long lo
     rc = queue_batch_graphed(dd, n, inputs + k0, strides + k0, p, snr_threshold, stream, k0 == 0);
     if (rc != SC_DD_OK) return rc;
     if (k0 == 0) cudaEventRecord(dd->ev[3], stream);
-    // Headers of all n searches, then the first kHostCands candidates of each (strided copy).
+    // The last kernel of each search has left its header and first candidates in pinned memory.
     const int head = std::min(kHostCands, dd->cand_cap);
-    if ((e = cudaMemcpyAsync(dd->host_hdrs(), dd->hdrs, sizeof(scb::SearchHeader) * n, cudaMemcpyDeviceToHost,
-                             stream)) != cudaSuccess ||
-        (e = cudaMemcpy2DAsync(dd->host_cands(), sizeof(scb::Candidate) * kHostCands, dd->cands,
-                               sizeof(scb::Candidate) * dd->cand_cap, sizeof(scb::Candidate) * head, n,
-                               cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
-        (prec && (e = cudaMemcpyAsync(dd->host_flag_counts, dd->flag_counts, sizeof(int) * n, cudaMemcpyDeviceToHost,
-                                      stream)) != cudaSuccess) ||
-        (prec && k0 == 0 &&
-         (e = cudaMemcpyAsync(dd->host_norm, dd->norm_moments + 2 * scb::kVarChunks, sizeof(double) * 2,
-                              cudaMemcpyDeviceToHost, stream)) != cudaSuccess) ||
-        (e = cudaStreamSynchronize(stream)) != cudaSuccess)
-      return cuda_fail(e, "result copy");
-    d2h += (long long)(sizeof(scb::SearchHeader) + sizeof(scb::Candidate) * head) * n +
+    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_fail(e, "search");
+    d2h += (long long)sizeof(scb::SearchHeader) * n +
            (prec ? (long long)sizeof(int) * n + (k0 == 0 ? 2 * (long long)sizeof(double) : 0) : 0);
     for (int k = 0; k < n; ++k) {
       const scb::SearchHeader h = dd->host_hdrs()[k];
@@ -480,6 +481,7 @@ int run_searches(sc_dd* dd, int count, const float* const* inputs, const long lo
       std::vector<scb::Candidate> cands(ncand);
       const scb::Candidate* hc = dd->host_cands() + (size_t)kHostCands * k;
       std::copy(hc, hc + std::min(ncand, head), cands.begin());
+      d2h += (long long)sizeof(scb::Candidate) * std::min(ncand, head);
       if (ncand > head) {
         if ((e = cudaMemcpyAsync(cands.data() + head, dd->cands + (size_t)dd->cand_cap * k + head,
                                  sizeof(scb::Candidate) * (ncand - head), cudaMemcpyDeviceToHost, stream)) !=
@@ -695,21 +697,18 @@ int sc_dd_add_incoherent_power(sc_dd* dd, const float* dev_input, long long row_
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   int rc = ensure_inc(dd, num_hits);
   if (rc != SC_DD_OK) return rc;
-  std::vector<int> idx(num_hits), steps(num_hits);
-  std::vector<float> vals(num_hits);
+  // A few hundred paths at most: the kernel reads them and writes their sums over PCIe, which
+  // leaves one launch where three copies stood beside it.
   for (int i = 0; i < num_hits; ++i) {
-    idx[i] = hits[i].index;
-    steps[i] = hits[i].drift_steps;
+    dd->inc_index[i] = hits[i].index;
+    dd->inc_steps[i] = hits[i].drift_steps;
   }
   cudaError_t e;
-  if ((e = cudaMemcpyAsync(dd->inc_index, idx.data(), sizeof(int) * num_hits, cudaMemcpyHostToDevice, stream)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(dd->inc_steps, steps.data(), sizeof(int) * num_hits, cudaMemcpyHostToDevice, stream)) != cudaSuccess ||
-      (e = scb::path_values(dev_input, row_stride, dd->Tr, dd->N, dd->inc_index, dd->inc_steps, dd->inc_vals,
+  if ((e = scb::path_values(dev_input, row_stride, dd->Tr, dd->N, dd->inc_index, dd->inc_steps, dd->inc_vals,
                             num_hits, stream)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(vals.data(), dd->inc_vals, sizeof(float) * num_hits, cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
       (e = cudaStreamSynchronize(stream)) != cudaSuccess)
     return cuda_fail(e, "sc_dd_add_incoherent_power");
-  for (int i = 0; i < num_hits; ++i) hits[i].incoherent_power = vals[i];
+  for (int i = 0; i < num_hits; ++i) hits[i].incoherent_power = dd->inc_vals[i];
   return SC_DD_OK;
 }
 

@@ -80,6 +80,29 @@ __device__ __forceinline__ float path_sum_pow2(int n, int off, Get get) {
   return stack[0];
 }
 
+// The same sum with its rows taken sixteen at a time: a block of 16 rows has the sub-offset
+// off >> (n - 4), its channel offsets are sums of four shifts, and its 16 values are loaded
+// before any is added, so one path's loads overlap instead of each waiting for the last
+// (drift recovery of 192 candidates of 512 paths of 256 rows: 136 -> 36 us; the 16-bit forms'
+// recomputation of 16 beams' listed channels: 235 -> 55 us).
+template <typename Get>
+__device__ __forceinline__ float path_sum_by16(int n, int off, Get get) {
+  if (n < 4) return path_sum_pow2(n, off, get);
+  const int o = off >> (n - 4);
+  const int s0 = ((o >> 3) + 1) >> 1, s1 = ((o >> 2) + 1) >> 1, s2 = ((o >> 1) + 1) >> 1, s3 = (o + 1) >> 1;
+  return path_sum_pow2(n - 4, off, [&](int b, int p) {
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      v[j] = get(16 * b + j, p + ((j & 1) ? s0 : 0) + ((j & 2) ? s1 : 0) + ((j & 4) ? s2 : 0) + ((j & 8) ? s3 : 0));
+#pragma unroll
+    for (int h = 1; h < 16; h *= 2)
+#pragma unroll
+      for (int j = 0; j < 16; j += 2 * h) v[j] = v[j] + v[j + h];
+    return v[0];
+  });
+}
+
 // Float -> unsigned key with the same order as the float values (non-NaN).
 __device__ __forceinline__ uint32_t float_key(float f) {
   const uint32_t u = __float_as_uint(f);

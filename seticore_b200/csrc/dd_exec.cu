@@ -60,6 +60,9 @@ SearchDesc to_desc(const ExecSearch& e) {
   s.hdr = e.hdr;
   s.cands = e.cands;
   s.cand_cap = e.cand_cap;
+  s.report = e.report;
+  s.report.flag_count = e.flag_count;
+  s.report.norm = e.norm_moments ? e.norm_moments + 2 * kVarChunks : nullptr;
   return s;
 }
 

@@ -4,7 +4,7 @@
 //   are cut into non-overlapping windows of window_size; a window's candidate is the
 //   first channel holding its largest top sum, if that sum is strictly above the
 //   threshold; it survives if no channel in [c - window_size + 1, c + window_size) has a
-//   strictly larger top sum.  One warp per window.
+//   strictly larger top sum.  One warp or block per window.
 // resolve_kernel: recovers the drift of each survivor.  The reference keeps, per channel,
 //   the first (drift block, offset) in scan order whose sum beat the running maximum
 //   (dedoppler.cu:49-53); that is the first eligible path, in (drift block, offset)
@@ -24,48 +24,137 @@ namespace scb {
 
 namespace {
 
-__global__ void window_kernel(const __grid_constant__ SearchBatch b) {
+// The first channel of [start, end) with the largest value above `best`, over GROUP threads
+// (a warp or the block), each of which holds its own first best on return.  Eight loads in
+// flight per thread: a window's time is its loads' latency.
+template <int GROUP>
+__device__ __forceinline__ void window_best(const float* __restrict__ top, long long start, long long end, int t,
+                                            float& best, int& bidx) {
+  constexpr int K = 8;
+  for (long long f0 = start + t; f0 < end; f0 += GROUP * K) {
+    float v[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = f0 + GROUP * k < end ? top[f0 + GROUP * k] : 0.0f;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (f0 + GROUP * k < end && v[k] > best) {
+        best = v[k];
+        bidx = (int)(f0 + GROUP * k);
+      }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
+    if (oi >= 0 && (bidx < 0 || ov > best || (ov == best && oi < bidx))) {
+      best = ov;
+      bidx = oi;
+    }
+  }
+}
+
+// Whether a value above `best` lies in [lo, hi) among this thread's share.
+template <int GROUP>
+__device__ __forceinline__ bool window_larger(const float* __restrict__ top, long long lo, long long hi, int t, float best) {
+  constexpr int K = 8;
+  bool larger = false;
+  for (long long f0 = lo + t; f0 < hi && !larger; f0 += GROUP * K) {
+    float v[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = f0 + GROUP * k < hi ? top[f0 + GROUP * k] : best;
+#pragma unroll
+    for (int k = 0; k < K; ++k) larger = larger || v[k] > best;
+  }
+  return larger;
+}
+
+constexpr int kWindowThreads = 256;
+constexpr int kWarpWindow = 512;  // windows of at most this many channels take one warp each
+
+// Wider windows take a block each: there are few of them, and one warp for 2194 channels with one
+// load in flight needed 31 us on 46 windows (eight in flight: 17 us).  Narrow windows are many,
+// and a block each would leave most threads idle.
+__global__ void __launch_bounds__(kWindowThreads) window_kernel(const __grid_constant__ SearchBatch b) {
   const SearchDesc& sd = b.s[blockIdx.y];
   const float* __restrict__ top = sd.top;
   const int N = sd.N, w = sd.window_size, cap = sd.cand_cap;
   SearchHeader* hdr = sd.hdr;
   Candidate* cands = sd.cands;
   const float thr = hdr->threshold;
-  const int lane = threadIdx.x & 31;
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long nwin = ((long long)N + w - 1) / w;
-  for (long long i = gw; i < nwin; i += nw) {
-    const long long start = i * w;
-    const long long end = min((long long)N, start + w);
-    float best = thr;
-    long long bidx = -1;
-    for (long long f = start + lane; f < end; f += 32) {
-      const float v = top[f];
-      if (v > best) {
-        best = v;
-        bidx = f;
-      }
+  auto keep = [&](int idx, float best) {
+    const int slot = atomicAdd(&hdr->num_candidates, 1);
+    if (slot < cap) cands[slot] = Candidate{idx, 0, best, 0, 0ull};
+  };
+  if (w <= kWarpWindow) {
+    const long long nw = (long long)gridDim.x * (kWindowThreads / 32);
+    for (long long i = (long long)blockIdx.x * (kWindowThreads / 32) + warp; i < nwin; i += nw) {
+      float best = thr;
+      int bidx = -1;
+      window_best<32>(top, i * w, min((long long)N, (i + 1) * w), lane, best, bidx);
+      if (bidx < 0) continue;
+      const bool larger = window_larger<32>(top, max(0ll, (long long)bidx - w + 1), min((long long)N, (long long)bidx + w),
+                                            lane, best);
+      if (__any_sync(0xffffffffu, larger)) continue;
+      if (lane == 0) keep(bidx, best);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const long long oi = __shfl_xor_sync(0xffffffffu, bidx, o);
+    return;
+  }
+  __shared__ float s_best[kWindowThreads / 32];
+  __shared__ int s_idx[kWindowThreads / 32];
+  for (long long i = blockIdx.x; i < nwin; i += gridDim.x) {
+    float best = thr;
+    int bidx = -1;
+    window_best<kWindowThreads>(top, i * w, min((long long)N, (i + 1) * w), threadIdx.x, best, bidx);
+    if (lane == 0) {
+      s_best[warp] = best;
+      s_idx[warp] = bidx;
+    }
+    __syncthreads();
+    best = s_best[0];
+    bidx = s_idx[0];
+    for (int k = 1; k < kWindowThreads / 32; ++k) {
+      const float ov = s_best[k];
+      const int oi = s_idx[k];
       if (oi >= 0 && (bidx < 0 || ov > best || (ov == best && oi < bidx))) {
         best = ov;
         bidx = oi;
       }
     }
-    if (bidx < 0) continue;
-    const long long lo = max(0ll, bidx - w + 1);
-    const long long hi = min((long long)N, bidx + w);
-    bool larger = false;
-    for (long long f = lo + lane; f < hi && !larger; f += 32) larger = top[f] > best;
-    if (__any_sync(0xffffffffu, larger)) continue;
-    if (lane == 0) {
-      const int slot = atomicAdd(&hdr->num_candidates, 1);
-      if (slot < cap) cands[slot] = Candidate{(int)bidx, 0, best, 0, 0ull};
+    if (bidx < 0) {
+      __syncthreads();  // before the next window's writes
+      continue;
     }
+    const bool larger = window_larger<kWindowThreads>(top, max(0ll, (long long)bidx - w + 1),
+                                                      min((long long)N, (long long)bidx + w), threadIdx.x, best);
+    if (!__syncthreads_or(larger) && threadIdx.x == 0) keep(bidx, best);
   }
+}
+
+// The end of a search's drift recovery: the last of its CTAs to arrive writes the header and
+// the first candidates to host memory, a few hundred bytes: two copies of every search's whole
+// candidate window stood after the launches before (6 KB per search, at a large pitch).
+__device__ void report_results(const SearchDesc& sd) {
+  const HostReport& r = sd.report;
+  if (!r.hdr) return;
+  __shared__ bool last_block;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last_block = atomicAdd(&sd.hdr->ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last_block) return;
+  __threadfence();
+  const int n = min(min(sd.hdr->num_candidates, sd.cand_cap), r.head);
+  const unsigned long long* src = reinterpret_cast<const unsigned long long*>(sd.cands);
+  unsigned long long* dst = reinterpret_cast<unsigned long long*>(r.cands);
+  static_assert(sizeof(Candidate) == 24 && sizeof(SearchHeader) % 8 == 0, "records of whole 8-byte words");
+  for (int i = threadIdx.x; i < 3 * n; i += blockDim.x) dst[i] = __ldcg(src + i);
+  const unsigned long long* hs = reinterpret_cast<const unsigned long long*>(sd.hdr);
+  if (threadIdx.x < (int)(sizeof(SearchHeader) / 8))
+    reinterpret_cast<unsigned long long*>(r.hdr)[threadIdx.x] = __ldcg(hs + threadIdx.x);
+  if (threadIdx.x == 0 && r.flag_out) *r.flag_out = *r.flag_count;
+  if (threadIdx.x < 2 && r.norm_out) r.norm_out[threadIdx.x] = r.norm[threadIdx.x];
 }
 
 // One thread per (candidate, path): every eligible path of every surviving channel is
@@ -90,7 +179,7 @@ __global__ void resolve_kernel(const __grid_constant__ SearchBatch b) {
     const int off = p - (p / Tr) * Tr;
     const long long e = (long long)(Tr - 1) * db;
     if (c + e < 0 || c + e + off >= N) continue;
-    const float v = path_sum_pow2(levels, off, [&](int t, int pos) {
+    const float v = path_sum_by16(levels, off, [&](int t, int pos) {
       return __ldg(in + (long long)t * stride + c + (long long)db * t + pos);
     });
     if (v > 0.0f) {  // the reference's top sums start at zero and update on strict >
@@ -98,6 +187,7 @@ __global__ void resolve_kernel(const __grid_constant__ SearchBatch b) {
       atomicMax(&cands[i].best, key);
     }
   }
+  report_results(sd);
 }
 
 __global__ void path_values_kernel(const float* __restrict__ in, long long stride, int Tr, int N,
@@ -114,7 +204,7 @@ __global__ void path_values_kernel(const float* __restrict__ in, long long strid
     out[i] = __int_as_float(0x7fc00000);
     return;
   }
-  out[i] = path_sum_pow2(31 - __clz(Tr), off, [&](int t, int pos) {  // Tr is a power of two
+  out[i] = path_sum_by16(31 - __clz(Tr), off, [&](int t, int pos) {  // Tr is a power of two
     return __ldg(in + (long long)t * stride + c + (long long)db * t + pos);
   });
 }
@@ -159,6 +249,7 @@ __global__ void resolve_direct_kernel(const __grid_constant__ SearchBatch b) {
     }
     if (best) atomicMax(&cands[i].best, best);
   }
+  report_results(sd);
 }
 
 }  // namespace
@@ -167,14 +258,16 @@ cudaError_t search_hits_batch(const SearchBatch& b, int num_sms, cudaStream_t st
   if (b.count <= 0) return cudaSuccess;
   long long nwin = 1;
   for (int k = 0; k < b.count; ++k) {
-    const long long n = ((long long)b.s[k].N + b.s[k].window_size - 1) / b.s[k].window_size;
+    const long long w = b.s[k].window_size;
+    long long n = ((long long)b.s[k].N + w - 1) / w;
+    if (w <= kWarpWindow) n = (n + kWindowThreads / 32 - 1) / (kWindowThreads / 32);  // one window per warp
     if (n > nwin) nwin = n;
   }
-  long long wblocks = (nwin + 7) / 8;  // 8 warps per block, one window per warp
+  long long wblocks = nwin;
   const long long wcap = (8ll * num_sms + b.count - 1) / b.count;
   if (wblocks > wcap) wblocks = wcap;
   if (wblocks < 1) wblocks = 1;
-  window_kernel<<<dim3((unsigned)wblocks, b.count), 256, 0, stream>>>(b);
+  window_kernel<<<dim3((unsigned)wblocks, b.count), kWindowThreads, 0, stream>>>(b);
   int rblocks = (4 * num_sms + b.count - 1) / b.count;
   if (rblocks < 4) rblocks = 4;
   // Drift recovery, one launch per row count: the direct form up to 16 rows, one path per

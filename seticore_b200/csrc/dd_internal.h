@@ -90,6 +90,21 @@ struct SearchHeader {
   int order_exact;  // 1: the statistics were formed in the reference's nth_element order
   int ties;         // most copies of one value among the three order statistics' values
   float median, std_dev, mean, threshold;
+  unsigned ticket;  // CTAs of the drift recovery that are done (the last one writes the report)
+  int pad;
+};
+
+// Where the last kernel of a search leaves its results: host memory that the device can write
+// (pinned), so that no copy is queued after it.  Null pointers are skipped.
+struct HostReport {
+  SearchHeader* hdr;
+  Candidate* cands;       // the first `head` candidates
+  int head;
+  int pad;
+  const int* flag_count;  // 16-bit forms: listed channels, and the scale of the normalised copy
+  int* flag_out;
+  const double* norm;
+  double* norm_out;       // mean and standard deviation
 };
 
 // Everything the batched kernels need to know about one search.
@@ -111,6 +126,7 @@ struct SearchDesc {
   Candidate* cands;
   int cand_cap;
   int pad;
+  HostReport report;
 };
 
 struct SearchBatch {
@@ -385,6 +401,7 @@ struct ExecSearch {
   int* flag_count;
   double* norm_moments;
   unsigned* norm_ticket;
+  HostReport report;  // its device pointers (flag_count, norm) are filled by exec_queue
   static size_t scratch_bytes(int Tr, int N, int cand_cap, int n_partials, int elem);
   void carve(char* base, int n_partials);
 };

@@ -271,10 +271,17 @@ int ensure_device(sc_dd_pool* p, size_t arena, size_t lvl, cudaStream_t stream) 
   return SC_DD_OK;
 }
 
-// Queues one sub-batch plus the copies of its results into p->host.
+// Queues one sub-batch; its results land in p->host.
 cudaError_t queue_sub(sc_dd_pool* p, std::vector<Planned>& sub, cudaStream_t s) {
   std::vector<scb::ExecSearch> es(sub.size());
-  for (size_t k = 0; k < sub.size(); ++k) es[k] = sub[k].es;
+  char* h = p->host;
+  for (size_t k = 0; k < sub.size(); ++k) {  // the last kernel of each search writes its results there
+    es[k] = sub[k].es;
+    es[k].report.hdr = reinterpret_cast<scb::SearchHeader*>(h);
+    es[k].report.cands = reinterpret_cast<scb::Candidate*>(h + sizeof(scb::SearchHeader));
+    es[k].report.head = std::min(kHostCands, es[k].cand_cap);
+    h += sizeof(scb::SearchHeader) + sizeof(scb::Candidate) * kHostCands;
+  }
   scb::ExecHooks hooks;
   hooks.ctx = p;
   hooks.tree_launch = pool_tree_launch;
@@ -282,18 +289,7 @@ cudaError_t queue_sub(sc_dd_pool* p, std::vector<Planned>& sub, cudaStream_t s) 
   // The tuner times one level search at a time on its own stream: no side stream then.
   cudaError_t e = scb::exec_queue(es.data(), (int)es.size(), p->lvl_a, p->lvl_b, p->num_sms, s, hooks,
                                   p->tuning_now || p->side.n == 0 ? nullptr : &p->side);
-  if (e != cudaSuccess) return e;
-  char* h = p->host;
-  for (size_t k = 0; k < sub.size(); ++k) {
-    const scb::ExecSearch& q = sub[k].es;
-    const int head = std::min(kHostCands, q.cand_cap);
-    if ((e = cudaMemcpyAsync(h, q.hdr, sizeof(scb::SearchHeader), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(h + sizeof(scb::SearchHeader), q.cands, sizeof(scb::Candidate) * head,
-                             cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-      return e;
-    h += sizeof(scb::SearchHeader) + sizeof(scb::Candidate) * kHostCands;
-  }
-  return cudaSuccess;
+  return e;
 }
 
 }  // namespace

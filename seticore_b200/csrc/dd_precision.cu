@@ -525,7 +525,7 @@ __global__ void recompute_kernel(const __grid_constant__ PrecisionBatch b) {
       const long long e = (long long)(Tr - 1) * db;
       if (c + e >= 0 && c + e + off < N) {  // findTopPathSums' early return (dedoppler.cu:40-46)
         const float* base = d.input + c;
-        best = fmaxf(0.0f, path_sum_pow2(levels, off, [&](int t, int pos) {
+        best = fmaxf(0.0f, path_sum_by16(levels, off, [&](int t, int pos) {
           return __ldg(base + (long long)t * d.row_stride + (long long)db * t + pos);
         }));
       }
