@@ -92,15 +92,11 @@ struct sc_dd {
   double foff = 0, tsamp = 0;
   int has_dc_spike = 0;
   int device = 0, num_sms = 148;
-  int n_partials = 0;
   // Per-slot scratch, slot k at offset k * (per-slot size) in each array.
   int slots = 0;
   int cand_cap = 0;  // candidates per slot
   float* top = nullptr;
   float* colsum = nullptr;
-  scb::SelectState* sel = nullptr;
-  scb::MomentPartial* partials = nullptr;
-  double* var = nullptr;
   float* work = nullptr;  // [slot][order_work_floats(N)] column sums in nth_element order
   int* lists = nullptr;   // [slot][order_list_entries(N)] partition pairs
   scb::SearchHeader* hdrs = nullptr;
@@ -128,6 +124,9 @@ struct sc_dd {
   unsigned* norm_tickets = nullptr;  // [slot]
   int* host_flag_counts = nullptr;   // pinned [slot]
   double* host_norm = nullptr;       // pinned [2]: mean, std of search 0
+  // Floats per slot of the per-channel arrays: whole 256-byte lines, so that every slot takes
+  // 16-byte loads whatever N is.
+  size_t slot_floats() const { return ((size_t)N + 63) & ~size_t(63); }
   size_t device_bytes = 0;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // call start, tree start/end, call end
   sc_dd_stats last{};
@@ -179,12 +178,9 @@ void drop_graphs(sc_dd* d) {
 }
 
 void free_slots(sc_dd* d) {
-  const size_t N = d->N, S = d->slots;
+  const size_t N = d->slot_floats(), S = d->slots;
   dfree(d, &d->top, sizeof(float) * N * S);
   dfree(d, &d->colsum, sizeof(float) * N * S);
-  dfree(d, &d->sel, sizeof(scb::SelectState) * S);
-  dfree(d, &d->partials, sizeof(scb::MomentPartial) * d->n_partials * S);
-  dfree(d, &d->var, sizeof(double) * 2 * scb::kVarChunks * S);
   dfree(d, &d->work, sizeof(float) * scb::order_work_floats(d->N) * S);
   dfree(d, &d->lists, sizeof(int) * scb::order_list_entries(d->N) * S);
   dfree(d, &d->hdrs, sizeof(scb::SearchHeader) * S);
@@ -195,8 +191,8 @@ void free_slots(sc_dd* d) {
 }
 
 void free_prec(sc_dd* d) {
-  const size_t S = d->prec_slots, N = d->N;
-  dfree(d, &d->norm16, scb::norm_buffer_bytes(d->Tr, (int)N) * S);
+  const size_t S = d->prec_slots, N = d->slot_floats();
+  dfree(d, &d->norm16, scb::norm_buffer_bytes(d->Tr, d->N) * S);
   dfree(d, &d->top16, sizeof(float) * N * S);
   dfree(d, &d->flags, sizeof(int) * N * S);
   dfree(d, &d->flag_counts, sizeof(int) * S);
@@ -214,9 +210,9 @@ int ensure_prec(sc_dd* d, int slots) {
   cudaDeviceSynchronize();
   drop_graphs(d);
   free_prec(d);
-  const size_t S = slots, N = d->N;
+  const size_t S = slots, N = d->slot_floats();
   cudaError_t e;
-  if ((e = dalloc(d, &d->norm16, scb::norm_buffer_bytes(d->Tr, (int)N) * S)) != cudaSuccess ||
+  if ((e = dalloc(d, &d->norm16, scb::norm_buffer_bytes(d->Tr, d->N) * S)) != cudaSuccess ||
       (e = dalloc(d, &d->top16, sizeof(float) * N * S)) != cudaSuccess ||
       (e = dalloc(d, &d->flags, sizeof(int) * N * S)) != cudaSuccess ||
       (e = dalloc(d, &d->flag_counts, sizeof(int) * S)) != cudaSuccess ||
@@ -273,13 +269,10 @@ int ensure_slots(sc_dd* d, int slots, int cand_cap) {
   drop_graphs(d);
   free_slots(d);
   d->cand_cap = nc;
-  const size_t N = d->N, S = ns;
+  const size_t N = d->slot_floats(), S = ns;
   cudaError_t e;
   if ((e = dalloc(d, &d->top, sizeof(float) * N * S)) != cudaSuccess ||
       (e = dalloc(d, &d->colsum, sizeof(float) * N * S)) != cudaSuccess ||
-      (e = dalloc(d, &d->sel, sizeof(scb::SelectState) * S)) != cudaSuccess ||
-      (e = dalloc(d, &d->partials, sizeof(scb::MomentPartial) * d->n_partials * S)) != cudaSuccess ||
-      (e = dalloc(d, &d->var, sizeof(double) * 2 * scb::kVarChunks * S)) != cudaSuccess ||
       (e = dalloc(d, &d->work, sizeof(float) * scb::order_work_floats(d->N) * S)) != cudaSuccess ||
       (e = dalloc(d, &d->lists, sizeof(int) * scb::order_list_entries(d->N) * S)) != cudaSuccess ||
       (e = dalloc(d, &d->hdrs, sizeof(scb::SearchHeader) * S)) != cudaSuccess ||
@@ -292,7 +285,6 @@ int ensure_slots(sc_dd* d, int slots, int cand_cap) {
                 std::string("scratch allocation failed: ") + cudaGetErrorString(e));
   }
   d->slots = ns;
-  if ((e = cudaMemset(d->sel, 0, sizeof(scb::SelectState) * S)) != cudaSuccess) return cuda_fail(e, "scratch memset");
   return SC_DD_OK;
 }
 
@@ -337,12 +329,9 @@ int queue_batch(sc_dd* dd, int n, const float* const* inputs, const long long* s
     q.snr_threshold = snr_threshold;
     q.elem = elem;
     q.cand_cap = dd->cand_cap;
-    const size_t N = dd->N;
+    const size_t N = dd->slot_floats();
     q.top = dd->top + N * k;
     q.colsum = dd->colsum + N * k;
-    q.sel = dd->sel + k;
-    q.partials = dd->partials + (size_t)dd->n_partials * k;
-    q.var = dd->var + (size_t)2 * scb::kVarChunks * k;
     q.work = dd->work + scb::order_work_floats(dd->N) * k;
     q.lists = dd->lists + scb::order_list_entries(dd->N) * k;
     q.hdr = dd->hdrs + k;
@@ -605,7 +594,6 @@ int sc_dd_create(int num_timesteps, int num_channels, double foff_mhz, double ts
     delete d;
     return cuda_fail(e, "sc_dd_create: no CUDA device");
   }
-  d->n_partials = 2 * d->num_sms;
   // One slot; candidates for windows of 16 channels or more (grown when a call needs more).
   int rc = ensure_slots(d, 1, std::min(num_channels / 2 + 2, num_channels / 16 + 2));
   if (rc == SC_DD_OK && d->Tr > 32) {

@@ -18,14 +18,13 @@ namespace scb {
 
 namespace {
 
-// Zeroes, per search of the batch: top (and the 16-bit tops), the result header, the
-// order-statistic state and the flagged-channel count.
+// Zeroes, per search of the batch: top (and the 16-bit tops), the result header and the
+// flagged-channel count.
 __global__ void clear_kernel(const __grid_constant__ SearchBatch b, const __grid_constant__ PrecisionBatch pb) {
   const SearchDesc& d = b.s[blockIdx.y];
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d.N; c += gridDim.x * blockDim.x) d.top[c] = 0.0f;
   if (blockIdx.x == 0 && threadIdx.x < (int)(sizeof(SearchHeader) / 4))
     reinterpret_cast<int*>(d.hdr)[threadIdx.x] = 0;
-  if (blockIdx.x == 0) reset_select(d.sel, d.first, d.mid, d.last);  // the order-statistic state
   if (pb.count > 0 && blockIdx.y < (unsigned)pb.count && pb.s[blockIdx.y].flag_count) {
     const PrecisionDesc& q = pb.s[blockIdx.y];
     float* t16 = const_cast<float*>(q.top16);
@@ -52,9 +51,6 @@ SearchDesc to_desc(const ExecSearch& e) {
   s.snr_threshold = e.snr_threshold;
   s.top = e.top;
   s.colsum = e.colsum;
-  s.sel = e.sel;
-  s.partials = e.partials;
-  s.var = e.var;
   s.work = e.work;
   s.lists = e.lists;
   s.hdr = e.hdr;
@@ -285,10 +281,9 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
   return cudaGetLastError();
 }
 
-size_t ExecSearch::scratch_bytes(int Tr, int N, int cand_cap, int n_partials, int elem) {
+size_t ExecSearch::scratch_bytes(int Tr, int N, int cand_cap, int elem) {
   auto a = [](size_t x) { return (x + 255) & ~size_t(255); };
-  size_t b = a(sizeof(float) * N) * 2 + a(sizeof(SelectState)) + a(sizeof(MomentPartial) * n_partials) +
-             a(sizeof(double) * 2 * kVarChunks) + a(sizeof(float) * order_work_floats(N)) +
+  size_t b = a(sizeof(float) * N) * 2 + a(sizeof(float) * order_work_floats(N)) +
              a(sizeof(int) * order_list_entries(N)) + a(sizeof(SearchHeader)) + a(sizeof(Candidate) * cand_cap);
   if (elem != kElemF32) {
     b += a(norm_buffer_bytes(Tr, N)) + a(sizeof(float) * N) + a(sizeof(int) * N) + a(sizeof(int)) +
@@ -297,19 +292,13 @@ size_t ExecSearch::scratch_bytes(int Tr, int N, int cand_cap, int n_partials, in
   return b;
 }
 
-void ExecSearch::carve(char* base, int n_partials) {
+void ExecSearch::carve(char* base) {
   auto a = [](size_t x) { return (x + 255) & ~size_t(255); };
   char* p = base;
   top = reinterpret_cast<float*>(p);
   p += a(sizeof(float) * N);
   colsum = reinterpret_cast<float*>(p);
   p += a(sizeof(float) * N);
-  sel = reinterpret_cast<SelectState*>(p);
-  p += a(sizeof(SelectState));
-  partials = reinterpret_cast<MomentPartial*>(p);
-  p += a(sizeof(MomentPartial) * n_partials);
-  var = reinterpret_cast<double*>(p);
-  p += a(sizeof(double) * 2 * kVarChunks);
   work = reinterpret_cast<float*>(p);
   p += a(sizeof(float) * order_work_floats(N));
   lists = reinterpret_cast<int*>(p);

@@ -28,18 +28,21 @@ namespace {
 // (a warp or the block), each of which holds its own first best on return.  Eight loads in
 // flight per thread: a window's time is its loads' latency.
 template <int GROUP>
-__device__ __forceinline__ void window_best(const float* __restrict__ top, long long start, long long end, int t,
-                                            float& best, int& bidx) {
+__device__ __forceinline__ void window_best(const float* __restrict__ top, int start, int end, int t, float& best,
+                                            int& bidx) {
   constexpr int K = 8;
-  for (long long f0 = start + t; f0 < end; f0 += GROUP * K) {
+  const float floor_v = best;
+  const float* __restrict__ p = top + start;
+  const int n = end - start;
+  for (int f0 = t; f0 < n; f0 += GROUP * K) {
     float v[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = f0 + GROUP * k < end ? top[f0 + GROUP * k] : 0.0f;
+    for (int k = 0; k < K; ++k) v[k] = f0 + GROUP * k < n ? __ldg(p + f0 + GROUP * k) : floor_v;  // floor_v: not above best
 #pragma unroll
     for (int k = 0; k < K; ++k)
-      if (f0 + GROUP * k < end && v[k] > best) {
+      if (v[k] > best) {
         best = v[k];
-        bidx = (int)(f0 + GROUP * k);
+        bidx = start + f0 + GROUP * k;
       }
   }
 #pragma unroll
@@ -55,13 +58,15 @@ __device__ __forceinline__ void window_best(const float* __restrict__ top, long 
 
 // Whether a value above `best` lies in [lo, hi) among this thread's share.
 template <int GROUP>
-__device__ __forceinline__ bool window_larger(const float* __restrict__ top, long long lo, long long hi, int t, float best) {
+__device__ __forceinline__ bool window_larger(const float* __restrict__ top, int lo, int hi, int t, float best) {
   constexpr int K = 8;
+  const float* __restrict__ p = top + lo;
+  const int n = hi - lo;
   bool larger = false;
-  for (long long f0 = lo + t; f0 < hi && !larger; f0 += GROUP * K) {
+  for (int f0 = t; f0 < n && !larger; f0 += GROUP * K) {
     float v[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = f0 + GROUP * k < hi ? top[f0 + GROUP * k] : best;
+    for (int k = 0; k < K; ++k) v[k] = f0 + GROUP * k < n ? __ldg(p + f0 + GROUP * k) : best;
 #pragma unroll
     for (int k = 0; k < K; ++k) larger = larger || v[k] > best;
   }
@@ -69,11 +74,11 @@ __device__ __forceinline__ bool window_larger(const float* __restrict__ top, lon
 }
 
 constexpr int kWindowThreads = 256;
-constexpr int kWarpWindow = 512;  // windows of at most this many channels take one warp each
 
-// Wider windows take a block each: there are few of them, and one warp for 2194 channels with one
-// load in flight needed 31 us on 46 windows (eight in flight: 17 us).  Narrow windows are many,
-// and a block each would leave most threads idle.
+// A search whose windows are no more than its blocks takes a block for each: one warp for 2194
+// channels with one load in flight needed 31 us on 46 windows (eight in flight 17 us, a block
+// 8 us).  With more windows than blocks a warp each is the faster (64 searches of 1338 windows
+// of 784 channels: 80 us, and 239 us by blocks, most of whose threads idle).
 __global__ void __launch_bounds__(kWindowThreads) window_kernel(const __grid_constant__ SearchBatch b) {
   const SearchDesc& sd = b.s[blockIdx.y];
   const float* __restrict__ top = sd.top;
@@ -87,15 +92,14 @@ __global__ void __launch_bounds__(kWindowThreads) window_kernel(const __grid_con
     const int slot = atomicAdd(&hdr->num_candidates, 1);
     if (slot < cap) cands[slot] = Candidate{idx, 0, best, 0, 0ull};
   };
-  if (w <= kWarpWindow) {
+  if (nwin > gridDim.x) {
     const long long nw = (long long)gridDim.x * (kWindowThreads / 32);
     for (long long i = (long long)blockIdx.x * (kWindowThreads / 32) + warp; i < nwin; i += nw) {
       float best = thr;
       int bidx = -1;
-      window_best<32>(top, i * w, min((long long)N, (i + 1) * w), lane, best, bidx);
+      window_best<32>(top, (int)(i * w), (int)min((long long)N, (i + 1) * w), lane, best, bidx);
       if (bidx < 0) continue;
-      const bool larger = window_larger<32>(top, max(0ll, (long long)bidx - w + 1), min((long long)N, (long long)bidx + w),
-                                            lane, best);
+      const bool larger = window_larger<32>(top, max(0, bidx - w + 1), (int)min((long long)N, (long long)bidx + w), lane, best);
       if (__any_sync(0xffffffffu, larger)) continue;
       if (lane == 0) keep(bidx, best);
     }
@@ -106,7 +110,7 @@ __global__ void __launch_bounds__(kWindowThreads) window_kernel(const __grid_con
   for (long long i = blockIdx.x; i < nwin; i += gridDim.x) {
     float best = thr;
     int bidx = -1;
-    window_best<kWindowThreads>(top, i * w, min((long long)N, (i + 1) * w), threadIdx.x, best, bidx);
+    window_best<kWindowThreads>(top, (int)(i * w), (int)min((long long)N, (i + 1) * w), threadIdx.x, best, bidx);
     if (lane == 0) {
       s_best[warp] = best;
       s_idx[warp] = bidx;
@@ -126,8 +130,8 @@ __global__ void __launch_bounds__(kWindowThreads) window_kernel(const __grid_con
       __syncthreads();  // before the next window's writes
       continue;
     }
-    const bool larger = window_larger<kWindowThreads>(top, max(0ll, (long long)bidx - w + 1),
-                                                      min((long long)N, (long long)bidx + w), threadIdx.x, best);
+    const bool larger = window_larger<kWindowThreads>(top, max(0, bidx - w + 1), (int)min((long long)N, (long long)bidx + w),
+                                                      threadIdx.x, best);
     if (!__syncthreads_or(larger) && threadIdx.x == 0) keep(bidx, best);
   }
 }
@@ -260,7 +264,6 @@ cudaError_t search_hits_batch(const SearchBatch& b, int num_sms, cudaStream_t st
   for (int k = 0; k < b.count; ++k) {
     const long long w = b.s[k].window_size;
     long long n = ((long long)b.s[k].N + w - 1) / w;
-    if (w <= kWarpWindow) n = (n + kWindowThreads / 32 - 1) / (kWindowThreads / 32);  // one window per warp
     if (n > nwin) nwin = n;
   }
   long long wblocks = nwin;

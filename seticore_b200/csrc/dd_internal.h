@@ -8,7 +8,7 @@ namespace scb {
 
 constexpr int kMaxSeg = 4;       // staged windows per tree work item when jobs have their own rows
 constexpr int kMaxBatch = 64;    // searches per batched launch (descriptors travel as kernel parameters)
-constexpr int kVarChunks = 1024; // variance-emulation chunks per search, at most
+constexpr int kVarChunks = 1024; // blocks of the 16-bit forms' moments per search, at most
 // The 16-bit forms' moments buffer per search (doubles): per-block sums [0, K), sums of
 // squares [K, 2K), then the normalisation's mean and standard deviation and the minimum and
 // maximum of the unrounded rows at 2K .. 2K + 3, then per-block (minimum, maximum) pairs
@@ -19,58 +19,6 @@ constexpr int kNormMomentsDoubles = 4 * kVarChunks + 4;
 constexpr int kElemF32 = 0;
 constexpr int kElemBF16 = 1;
 constexpr int kElemF16 = 2;
-
-constexpr int kSelBins = 4096;   // histogram bins per order-statistic pass
-constexpr int kSelCands = 4096;  // candidates kept per order statistic for the exact pick
-
-// Order-statistic state for the three column-sum ranks (first, mid, last).  Each target's
-// key range narrows by histogram passes until it holds one key (mode 2) or at most kSelCands
-// values (mode 1), which a compaction pass collects for an exact pick.  Keys are the
-// order-preserving unsigned images of the floats (sel_key: -0 keyed as +0).
-struct SelectState {
-  uint32_t prefix[3];  // the selected keys, once known (read by the variance kernels)
-  uint32_t lo[3];      // current range of each target: [lo, lo + 2^wshift)
-  uint32_t wshift[3];
-  uint32_t rank[3];    // rank of the target inside its range
-  uint32_t count[3];   // values inside the range
-  uint32_t mode[3];    // 0: narrow further, 1: pick from candidates, 2: exact (one key)
-  uint32_t ncand[3];
-  uint32_t kmin, kmax;
-  unsigned ticket;
-  // filled by the order-statistic finaliser for the variance kernels
-  float mean;
-  int pad;
-  long long n_lo, n_hi, n;
-  unsigned hist[3][kSelBins];
-  uint32_t cand[3][kSelCands];
-};
-
-#ifdef __CUDACC__
-// Resets the order-statistic state of one search; run by every thread of one block.
-__device__ __forceinline__ void reset_select(SelectState* st, int first, int mid, int last) {
-  if (threadIdx.x < 3) {
-    const int j = threadIdx.x;
-    st->prefix[j] = 0;
-    st->lo[j] = 0;
-    st->wshift[j] = 0;
-    st->rank[j] = (uint32_t)(j == 0 ? first : (j == 1 ? mid : last));
-    st->count[j] = 0;
-    st->mode[j] = 0;
-    st->ncand[j] = 0;
-  }
-  if (threadIdx.x == 0) {
-    st->kmin = 0xffffffffu;
-    st->kmax = 0u;
-    st->ticket = 0;
-  }
-  for (int i = threadIdx.x; i < 3 * kSelBins; i += blockDim.x) (&st->hist[0][0])[i] = 0;
-}
-#endif
-
-struct MomentPartial {
-  double s1, s2;  // s2 unused (kept for layout)
-  unsigned long long lt_first, eq_first, lt_last, eq_last;
-};
 
 // A confirmed window maximum: channel and top sum, plus the best path found by the resolve
 // kernel, packed as (order key of the sum) << 32 | ~(path number) so that one 64-bit
@@ -117,9 +65,6 @@ struct SearchDesc {
   double snr_threshold;
   float* top;
   float* colsum;
-  SelectState* sel;
-  MomentPartial* partials;  // at least as many as the statistics grid's x dimension
-  double* var;              // 2 * kVarChunks
   float* work;              // order_work_floats(N): the column sums in nth_element order
   int* lists;               // order_list_entries(N): the swap pairs of a partition step
   SearchHeader* hdr;
@@ -297,17 +242,15 @@ cudaError_t flag_channels_batch(const PrecisionBatch& b, int num_sms, cudaStream
 // original power in the tree's pairing, the maximum floored at 0.
 cudaError_t recompute_batch(const PrecisionBatch& b, int num_sms, cudaStream_t stream);
 
-// Column sums of each search (searches whose tree computes them skip this); also resets
-// each search's order-statistic state.
+// Column sums of each search (searches whose tree computes them skip this).
 cudaError_t column_sums_batch(const SearchBatch& b, cudaStream_t stream);
 // Order statistics, mean, standard deviation and threshold of each search, from its column
-// sums and a reset select state (column_sums_batch or exec_queue's clear launch): the
-// order statistics exactly and the float variance emulated in channel order (dd_stats.cu),
-// then, for the searches whose order statistics sit on repeated values, everything again
-// in the reference's own nth_element order, bit-identical (dd_order.cu).
+// sums: the order statistics exactly and the float variance emulated in channel order (dd_stats.cu),
+// but, for the searches whose order statistics sit on repeated values (min_ties copies or
+// more), the deviation in the reference's own nth_element order, bit-identical (dd_order.cu).
 cudaError_t search_stats_batch(const SearchBatch& b, int num_sms, cudaStream_t stream);
-cudaError_t search_stats_emulated(const SearchBatch& b, int num_sms, cudaStream_t stream);
-cudaError_t search_stats_exact(const SearchBatch& b, int num_sms, cudaStream_t stream);
+cudaError_t search_stats_emulated(const SearchBatch& b, int num_sms, int min_ties, cudaStream_t stream);
+cudaError_t search_stats_exact(const SearchBatch& b, int min_ties, cudaStream_t stream);
 // The exact statistics run for a search whose three order statistics' values include one
 // held by at least this many column sums (automatic mode), or for every search.
 constexpr int kExactStatsTies = 8;
@@ -322,24 +265,24 @@ bool exact_statistics_always();
 #define SCB_HD
 #endif
 SCB_HD constexpr size_t order_work_floats(int N) { return ((size_t)N + 7) & ~(size_t)3; }
-// One std::nth_element call of the exact statistics while its range is partitioned by
-// multi-CTA rounds (dd_order.cu); three per search, after the pair lists.
+// One std::nth_element call of the exact statistics while a cluster partitions its range
+// (dd_order.cu); three per search, after the pair lists.
 constexpr int kOrderMaxSegs = 2048;  // counting segments of one partition step
 struct OrderTask {
   int first, last, nth, depth;  // the call's current range, its target and depth budget
   int sfirst, slast;            // the range of the partition step in progress
-  int active;                   // 1: the rounds partition this call; 0: its finisher does the rest
+  int active;                   // 1: the cluster partitions this call; 0: one CTA does the rest
   int error;
-  int K, cut, lk, rk;           // pairs, cut, K-th value >= pivot, (K-1)-th value <= pivot
-  unsigned ticket;              // CTAs of a round done so far
+  int K, cut;                   // pairs and cut of the step
   float pivot;
-  int nseg, seglen;
+  int pad;
   int seg_ge[kOrderMaxSegs + 1];  // per segment: values >= pivot, then the exclusive prefix
   int seg_le[kOrderMaxSegs + 1];
 };
 SCB_HD constexpr size_t order_pair_entries(int N) { return 8 * ((size_t)N / 4 + 2); }
 SCB_HD constexpr size_t order_list_entries(int N) {
-  return order_pair_entries(N) + 3 * (sizeof(OrderTask) / sizeof(int)) + 64;
+  // whole 256-byte lines, so that the lists of every slot of an array start aligned
+  return (order_pair_entries(N) + 3 * (sizeof(OrderTask) / sizeof(int)) + 64 + 63) / 64 * 64;
 }
 
 // Window de-duplication (dedoppler.cu:264-303) and drift recovery of the survivors.
@@ -388,9 +331,6 @@ struct ExecSearch {
   // scratch (carve() lays it out from one base pointer)
   float* top;
   float* colsum;
-  SelectState* sel;
-  MomentPartial* partials;
-  double* var;
   float* work;
   int* lists;
   SearchHeader* hdr;
@@ -402,8 +342,8 @@ struct ExecSearch {
   double* norm_moments;
   unsigned* norm_ticket;
   HostReport report;  // its device pointers (flag_count, norm) are filled by exec_queue
-  static size_t scratch_bytes(int Tr, int N, int cand_cap, int n_partials, int elem);
-  void carve(char* base, int n_partials);
+  static size_t scratch_bytes(int Tr, int N, int cand_cap, int elem);
+  void carve(char* base);
 };
 
 // Callbacks of exec_queue: the launch shape of each tree launch (autotuning) and points at

@@ -4,9 +4,8 @@
 // capture or beamforming pipeline that reserved the GPU's memory up front and must not
 // call cudaMalloc (which can synchronise the device) inside its processing loop, or a
 // host framework whose allocator owns all device memory.  This entry point serves them.
-// It runs the same kernels as sc_dd_search, but its scratch (top path sums, column sums,
-// order-statistic state, variance partials, the exact statistics' work array and pair
-// lists, and the candidate block) lives in the
+// It runs the same kernels as sc_dd_search, but its scratch (top path sums, column sums, the
+// exact statistics' work array and pair lists, and the candidate block) lives in the
 // fixed-size device array below instead of an engine's cudaMalloc'd buffers, and its
 // host side allocates nothing either: the statistics and candidates come back through a
 // small stack buffer, and the hits are written straight into the caller's array.
@@ -27,7 +26,6 @@ namespace {
 
 constexpr int kStaticMaxChannels = SC_DD_STATIC_MAX_CHANNELS;
 constexpr int kStaticMaxCands = 65536;
-constexpr int kStaticPartials = 1024;
 constexpr int kMaxDevices = 64;
 constexpr int kHostChunk = 256;
 
@@ -36,10 +34,7 @@ constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 // Byte offsets of each scratch region inside the static array.
 constexpr size_t kOffTop = 0;
 constexpr size_t kOffColsum = kOffTop + align256(sizeof(float) * kStaticMaxChannels);
-constexpr size_t kOffSelect = kOffColsum + align256(sizeof(float) * kStaticMaxChannels);
-constexpr size_t kOffPartials = kOffSelect + align256(sizeof(scb::SelectState));
-constexpr size_t kOffVar = kOffPartials + align256(sizeof(scb::MomentPartial) * kStaticPartials);
-constexpr size_t kOffWork = kOffVar + align256(sizeof(double) * 2 * scb::kVarChunks);
+constexpr size_t kOffWork = kOffColsum + align256(sizeof(float) * kStaticMaxChannels);
 constexpr size_t kOffLists = kOffWork + align256(sizeof(float) * scb::order_work_floats(kStaticMaxChannels));
 constexpr size_t kOffResult = kOffLists + align256(sizeof(int) * scb::order_list_entries(kStaticMaxChannels));
 constexpr size_t kScratchBytes =
@@ -126,16 +121,13 @@ int sc_dd_search_static(const float* dev_input, long long row_stride, int num_ti
   char* b = static_cast<char*>(base);
   float* top = reinterpret_cast<float*>(b + kOffTop);
   float* colsum = reinterpret_cast<float*>(b + kOffColsum);
-  scb::SelectState* sel = reinterpret_cast<scb::SelectState*>(b + kOffSelect);
-  scb::MomentPartial* partials = reinterpret_cast<scb::MomentPartial*>(b + kOffPartials);
-  double* var = reinterpret_cast<double*>(b + kOffVar);
   float* work = reinterpret_cast<float*>(b + kOffWork);
   int* lists = reinterpret_cast<int*>(b + kOffLists);
   scb::SearchHeader* hdr = reinterpret_cast<scb::SearchHeader*>(b + kOffResult);
   scb::Candidate* cands = reinterpret_cast<scb::Candidate*>(b + kOffResult + sizeof(scb::SearchHeader));
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
 
-  // Clear what must start at zero; the order-statistic state is reset by the first kernel.
+  // Clear what must start at zero.
   if ((e = cudaMemsetAsync(top, 0, sizeof(float) * N, stream)) != cudaSuccess ||
       (e = cudaMemsetAsync(hdr, 0, sizeof(scb::SearchHeader), stream)) != cudaSuccess)
     return cuda_fail(e, "sc_dd_search_static: memset");
@@ -159,15 +151,11 @@ int sc_dd_search_static(const float* dev_input, long long row_stride, int num_ti
   sd.snr_threshold = snr_threshold;
   sd.top = top;
   sd.colsum = colsum;
-  sd.sel = sel;
-  sd.partials = partials;
-  sd.var = var;
   sd.work = work;
   sd.lists = lists;
   sd.hdr = hdr;
   sd.cands = cands;
   sd.cand_cap = kStaticMaxCands;
-  if (kStaticPartials < 2 * num_sms) return fail(SC_DD_EINTERNAL, "sc_dd_search_static: too many SMs for the partials");
   if ((e = scb::column_sums_batch(batch, stream)) != cudaSuccess ||
       (e = scb::search_stats_batch(batch, num_sms, stream)) != cudaSuccess)
     return cuda_fail(e, "sc_dd_search_static: statistics kernels");

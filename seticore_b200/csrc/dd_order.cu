@@ -33,6 +33,8 @@
 //   before each term is a prefix sum of the k.  The first term whose sum would leave the
 //   binade is added with a real floating-point add and the scan restarts from the new
 //   binade.  The result is the sequential sum, bit for bit.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -45,6 +47,8 @@ namespace scb {
 
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr int kOrdThreads = 1024;
 constexpr int kOrdWarps = kOrdThreads / 32;
 constexpr int kV4 = 8;                   // float4 groups per lane in one warp step
@@ -52,14 +56,27 @@ constexpr int kStep = 32 * 4 * kV4;      // positions per warp step
 constexpr int kMaxSegs = kOrderMaxSegs;  // counting segments per partition step
 constexpr int kSmemRange = 16384;        // ranges of at most this many values run in shared memory
 constexpr int kSmemPairs = kSmemRange / 2 + 1;
+constexpr int kSerialRange = 256;        // ranges of at most this many values are finished by one thread
+constexpr int kOrderCluster = 8;         // CTAs per search
+constexpr int kSumSeg = 4096;            // terms per speculative piece of the float sum
 constexpr int kSeqPrefix = 2048;         // leading terms of a sum added one by one (thread 0)
 constexpr int kTermsPerThreadF = 16;     // terms per thread in one scan chunk of a float sum
 constexpr int kTermsPerThreadD = 8;      // ... of a double sum (two registers per term)
 constexpr int kSumChunk = kOrdThreads * kTermsPerThreadF;
 constexpr int kSumBuf = kSumChunk + kSumChunk / 16;  // one pad word per 16 terms: conflict-free
 
+// A piece of kSumSeg terms of the float sum, evaluated before the accumulator that meets it is known:
+// on the grid of the binade that an approximate prefix sum predicts, the steps it adds and the
+// parity it leaves for either parity of the accumulator before it.  Both compose along the terms.
+struct SumPiece {
+  int eb;       // biased exponent of the predicted accumulator (0: not evaluated)
+  int k[2];     // grid steps added for accumulator parity 0 and 1 (saturated: 2^25 is too many)
+  int map;      // parity after, as map_then takes it
+};
 // Shared memory of the kernel beyond the dynamic shared-memory range buffer.
 struct OrdShared {
+  SumPiece piece[kOrdWarps];
+  double warp_d[kOrdWarps], warp_d2[kOrdWarps];
   int seg_ge[kMaxSegs + 1];  // per segment: values >= pivot; then their exclusive prefix
   int seg_le[kMaxSegs + 1];  // per segment: values <= pivot; then their exclusive prefix
   float pivot;
@@ -222,14 +239,20 @@ __device__ __forceinline__ int warp_incl_scan(int x) {
 // One warp step: the float4 groups at a0 + 128 q + 4 lane (q < kV4, a0 a multiple of 4)
 // that overlap [x0, x1), loaded together (an element's position order is (q, lane, c)).
 // The buffers are padded so that a group overlapping the end of a range stays inside them.
+// GLOBAL: from the work array, which the cluster's other CTAs write too (read in L2); else shared.
+template <bool GLOBAL>
 struct VChunk {
   float4 v[kV4];
-  __device__ __forceinline__ void load(const float* __restrict__ a, int a0, int x0, int x1) {
+  __device__ __forceinline__ void load(const float* a, int a0, int x0, int x1) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int q = 0; q < kV4; ++q) {
       const int p = a0 + 128 * q + 4 * lane;
-      v[q] = (p + 3 >= x0 && p < x1) ? *reinterpret_cast<const float4*>(a + p) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p + 3 >= x0 && p < x1) {
+        if constexpr (GLOBAL) v[q] = __ldcg(reinterpret_cast<const float4*>(a + p));
+        else v[q] = *reinterpret_cast<const float4*>(a + p);
+      }
     }
   }
   __device__ __forceinline__ float at(int q, int c) const {
@@ -266,11 +289,12 @@ struct Segs {
 
 // Position of the value of rank r (0-based, in position order) among the values of one kind
 // in segment g; every lane gets it.  The caller guarantees the segment holds it.
-__device__ int find_rank(const float* __restrict__ a, const Segs& sg, int g, float p, bool kind_ge, int r) {
+template <bool GLOBAL>
+__device__ int find_rank(const float* a, const Segs& sg, int g, float p, bool kind_ge, int r) {
   const int lane = threadIdx.x & 31;
   const int x0 = sg.x0(g), x1 = sg.x1(g);
   for (int a0 = sg.start(g); a0 < x1; a0 += kStep) {
-    VChunk w;
+    VChunk<GLOBAL> w;
     w.load(a, a0, x0, x1);
 #pragma unroll
     for (int q = 0; q < kV4; ++q) {
@@ -298,28 +322,19 @@ __device__ int find_rank(const float* __restrict__ a, const Segs& sg, int g, flo
   return INT_MAX;  // not reached when the caller's rank is inside the segment
 }
 
-// __unguarded_partition_pivot(first, last) over a[first, last), block-wide: returns the cut.
-// lpos/lval/rpos/rval hold at least (last - first) / 2 + 1 entries.
-// placed: the median of three is already at `first` (a step prepared by the rounds).
-__device__ int partition_step(float* __restrict__ a, int first, int last, int* __restrict__ lpos,
-                              float* __restrict__ lval, int* __restrict__ rpos, float* __restrict__ rval,
-                              OrdShared& S, bool placed = false) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    if (!placed) move_median_to_first(a, first, first + 1, first + (last - first) / 2, last - 1);
-    S.pivot = a[first];
-    S.cross = 0;
-  }
-  __syncthreads();
-  const float p = S.pivot;
-  const Segs sg(first + 1, last);
-  const int nseg = sg.nseg;
-  // 1. Counts per segment.
-  for (int g = warp; g < nseg; g += kOrdWarps) {
+// The parts of __unguarded_partition_pivot(first, last) over a[first, last), pivot p already moved to
+// `first`.  A step in shared memory runs them by one block; a step over more values shares parts
+// 1, 3 and 4 among the CTAs of the cluster.
+//
+// 1. Per segment, the values >= p and <= p; warp w of nw takes segments w, w + nw, ...
+template <bool GLOBAL>
+__device__ void count_segments(const float* a, const Segs& sg, float p, int w0, int nw, int* seg_ge, int* seg_le) {
+  const int lane = threadIdx.x & 31;
+  for (int g = w0; g < sg.nseg; g += nw) {
     const int x0 = sg.x0(g), x1 = sg.x1(g);
     int cge = 0, cle = 0;
     for (int a0 = sg.start(g); a0 < x1; a0 += kStep) {
-      VChunk w;
+      VChunk<GLOBAL> w;
       w.load(a, a0, x0, x1);
 #pragma unroll
       for (int q = 0; q < kV4; ++q) {
@@ -332,27 +347,35 @@ __device__ int partition_step(float* __restrict__ a, int first, int last, int* _
     cge = __reduce_add_sync(0xffffffffu, cge);
     cle = __reduce_add_sync(0xffffffffu, cle);
     if (lane == 0) {
-      S.seg_ge[g] = cge;
-      S.seg_le[g] = cle;
+      seg_ge[g] = cge;
+      seg_le[g] = cle;
     }
   }
-  __syncthreads();
+}
+
+// 2. One block, the counts in S.seg_ge and S.seg_le: their exclusive prefixes in place, S.K pairs, and
+// the cut (returned).
+template <bool GLOBAL>
+__device__ int scan_and_cut(const float* a, const Segs& sg, float p, OrdShared& S) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nseg = sg.nseg;
+  if (tid == 0) S.cross = 0;
   block_exclusive_scan<kOrdThreads>(S.seg_ge, nseg, S.warp_i);
   block_exclusive_scan<kOrdThreads>(S.seg_le, nseg, S.warp_i);
   const int total_ge = S.seg_ge[nseg], total_le = S.seg_le[nseg];
-  // 2. The segment where cL stops being <= cR: the last segment g whose start has
-  //    cL = seg_ge[g] <= cR = total_le - seg_le[g] (segment 0 always qualifies).
+  // The segment where cL stops being <= cR: the last segment g whose start has
+  // cL = seg_ge[g] <= cR = total_le - seg_le[g] (segment 0 always qualifies).
   for (int g = tid; g < nseg; g += kOrdThreads)
     if (S.seg_ge[g] <= total_le - S.seg_le[g]) atomicMax(&S.cross, g);
   __syncthreads();
-  // 3. K = max over positions x of the crossing segment of min(cL(x), cR(x)) (warp 0).
+  // K = max over positions x of the crossing segment of min(cL(x), cR(x)) (warp 0).
   if (warp == 0) {
     const int g = S.cross;
     const int x0 = sg.x0(g), x1 = sg.x1(g);
     int cl = S.seg_ge[g], cr = total_le - S.seg_le[g];
     int best = 0;
     for (int a0 = sg.start(g); a0 < x1; a0 += kStep) {
-      VChunk w;
+      VChunk<GLOBAL> w;
       w.load(a, a0, x0, x1);
 #pragma unroll
       for (int q = 0; q < kV4; ++q) {
@@ -379,7 +402,7 @@ __device__ int partition_step(float* __restrict__ a, int first, int last, int* _
   }
   __syncthreads();
   const int K = S.K;
-  // 4. L[K] (warp 0) and R[K-1] (warp 1): the segment holding the rank, then a scan of it.
+  // L[K] (warp 0) and R[K-1] (warp 1): the segment holding the rank, then a scan of it.
   if (warp < 2) {
     const bool kind_ge = warp == 0;
     const int* pre = kind_ge ? S.seg_ge : S.seg_le;
@@ -393,7 +416,7 @@ __device__ int partition_step(float* __restrict__ a, int first, int last, int* _
         if (pre[m] <= rank) lo = m;
         else hi = m - 1;
       }
-      pos = find_rank(a, sg, lo, p, kind_ge, rank - pre[lo]);
+      pos = find_rank<GLOBAL>(a, sg, lo, p, kind_ge, rank - pre[lo]);
     }
     if (lane == 0) {
       if (kind_ge) S.lk = pos;
@@ -401,15 +424,24 @@ __device__ int partition_step(float* __restrict__ a, int first, int last, int* _
     }
   }
   __syncthreads();
-  const int cut = K == 0 ? S.lk : min(S.lk, S.rk);
-  if (K == 0) return cut;
-  // 5. The K pairs: positions and values, listed by rank.
-  for (int g = warp; g < nseg; g += kOrdWarps) {
-    int rge = S.seg_ge[g], rle = S.seg_le[g];
-    if (rge >= K && total_le - S.seg_le[g + 1] >= K) continue;  // no pair has a value in this segment
+  return K == 0 ? S.lk : min(S.lk, S.rk);
+}
+
+// 3. The K pairs: positions and values, listed by rank.  seg_ge, seg_le: the prefixes.
+template <bool GLOBAL>
+__device__ void list_pairs(const float* a, const Segs& sg, float p, int K, int total_le, const int* seg_ge,
+                           const int* seg_le, int w0, int nw, int* lpos, float* lval, int* rpos, float* rval) {
+  const int lane = threadIdx.x & 31;
+  auto pre = [](const int* s, int g) {
+    if constexpr (GLOBAL) return __ldcg(s + g);
+    else return s[g];
+  };
+  for (int g = w0; g < sg.nseg; g += nw) {
+    int rge = pre(seg_ge, g), rle = pre(seg_le, g);
+    if (rge >= K && total_le - pre(seg_le, g + 1) >= K) continue;  // no pair has a value in this segment
     const int x0 = sg.x0(g), x1 = sg.x1(g);
     for (int a0 = sg.start(g); a0 < x1; a0 += kStep) {
-      VChunk w;
+      VChunk<GLOBAL> w;
       w.load(a, a0, x0, x1);
 #pragma unroll
       for (int q = 0; q < kV4; ++q) {
@@ -443,99 +475,132 @@ __device__ int partition_step(float* __restrict__ a, int first, int last, int* _
       }
     }
   }
-  __syncthreads();
-  // 6. The swaps: the k-th value >= pivot goes where the k-th value <= pivot was, and back.
-  for (int k0 = tid; k0 < K; k0 += 4 * kOrdThreads) {
+}
+
+// 4. The swaps: the k-th value >= p goes where the k-th value <= p was, and back; thread t of nt.
+template <bool GLOBAL>
+__device__ void swap_pairs(float* a, int K, int t, int nt, const int* lpos, const float* lval, const int* rpos,
+                           const float* rval) {
+  auto at = [](const auto* p) {
+    if constexpr (GLOBAL) return __ldcg(p);
+    else return *p;
+  };
+  for (int k0 = t; k0 < K; k0 += 4 * nt) {
     int i[4], j[4];
     float vi[4], vj[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int k = k0 + u * kOrdThreads;
+      const int k = k0 + u * nt;
       if (k < K) {
-        i[u] = lpos[k];
-        j[u] = rpos[k];
-        vi[u] = lval[k];
-        vj[u] = rval[k];
+        i[u] = at(lpos + k);
+        j[u] = at(rpos + k);
+        vi[u] = at(lval + k);
+        vj[u] = at(rval + k);
       }
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      if (k0 + u * kOrdThreads < K) {
+      if (k0 + u * nt < K) {
         a[i[u]] = vj[u];
         a[j[u]] = vi[u];
       }
     }
   }
+}
+
+// __unguarded_partition_pivot(first, last) over a[first, last) in shared memory, block-wide:
+// returns the cut.  The lists hold at least (last - first) / 2 + 1 entries.
+__device__ int partition_step(float* a, int first, int last, int* lpos, float* lval, int* rpos, float* rval, OrdShared& S) {
+  const int tid = threadIdx.x, warp = tid >> 5;
+  if (tid == 0) {
+    move_median_to_first(a, first, first + 1, first + (last - first) / 2, last - 1);
+    S.pivot = a[first];
+  }
+  __syncthreads();
+  const float p = S.pivot;
+  const Segs sg(first + 1, last);
+  count_segments<false>(a, sg, p, warp, kOrdWarps, S.seg_ge, S.seg_le);
+  __syncthreads();
+  const int cut = scan_and_cut<false>(a, sg, p, S);
+  const int K = S.K;
+  if (K == 0) return cut;
+  list_pairs<false>(a, sg, p, K, S.seg_le[sg.nseg], S.seg_ge, S.seg_le, warp, kOrdWarps, lpos, lval, rpos, rval);
+  __syncthreads();
+  swap_pairs<false>(a, K, tid, kOrdThreads, lpos, lval, rpos, rval);
   __syncthreads();
   return cut;
 }
 
-// The rest of std::nth_element(a + first, a + nth, a + last) as libstdc++ runs it, from a
-// range and depth budget reached so far (pending: a step of [first, last) is prepared -- its
-// pivot in place, its depth charged -- and runs first): partition steps while the range holds more than 3
-// values; at the depth limit a heap selection of [first, nth] and a swap of a[first] with
-// a[nth]; else a final insertion sort.  Ranges of up to kSmemRange values are moved to shared
-// memory (sdata, slists) for the rest.  lpos..rval: the pair lists, `big` entries each.  A
-// cut outside (first, last) -- impossible for a correct partition -- stops the selection and
-// sets *bad, so that no later access leaves the range.
-__device__ void introselect_from(float* a, int first, int nth, int last, int depth, bool pending, int* lists, int big,
-                                 float* sdata, int* slists, OrdShared& S, bool* bad) {
-  if (*bad || first == last || nth == last) return;
-  if (pending) {
-    const int cut = partition_step(a, first, last, lists, reinterpret_cast<float*>(lists + big), lists + 2 * big,
-                                   reinterpret_cast<float*>(lists + 3 * big), S, true);
-    if (cut <= first || cut >= last) {
-      *bad = true;
-      return;
-    }
-    if (cut <= nth) first = cut;
-    else last = cut;
-  }
-  while (last - first > 3 && last - first > kSmemRange) {
-    if (depth == 0) {
-      if (threadIdx.x == 0) {
-        heap_select_(a + first, nth + 1 - first, last - first);
-        const float t = a[first];
-        a[first] = a[nth];
-        a[nth] = t;
-      }
-      __syncthreads();
-      return;
-    }
+// Introselect's partition steps on [fr, lr) by one thread, in shared memory, until the range holds at
+// most 3 values, the depth budget is spent or the range is bad (the caller's cut check).
+__device__ void small_steps(float* v, int& fr, int& lr, int nr, int& depth, bool* bad) {
+  while (lr - fr > 3 && depth > 0) {
     --depth;
-    const int cut = partition_step(a, first, last, lists, reinterpret_cast<float*>(lists + big), lists + 2 * big,
-                                   reinterpret_cast<float*>(lists + 3 * big), S);
-    if (cut <= first || cut >= last) {
+    move_median_to_first(v, fr, fr + 1, fr + (lr - fr) / 2, lr - 1);
+    const float p = v[fr];
+    // __unguarded_partition(fr + 1, lr, pivot): the pivot bounds both scans.
+    int i = fr + 1, j = lr;
+    for (;;) {
+      while (i < lr && v[i] < p) ++i;
+      --j;
+      while (j > fr && p < v[j]) --j;
+      if (!(i < j)) break;
+      const float t = v[i];
+      v[i] = v[j];
+      v[j] = t;
+      ++i;
+    }
+    if (i <= fr || i >= lr) {
       *bad = true;
       return;
     }
-    if (cut <= nth) first = cut;
-    else last = cut;
+    if (i <= nr) fr = i;
+    else lr = i;
   }
+}
+
+// The rest of std::nth_element(a + first, a + nth, a + last) as libstdc++ runs it, one block, from the
+// range and depth budget that the cluster's steps left: at most kSmemRange values, which move
+// to shared memory (sdata, slists), or a spent budget.  Partition steps while the range holds
+// more than 3 values; at the depth limit a heap selection of [first, nth] and a swap of
+// a[first] with a[nth]; else a final insertion sort.  A cut outside (first, last) -- impossible
+// for a correct partition -- stops the selection and sets *bad, so that no later access
+// leaves the range.
+__device__ void introselect_from(float* a, int first, int nth, int last, int depth, float* sdata, int* slists, OrdShared& S,
+                                 bool* bad) {
+  if (first == last || nth == last) return;
   const int f0 = first, n = last - first;
-  if (n > 3) {
-    for (int i = threadIdx.x; i < n; i += kOrdThreads) sdata[i] = a[f0 + i];
-    __syncthreads();
-    int fr = 0, lr = n;
-    const int nr = nth - f0;
-    bool heap = false;
-    while (lr - fr > 3) {
-      if (depth == 0) {
-        heap = true;
-        break;
-      }
-      --depth;
-      const int cut = partition_step(sdata, fr, lr, slists, reinterpret_cast<float*>(slists + kSmemPairs),
-                                     slists + 2 * kSmemPairs, reinterpret_cast<float*>(slists + 3 * kSmemPairs), S);
-      if (cut <= fr || cut >= lr) {
-        *bad = true;
-        break;
-      }
-      if (cut <= nr) fr = cut;
-      else lr = cut;
+  if (n > kSmemRange) {  // the depth budget is spent
+    if (threadIdx.x == 0) {
+      heap_select_(a + first, nth + 1 - first, last - first);
+      const float t = a[first];
+      a[first] = a[nth];
+      a[nth] = t;
     }
-    if (threadIdx.x == 0 && !*bad) {
-      if (heap) {
+    __syncthreads();
+    return;
+  }
+  for (int i = threadIdx.x; i < n; i += kOrdThreads) sdata[i] = __ldcg(a + f0 + i);
+  __syncthreads();
+  int fr = 0, lr = n;
+  const int nr = nth - f0;
+  while (lr - fr > kSerialRange && depth > 0) {
+    --depth;
+    const int cut = partition_step(sdata, fr, lr, slists, reinterpret_cast<float*>(slists + kSmemPairs),
+                                   slists + 2 * kSmemPairs, reinterpret_cast<float*>(slists + 3 * kSmemPairs), S);
+    if (cut <= fr || cut >= lr) {
+      *bad = true;
+      break;
+    }
+    if (cut <= nr) fr = cut;
+    else lr = cut;
+  }
+  if (threadIdx.x == 0 && !*bad) {
+    small_steps(sdata, fr, lr, nr, depth, bad);
+    if (*bad) {
+      S.K = -1;
+    } else {
+      if (lr - fr > 3) {  // the depth budget is spent
         heap_select_(sdata + fr, nr + 1 - fr, lr - fr);
         const float t = sdata[fr];
         sdata[fr] = sdata[nr];
@@ -543,12 +608,12 @@ __device__ void introselect_from(float* a, int first, int nth, int last, int dep
       } else {
         insertion_sort(sdata, fr, lr);
       }
+      S.K = 0;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += kOrdThreads) a[f0 + i] = sdata[i];
-  } else if (threadIdx.x == 0) {
-    insertion_sort(a, first, last);
   }
+  __syncthreads();
+  if (!*bad && S.K < 0) *bad = true;
+  for (int i = threadIdx.x; i < n; i += kOrdThreads) a[f0 + i] = sdata[i];
   __syncthreads();
 }
 
@@ -657,32 +722,38 @@ __device__ __forceinline__ void stage_terms(const float* __restrict__ v, long lo
   }
 }
 
-// Sum of term(v[i]) for i in [lo, hi] in index order, rounded after every add as an Acc
-// accumulator starting at 0 does.  Block-wide; every thread gets the result.  sbuf: kSumBuf
-// floats of shared memory.
+// The first terms of a sum, [lo, min(hi + 1, lo + kSeqPrefix)), added one by one into s_sum (shared)
+// from 0; returns the position after them.
 template <typename Acc, typename TermFn>
-__device__ Acc exact_sequential_sum(const float* __restrict__ v, long long lo, long long hi, TermFn term, float* sbuf,
-                                    OrdShared& S) {
+__device__ long long sequential_start(const float* __restrict__ v, long long lo, long long hi, TermFn term, float* sbuf,
+                                      Acc& s_sum) {
+  const long long pre_end = min(hi + 1, lo + kSeqPrefix);
+  stage_terms<kSeqPrefix / kOrdThreads>(v, lo, pre_end, term, sbuf);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    Acc acc = Acc(0);
+    for (int r = 0; r < (int)(pre_end - lo); ++r) acc = acc + (Acc)sbuf[r + (r >> 4)];
+    s_sum = acc;
+  }
+  __syncthreads();
+  return pre_end;
+}
+
+// Adds term(v[i]) for i in [pos, hi] to s_sum (shared) in index order, rounded after every add as an Acc
+// accumulator does.  Block-wide, TPT terms per thread at a time.  sbuf: kSumBuf floats of
+// shared memory.
+template <typename Acc, int TPT, typename TermFn>
+__device__ void sequential_range(const float* __restrict__ v, long long pos, long long hi, TermFn term, float* sbuf,
+                                 OrdShared& S, Acc& s_sum) {
   using Tr = AccTraits<Acc>;
   using PK = Packed<Tr::P>;
   using W = typename PK::W;
-  constexpr int TPT = sizeof(W) == 4 ? kTermsPerThreadF : kTermsPerThreadD;
   constexpr long long CH = (long long)kOrdThreads * TPT;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr long long kTop = (1ll << Tr::P) - 1;
   constexpr long long kLow = 1ll << (Tr::P - 1);
-  __shared__ Acc s_sum;
-  const long long pre_end = min(hi + 1, lo + kSeqPrefix);
-  stage_terms<TPT>(v, lo, pre_end, term, sbuf);
+  if (tid == 0) S.s_slow = 0;
   __syncthreads();
-  if (tid == 0) {
-    Acc acc = Acc(0);
-    for (int r = 0; r < (int)(pre_end - lo); ++r) acc = acc + (Acc)sbuf[r + (r >> 4)];
-    s_sum = acc;
-    S.s_slow = 0;
-  }
-  __syncthreads();
-  long long pos = pre_end;
   while (pos <= hi) {
     const long long chunk_end = min(hi + 1, pos + CH);
     stage_terms<TPT>(v, pos, chunk_end, term, sbuf);
@@ -841,34 +912,30 @@ __device__ Acc exact_sequential_sum(const float* __restrict__ v, long long lo, l
     s_sum = acc;
   }
   __syncthreads();
-  const Acc r = s_sum;
-  __syncthreads();
-  return r;
 }
 
-// The double sum of the floats v[lo..hi], in index order.  Every partial sum is a multiple
-// of 2^g, g the lowest set bit of any term, and at most sum |v| in magnitude; when that
-// bound is below 2^(52+g) every partial sum is a double, so every order of adding gives the
-// exact sum, and a parallel reduction equals the sequential one.  Otherwise the sequential
-// scan above runs.
-__device__ double ordered_double_sum(const float* __restrict__ v, long long lo, long long hi, float* sbuf,
-                                     OrdShared& S) {
+// A CTA's share of the double sum of v[lo..hi] in any order: the sum, the sum of magnitudes and the
+// lowest set bit of any term (INT_MAX: all zero, INT_MIN: a term is not finite).
+struct PlainSum {
+  double abs, sum;
+  int g, pad;
+};
+__device__ PlainSum plain_sum(const float* v, long long lo, long long hi, int cta, int ctas, OrdShared& S) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  __shared__ double s_abs[kOrdWarps], s_sum[kOrdWarps];
-  __shared__ int s_g[kOrdWarps];
   double sa = 0.0, ss = 0.0;
   int g = INT_MAX;
   const long long b0 = lo & ~3ll;  // whole float4 groups from an aligned start
-  for (long long i0 = b0 + 4ll * tid; i0 <= hi; i0 += 4ll * 4 * kOrdThreads) {
+  const long long nt = (long long)ctas * kOrdThreads;
+  for (long long i0 = b0 + 4ll * (cta * kOrdThreads + tid); i0 <= hi; i0 += 4ll * 4 * nt) {
     float4 q[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const long long i = i0 + 4ll * u * kOrdThreads;
+      const long long i = i0 + 4ll * u * nt;
       q[u] = i <= hi ? __ldcg(reinterpret_cast<const float4*>(v + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const long long i = i0 + 4ll * u * kOrdThreads;
+      const long long i = i0 + 4ll * u * nt;
       const float f4[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -890,38 +957,81 @@ __device__ double ordered_double_sum(const float* __restrict__ v, long long lo, 
     ss += __shfl_down_sync(0xffffffffu, ss, o);
     g = min(g, __shfl_down_sync(0xffffffffu, g, o));
   }
+  __syncthreads();
   if (lane == 0) {
-    s_abs[warp] = sa;
-    s_sum[warp] = ss;
-    s_g[warp] = g;
+    S.warp_d[warp] = sa;
+    S.warp_d2[warp] = ss;
+    S.warp_i[warp] = g;
   }
   __syncthreads();
-  double tot_abs = 0.0, tot = 0.0;
-  int gmin = INT_MAX;
+  PlainSum r{0.0, 0.0, INT_MAX, 0};
   for (int w = 0; w < kOrdWarps; ++w) {
-    tot_abs += s_abs[w];
-    tot += s_sum[w];
-    gmin = min(gmin, s_g[w]);
+    r.abs += S.warp_d[w];
+    r.sum += S.warp_d2[w];
+    r.g = min(r.g, S.warp_i[w]);
   }
   __syncthreads();
-  if (gmin == INT_MAX) return 0.0;  // every term is zero
-  if (gmin != INT_MIN && gmin > -1000 && tot_abs < ldexp(1.0, 52 + gmin)) return tot;
-  return exact_sequential_sum<double>(v, lo, hi, [](float f) { return f; }, sbuf, S);
+  return r;
+}
+// Every partial sum is a multiple of 2^g, g the lowest set bit of any term, and at most
+// sum |v| in magnitude; when that bound is below 2^(52+g) every partial sum is a double, so every
+// order of adding gives the exact sum, and a parallel reduction equals the sequential one.
+__device__ __forceinline__ bool any_order_is_exact(const PlainSum& p) {
+  return p.g == INT_MAX || (p.g != INT_MIN && p.g > -1000 && p.abs < ldexp(1.0, 52 + p.g));
+}
+
+constexpr int kPieceSat = 1 << 25;
+__device__ __forceinline__ SumPiece then(const SumPiece& f, const SumPiece& g) {
+  SumPiece r;
+  r.eb = f.eb;
+  r.k[0] = min(f.k[0] + ((f.map & 1) ? g.k[1] : g.k[0]), kPieceSat);
+  r.k[1] = min(f.k[1] + ((f.map & 2) ? g.k[1] : g.k[0]), kPieceSat);
+  r.map = (int)map_then((unsigned)f.map, (unsigned)g.map);
+  return r;
+}
+// One block: the piece v[pos, end), end - pos <= kSumSeg, on the grid of an accumulator of biased
+// exponent eb.  Every thread gets it.  A term that no such accumulator keeps in its binade
+// saturates the piece.
+template <typename TermFn>
+__device__ SumPiece sum_piece(const float* v, long long pos, long long end, int eb, TermFn term, OrdShared& S) {
+  using PK = Packed<24>;
+  constexpr int TPT = kSumSeg / kOrdThreads;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  SumPiece p{eb, {0, 0}, 2};
+#pragma unroll
+  for (int j = 0; j < TPT; ++j) {
+    const long long i = pos + tid * TPT + j;
+    const uint32_t w = i < end ? PK::make(term(__ldcg(v + i)), eb - 150) : 0u;
+    SumPiece t;
+    t.k[0] = PK::big(w) || PK::neg(w) ? kPieceSat : (int)min(PK::steps(w, 0), (long long)kPieceSat);
+    t.k[1] = PK::big(w) || PK::neg(w) ? kPieceSat : (int)min(PK::steps(w, 1), (long long)kPieceSat);
+    t.map = (int)PK::pmap(w);
+    p = then(p, t);
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {  // neighbouring runs, left then right
+    SumPiece y;
+    y.k[0] = __shfl_down_sync(0xffffffffu, p.k[0], o);
+    y.k[1] = __shfl_down_sync(0xffffffffu, p.k[1], o);
+    y.map = __shfl_down_sync(0xffffffffu, p.map, o);
+    if ((lane & (2 * o - 1)) == 0) p = then(p, y);
+  }
+  __syncthreads();
+  if (lane == 0) S.piece[warp] = p;
+  __syncthreads();
+  p = S.piece[0];
+  for (int w = 1; w < kOrdWarps; ++w) p = then(p, S.piece[w]);
+  return p;
 }
 
 // ---------------------------------------------------------------------------------------
-// The large partition steps as multi-CTA rounds
+// One cluster per search
 // ---------------------------------------------------------------------------------------
 //
-// While the range of an nth_element call is larger than kSmemRange, its partition steps run
-// as rounds of three launches over every search of the batch (and both ends' calls at once):
-// count (the last CTA of a task scans the counts and finds K and the cut), lists, and swap
-// (the last CTA updates the range and moves the next pivot into place).  A task whose range
-// fits shared memory, or whose depth budget is spent, goes inactive; its finisher (one CTA)
-// carries on from the same state, so any number of rounds gives the same result.
-
-constexpr int kRoundThreads = 256;
-constexpr int kRoundWarps = kRoundThreads / 32;
+// While the range of an nth_element call is larger than kSmemRange, the CTAs of the cluster share
+// its partition steps, meeting at the cluster's hardware barrier; the rest of the call is one
+// CTA's, in shared memory.  The two calls of the ends touch disjoint ranges and run side by side
+// on the cluster's halves.
 
 __device__ __forceinline__ OrderTask* order_tasks(const SearchDesc& sd) {
   return reinterpret_cast<OrderTask*>(sd.lists + order_pair_entries(sd.N));
@@ -940,7 +1050,7 @@ __device__ __forceinline__ int* task_lists(const SearchDesc& sd, int t, int* big
 
 // The start of call t's first step or the next one (one thread): if its range is still
 // larger than kSmemRange and the depth budget allows, the median of three moves to `first`
-// as __unguarded_partition_pivot does, and the step's range and segments are recorded.
+// as __unguarded_partition_pivot does, and the step's range is recorded.
 __device__ void task_next_step(float* a, OrderTask& T) {
   if (T.error || T.last - T.first <= kSmemRange || T.depth == 0) {
     T.active = 0;
@@ -951,9 +1061,6 @@ __device__ void task_next_step(float* a, OrderTask& T) {
   T.slast = T.last;
   move_median_to_first(a, T.first, T.first + 1, T.first + (T.last - T.first) / 2, T.last - 1);
   T.pivot = a[T.first];
-  const Segs sg(T.first + 1, T.last);
-  T.nseg = sg.nseg;
-  T.seglen = sg.seglen;
   T.active = 1;
 }
 
@@ -964,8 +1071,8 @@ __device__ void task_init(float* a, OrderTask& T, int first, int nth, int last) 
   T.last = last;
   T.nth = nth;
   T.depth = last > first ? 2 * (31 - __clz(last - first)) : 0;
+  T.sfirst = T.slast = first;
   T.error = 0;
-  T.ticket = 0;
   T.active = 0;
   if (first == last || nth == last) {
     T.first = T.last;  // nothing to do
@@ -974,329 +1081,245 @@ __device__ void task_init(float* a, OrderTask& T, int first, int nth, int last) 
   task_next_step(a, T);
 }
 
-// Last-CTA election of a round: true in the one CTA that finishes last.
-__device__ __forceinline__ bool last_cta(unsigned* ticket, unsigned total) {
-  __shared__ bool s_last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == total - 1;
-  __syncthreads();
-  if (s_last) __threadfence();
-  return s_last;
-}
-
-// The column sums copied to the work array; the last CTA of a search starts the middle call.
-__global__ void __launch_bounds__(kRoundThreads) order_init_kernel(const __grid_constant__ SearchBatch b,
-                                                                   int min_ties) {
-  const SearchDesc& sd = b.s[blockIdx.y];
-  const int N = sd.N;
-  if (N <= 0 || sd.hdr->ties < min_ties) return;
-  OrderTask* tasks = order_tasks(sd);
-  const int n4 = N / 4;  // both arrays start 256-byte aligned
-  const float4* __restrict__ src = reinterpret_cast<const float4*>(sd.colsum);
-  float4* dst = reinterpret_cast<float4*>(sd.work);
-  for (int i = blockIdx.x * kRoundThreads + threadIdx.x; i < n4; i += gridDim.x * kRoundThreads) dst[i] = __ldcg(src + i);
-  if (blockIdx.x == 0)
-    for (int i = 4 * n4 + threadIdx.x; i < N; i += kRoundThreads) sd.work[i] = __ldcg(sd.colsum + i);
-  if (last_cta(&tasks[0].ticket, gridDim.x) && threadIdx.x == 0) {
-    task_init(sd.work, tasks[0], 0, sd.mid, N);
-    tasks[1].active = tasks[2].active = 0;
-  }
-}
-
-// Zeroes the tickets of a search's calls (before the copy launch uses the first).
-__global__ void order_reset_kernel(const __grid_constant__ SearchBatch b) {
-  OrderTask* tasks = order_tasks(b.s[blockIdx.y]);
-  if (threadIdx.x < 3) {
-    tasks[threadIdx.x].ticket = 0;
-    tasks[threadIdx.x].active = 0;
-  }
-}
-
-// Round, launch 1: counts per segment; the last CTA of a task scans them and finds K, the
-// cut and the next range.
-__global__ void __launch_bounds__(kRoundThreads) round_count_kernel(const __grid_constant__ SearchBatch b, int t0,
-                                                                    int nt) {
-  const int t = t0 + (int)(blockIdx.y % nt);
-  const SearchDesc& sd = b.s[blockIdx.y / nt];
-  OrderTask& T = order_tasks(sd)[t];
-  if (!*(volatile int*)&T.active) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float* __restrict__ a = sd.work;
-  const float p = T.pivot;
-  const Segs sg(T.sfirst + 1, T.slast);
-  const int nseg = sg.nseg;
-  for (int g = blockIdx.x * kRoundWarps + warp; g < nseg; g += gridDim.x * kRoundWarps) {
-    const int x0 = sg.x0(g), x1 = sg.x1(g);
-    int cge = 0, cle = 0;
-    for (int a0 = sg.start(g); a0 < x1; a0 += kStep) {
-      VChunk w;
-      w.load(a, a0, x0, x1);
-#pragma unroll
-      for (int q = 0; q < kV4; ++q) {
-        unsigned mg, ml;
-        w.masks(q, a0, x0, x1, p, mg, ml);
-        cge += __popc(mg);
-        cle += __popc(ml);
-      }
-    }
-    cge = __reduce_add_sync(0xffffffffu, cge);
-    cle = __reduce_add_sync(0xffffffffu, cle);
-    if (lane == 0) {
-      T.seg_ge[g] = cge;
-      T.seg_le[g] = cle;
-    }
-  }
-  if (!last_cta(&T.ticket, gridDim.x)) return;
-  // The scans, in shared memory, written back for the lists launch.
-  __shared__ int s_ge[kMaxSegs + 1], s_le[kMaxSegs + 1];
-  __shared__ int s_tmp[kRoundWarps];
-  __shared__ int s_cross, s_K, s_lk, s_rk;
-  for (int g = threadIdx.x; g < nseg; g += kRoundThreads) {
-    s_ge[g] = __ldcg(&T.seg_ge[g]);
-    s_le[g] = __ldcg(&T.seg_le[g]);
-  }
-  if (threadIdx.x == 0) s_cross = 0;
-  __syncthreads();
-  block_exclusive_scan<kRoundThreads>(s_ge, nseg, s_tmp);
-  block_exclusive_scan<kRoundThreads>(s_le, nseg, s_tmp);
-  const int total_ge = s_ge[nseg], total_le = s_le[nseg];
-  for (int g = threadIdx.x; g <= nseg; g += kRoundThreads) {
-    T.seg_ge[g] = s_ge[g];
-    T.seg_le[g] = s_le[g];
-  }
-  for (int g = threadIdx.x; g < nseg; g += kRoundThreads)
-    if (s_ge[g] <= total_le - s_le[g]) atomicMax(&s_cross, g);
-  __syncthreads();
-  if (warp == 0) {  // K = max over the crossing segment of min(cL(x), cR(x))
-    const int g = s_cross;
-    const int x0 = sg.x0(g), x1 = sg.x1(g);
-    int cl = s_ge[g], cr = total_le - s_le[g];
-    int best = 0;
-    for (int a0 = sg.start(g); a0 < x1; a0 += kStep) {
-      VChunk w;
-      w.load(a, a0, x0, x1);
-#pragma unroll
-      for (int q = 0; q < kV4; ++q) {
-        unsigned mg, ml;
-        w.masks(q, a0, x0, x1, p, mg, ml);
-        const int packed = __popc(mg) | (__popc(ml) << 16);
-        const int inc = warp_incl_scan(packed);
-        const int ex = inc - packed;
-        const int base = a0 + 128 * q + 4 * lane;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const unsigned below = (1u << c) - 1u;
-          if (base + c >= x0 && base + c < x1)
-            best = max(best, min(cl + (ex & 0xffff) + __popc(mg & below), cr - (ex >> 16) - __popc(ml & below)));
-        }
-        const int tot = __shfl_sync(0xffffffffu, inc, 31);
-        cl += tot & 0xffff;
-        cr -= tot >> 16;
-      }
-    }
-    best = max(best, min(cl, cr));
-    best = __reduce_max_sync(0xffffffffu, best);
-    if (lane == 0) s_K = best;
-  }
-  __syncthreads();
-  const int K = s_K;
-  if (warp < 2) {  // L[K] (warp 0) and R[K-1] (warp 1)
-    const bool kind_ge = warp == 0;
-    const int* pre = kind_ge ? s_ge : s_le;
-    const int rank = kind_ge ? K : total_le - K;
-    const bool exists = kind_ge ? K < total_ge : K >= 1;
-    int pos = INT_MAX;
-    if (exists) {
-      int lo = 0, hi = nseg - 1;
-      while (lo < hi) {
-        const int m = (lo + hi + 1) >> 1;
-        if (pre[m] <= rank) lo = m;
-        else hi = m - 1;
-      }
-      pos = find_rank(a, sg, lo, p, kind_ge, rank - pre[lo]);
-    }
-    if (lane == 0) {
-      if (kind_ge) s_lk = pos;
-      else s_rk = pos;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int cut = K == 0 ? s_lk : min(s_lk, s_rk);
-    T.K = K;
-    T.cut = cut;
-    if (cut <= T.sfirst || cut >= T.slast) {  // impossible for a correct partition
-      T.error = 1;
-      T.K = 0;
-    } else if (cut <= T.nth) {
-      T.first = cut;
-    } else {
-      T.last = cut;
-    }
-    T.ticket = 0;
-  }
-}
-
-// Round, launch 2: the K pairs' positions and values, listed by rank.
-__global__ void __launch_bounds__(kRoundThreads) round_lists_kernel(const __grid_constant__ SearchBatch b, int t0,
-                                                                    int nt) {
-  const int t = t0 + (int)(blockIdx.y % nt);
-  const SearchDesc& sd = b.s[blockIdx.y / nt];
-  OrderTask& T = order_tasks(sd)[t];
-  if (!*(volatile int*)&T.active) return;
-  const int K = T.K;
-  if (K == 0) return;
+// The partition steps of one call by CTAs cta of `ctas` (the first leads), until its range fits
+// shared memory.  Every CTA of the cluster runs the same number of barriers: `other` is the call
+// that the rest of the cluster works on (or the same one).
+__device__ void cluster_steps(cg::cluster_group& cl, const SearchDesc& sd, OrderTask* tasks, int t, int other, int cta,
+                              int ctas, OrdShared& S) {
+  OrderTask& T = tasks[t];
+  OrderTask& O = tasks[other];
+  float* a = sd.work;
   int big;
   int* lists = task_lists(sd, t, &big);
-  int* __restrict__ lpos = lists;
-  float* __restrict__ lval = reinterpret_cast<float*>(lists + big);
-  int* __restrict__ rpos = lists + 2 * big;
-  float* __restrict__ rval = reinterpret_cast<float*>(lists + 3 * big);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const float* __restrict__ a = sd.work;
-  const float p = T.pivot;
-  const Segs sg(T.sfirst + 1, T.slast);
-  const int nseg = sg.nseg;
-  const int total_le = T.seg_le[nseg];
-  for (int g = blockIdx.x * kRoundWarps + warp; g < nseg; g += gridDim.x * kRoundWarps) {
-    int rge = T.seg_ge[g], rle = T.seg_le[g];
-    if (rge >= K && total_le - T.seg_le[g + 1] >= K) continue;
-    const int x0 = sg.x0(g), x1 = sg.x1(g);
-    for (int a0 = sg.start(g); a0 < x1; a0 += kStep) {
-      VChunk w;
-      w.load(a, a0, x0, x1);
-#pragma unroll
-      for (int q = 0; q < kV4; ++q) {
-        unsigned mg, ml;
-        w.masks(q, a0, x0, x1, p, mg, ml);
-        const int packed = __popc(mg) | (__popc(ml) << 16);
-        const int inc = warp_incl_scan(packed);
-        const int eg = rge + ((inc - packed) & 0xffff), el = rle + ((inc - packed) >> 16);
-        const int base = a0 + 128 * q + 4 * lane;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const unsigned below = (1u << c) - 1u;
-          if ((mg >> c) & 1u) {
-            const int r = eg + __popc(mg & below);
-            if (r < K) {
-              lpos[r] = base + c;
-              lval[r] = w.at(q, c);
-            }
-          }
-          if ((ml >> c) & 1u) {
-            const int rd = total_le - 1 - (el + __popc(ml & below));
-            if (rd < K) {
-              rpos[rd] = base + c;
-              rval[rd] = w.at(q, c);
-            }
-          }
+  int* lpos = lists;
+  float* lval = reinterpret_cast<float*>(lists + big);
+  int* rpos = lists + 2 * big;
+  float* rval = reinterpret_cast<float*>(lists + 3 * big);
+  const int tid = threadIdx.x, w0 = cta * kOrdWarps + (tid >> 5), nw = ctas * kOrdWarps;
+  // At most the depth budget of the larger call: each of its steps spends one.
+  while (__ldcg(&T.active) || __ldcg(&O.active)) {
+    const bool mine = __ldcg(&T.active) != 0;
+    const float p = __ldcg(&T.pivot);
+    const Segs sg(__ldcg(&T.sfirst) + 1, mine ? __ldcg(&T.slast) : __ldcg(&T.sfirst) + 2);
+    if (mine) count_segments<true>(a, sg, p, w0, nw, T.seg_ge, T.seg_le);
+    cl.sync();
+    if (mine && cta == 0) {
+      for (int g = tid; g < sg.nseg; g += kOrdThreads) {
+        S.seg_ge[g] = __ldcg(&T.seg_ge[g]);
+        S.seg_le[g] = __ldcg(&T.seg_le[g]);
+      }
+      __syncthreads();
+      const int cut = scan_and_cut<true>(a, sg, p, S);
+      for (int g = tid; g <= sg.nseg; g += kOrdThreads) {
+        T.seg_ge[g] = S.seg_ge[g];
+        T.seg_le[g] = S.seg_le[g];
+      }
+      if (tid == 0) {
+        T.K = S.K;
+        T.cut = cut;
+        if (cut <= T.sfirst || cut >= T.slast) {  // impossible for a correct partition
+          T.error = 1;
+          T.K = 0;
+        } else if (cut <= T.nth) {
+          T.first = cut;
+        } else {
+          T.last = cut;
         }
-        const int tot = __shfl_sync(0xffffffffu, inc, 31);
-        rge += tot & 0xffff;
-        rle += tot >> 16;
       }
     }
+    cl.sync();
+    const int K = mine ? __ldcg(&T.K) : 0;
+    if (K > 0)
+      list_pairs<true>(a, sg, p, K, __ldcg(&T.seg_le[sg.nseg]), T.seg_ge, T.seg_le, w0, nw, lpos, lval, rpos, rval);
+    cl.sync();
+    if (K > 0) swap_pairs<true>(a, K, cta * kOrdThreads + tid, ctas * kOrdThreads, lpos, lval, rpos, rval);
+    cl.sync();
+    if (mine && cta == 0 && tid == 0) {
+      __threadfence();
+      task_next_step(a, T);
+    }
+    cl.sync();
   }
 }
 
-// Round, launch 3: the swaps; the last CTA of a task starts its next step.
-__global__ void __launch_bounds__(kRoundThreads) round_swap_kernel(const __grid_constant__ SearchBatch b, int t0,
-                                                                   int nt) {
-  const int t = t0 + (int)(blockIdx.y % nt);
-  const SearchDesc& sd = b.s[blockIdx.y / nt];
-  OrderTask& T = order_tasks(sd)[t];
-  if (!*(volatile int*)&T.active) return;
-  const int K = T.K;
-  int big;
-  int* lists = task_lists(sd, t, &big);
-  const int* __restrict__ lpos = lists;
-  const float* __restrict__ lval = reinterpret_cast<const float*>(lists + big);
-  const int* __restrict__ rpos = lists + 2 * big;
-  const float* __restrict__ rval = reinterpret_cast<const float*>(lists + 3 * big);
-  float* __restrict__ a = sd.work;
-  const int stride = gridDim.x * kRoundThreads;
-  for (int k0 = blockIdx.x * kRoundThreads + threadIdx.x; k0 < K; k0 += 4 * stride) {
-    int i[4], j[4];
-    float vi[4], vj[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = k0 + u * stride;
-      if (k < K) {
-        i[u] = __ldcg(lpos + k);
-        j[u] = __ldcg(rpos + k);
-        vi[u] = __ldcg(lval + k);
-        vj[u] = __ldcg(rval + k);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (k0 + u * stride < K) {
-        a[i[u]] = vj[u];
-        a[j[u]] = vi[u];
-      }
-    }
-  }
-  if (last_cta(&T.ticket, gridDim.x) && threadIdx.x == 0) {
-    T.ticket = 0;
-    task_next_step(a, T);
-  }
-}
-
-// The rest of each call after the rounds, one CTA per call: blockIdx.x selects the call of
-// this launch (t0 + blockIdx.x).  After the middle call, its CTA starts both end calls.
-__global__ void __launch_bounds__(kOrdThreads, 1) order_finish_kernel(const __grid_constant__ SearchBatch b, int t0,
-                                                                     int min_ties) {
+// One cluster per search whose order statistics sit on repeated values (min_ties copies or more; the
+// others leave at once): the column sums permuted as the reference's three nth_element calls
+// leave them, then the median, the mean and the deviation exactly as the reference forms them.
+//
+// As 51 launches (three per partition step, whether a search needed them or not) these cost every
+// call 67 to 165 us and a search of 2^20 whole-number column sums 2.0 ms; the one launch costs
+// 2 to 5 us and 1.6 ms.
+__global__ void __cluster_dims__(kOrderCluster, 1, 1) __launch_bounds__(kOrdThreads, 1)
+    order_kernel(const __grid_constant__ SearchBatch b, int min_ties) {
   const SearchDesc& sd = b.s[blockIdx.y];
   const int N = sd.N;
-  if (N <= 0 || sd.hdr->ties < min_ties || *(volatile int*)&sd.hdr->error) return;
+  if (N <= 0 || sd.hdr->ties < min_ties || *(volatile int*)&sd.hdr->error) return;  // every CTA of the cluster alike
   __shared__ OrdShared S;
   extern __shared__ __align__(16) float dyn[];
+  cg::cluster_group cl = cg::this_cluster();
+  const int r = (int)cl.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* sdata = dyn;                                      // kSmemRange values
   int* slists = reinterpret_cast<int*>(dyn + kSmemRange);  // 4 * kSmemPairs entries
-  const int t = t0 + (int)blockIdx.x;
   OrderTask* tasks = order_tasks(sd);
-  OrderTask& T = tasks[t];
-  bool bad = T.error != 0;
-  int big;
-  int* lists = task_lists(sd, t, &big);
-  // A task still active after the rounds has its next step prepared: the range of that step
-  // is [sfirst, slast) = [first, last).
-  introselect_from(sd.work, T.first, T.nth, T.last, T.depth, T.active != 0, lists, big, sdata, slists, S, &bad);
-  if (bad) {
-    if (threadIdx.x == 0) atomicExch(&sd.hdr->error, 2);  // the results of this search are invalid
-    return;
+  float* a = sd.work;
+  // The column sums copied to the work array (16-byte words: both start 16-byte aligned).
+  const int n4 = N / 4;
+  for (int i = r * kOrdThreads + tid; i < n4; i += kOrderCluster * kOrdThreads)
+    reinterpret_cast<float4*>(a)[i] = __ldcg(reinterpret_cast<const float4*>(sd.colsum) + i);
+  if (r == 0)
+    for (int i = 4 * n4 + tid; i < N; i += kOrdThreads) a[i] = __ldcg(sd.colsum + i);
+  cl.sync();
+  if (r == 0 && tid == 0) {
+    __threadfence();
+    task_init(a, tasks[0], 0, sd.mid, N);
   }
-  if (t == 0 && threadIdx.x == 0) {
-    task_init(sd.work, tasks[1], 0, sd.first, sd.mid - 1);
-    task_init(sd.work, tasks[2], sd.mid + 1, sd.last, N);
+  cl.sync();
+  cluster_steps(cl, sd, tasks, 0, 0, r, kOrderCluster, S);
+  bool bad = false;
+  if (r == 0) {
+    __threadfence();
+    bad = tasks[0].error != 0;
+    if (!bad) introselect_from(a, tasks[0].first, sd.mid, tasks[0].last, tasks[0].depth, sdata, slists, S, &bad);
+    if (tid == 0) {
+      if (bad) {
+        atomicExch(&sd.hdr->error, 2);  // the results of this search are invalid
+        for (int t = 1; t < 3; ++t) {
+          tasks[t].first = tasks[t].last = tasks[t].nth = tasks[t].sfirst = 0;
+          tasks[t].active = tasks[t].error = 0;
+        }
+      } else {
+        __threadfence();
+        task_init(a, tasks[1], 0, sd.first, sd.mid - 1);
+        task_init(a, tasks[2], sd.mid + 1, sd.last, N);
+      }
+    }
   }
-}
+  cl.sync();
+  const int half = kOrderCluster / 2, t = r < half ? 1 : 2, cta = r % half;
+  cluster_steps(cl, sd, tasks, t, 3 - t, cta, half, S);
+  if (cta == 0) {
+    __threadfence();
+    const OrderTask& T = tasks[t];
+    bad = T.error != 0;
+    if (!bad) introselect_from(a, T.first, T.nth, T.last, T.depth, sdata, slists, S, &bad);
+    if (bad && tid == 0) atomicExch(&sd.hdr->error, 2);
+  }
+  cl.sync();
+  if (*(volatile int*)&sd.hdr->error) return;  // set before the barrier, if at all: every CTA alike
 
-// Kernel 3, one CTA per search: the median, the mean and the deviation exactly as the
-// reference forms them, from the work array in its nth_element order.
-__global__ void __launch_bounds__(kOrdThreads, 1) order_moments_kernel(const __grid_constant__ SearchBatch b,
-                                                                      int min_ties) {
-  const SearchDesc& sd = b.s[blockIdx.y];
-  const int N = sd.N;
-  if (N <= 0 || sd.hdr->ties < min_ties || *(volatile int*)&sd.hdr->error) return;
-  __shared__ OrdShared S;
-  extern __shared__ __align__(16) float dyn[];
-  float* sbuf = dyn;  // kSumBuf floats
-  const float* __restrict__ a = sd.work;
-  const int first = sd.first, last = sd.last;
-  const float median = __ldcg(a + sd.mid);
-  const int n = last + 1 - first;
   // float sum = std::accumulate(a + first, a + last + 1, 0.0): a double sum in order.
-  const double dsum = ordered_double_sum(a, first, last, sbuf, S);
-  const float m = __fdiv_rn((float)dsum, (float)n);
-  // accum += (f - m) * (f - m), float, in order.
-  const float accum = exact_sequential_sum<float>(a, first, last, [m](float f) {
+  const int first = sd.first, last = sd.last, n = last + 1 - first;
+  __shared__ PlainSum s_plain[kOrderCluster];
+  __shared__ double s_dsum;
+  float* sbuf = dyn;  // kSumBuf floats
+  {
+    const PlainSum p = plain_sum(a, first, last, r, kOrderCluster, S);
+    if (tid < kOrderCluster) cl.map_shared_rank(s_plain, tid)[r] = p;
+  }
+  cl.sync();
+  PlainSum tot = s_plain[0];
+  for (int q = 1; q < kOrderCluster; ++q) {
+    tot.abs += s_plain[q].abs;
+    tot.sum += s_plain[q].sum;
+    tot.g = min(tot.g, s_plain[q].g);
+  }
+  if (!any_order_is_exact(tot)) {
+    if (r == 0) {
+      auto same = [](float f) { return f; };
+      const long long pos = sequential_start(a, (long long)first, (long long)last, same, sbuf, s_dsum);
+      sequential_range<double, kTermsPerThreadD>(a, pos, (long long)last, same, sbuf, S, s_dsum);
+      if (tid < kOrderCluster) *cl.map_shared_rank(&s_dsum, tid) = s_dsum;
+    }
+    cl.sync();
+    tot.sum = s_dsum;
+  }
+  const float m = __fdiv_rn((float)(tot.g == INT_MAX ? 0.0 : tot.sum), (float)n);
+  // accum += (f - m) * (f - m), float, in order: an approximate prefix sum predicts the binade of
+  // the accumulator before every piece, the cluster evaluates the pieces on those grids, and
+  // one CTA strings them together, taking the pieces that leave their binade term by term.
+  auto term = [m](float f) {
     const float d = __fsub_rn(f, m);
     return __fmul_rn(d, d);
-  }, sbuf, S);
-  if (threadIdx.x == 0) {
-    const float std_dev = sqrtf(__fdiv_rn(accum, (float)n));
+  };
+  const int np = (n + kSumSeg - 1) / kSumSeg;
+  // In the pair lists' memory (8 bytes per channel): the pieces, then the prefix sums.
+  SumPiece* pieces = reinterpret_cast<SumPiece*>(sd.lists);
+  double* prefix = reinterpret_cast<double*>(pieces + np);
+  for (int c = r * kOrdWarps + warp; c < np; c += kOrderCluster * kOrdWarps) {
+    const int c1 = min(last + 1, first + (c + 1) * kSumSeg);
+    double acc = 0.0;
+    for (int i = first + c * kSumSeg + lane; i < c1; i += 32) acc += (double)term(__ldcg(a + i));
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0) prefix[c] = acc;
+  }
+  cl.sync();
+  if (r == 0 && warp == 0) {  // exclusive prefix, 32 pieces at a time
+    double run = 0.0;
+    for (int c0 = 0; c0 < np; c0 += 32) {
+      const double v = c0 + lane < np ? __ldcg(prefix + c0 + lane) : 0.0;
+      double inc = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+      }
+      if (c0 + lane < np) prefix[c0 + lane] = run + inc - v;
+      run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+  }
+  cl.sync();
+  for (int c = 1 + r; c < np; c += kOrderCluster) {  // piece 0 starts from zero: term by term
+    const int eb = (int)((__float_as_uint((float)__ldcg(prefix + c)) >> 23) & 0xffu);
+    SumPiece p{0, {0, 0}, 2};
+    if (eb > 24 && eb < 255)
+      p = sum_piece(a, (long long)first + (long long)c * kSumSeg, min((long long)last + 1, (long long)first + (c + 1ll) * kSumSeg),
+                    eb, term, S);
+    if (tid == 0) pieces[c] = p;
+    __syncthreads();
+  }
+  cl.sync();
+  if (r != 0) return;
+  __shared__ float s_sum;
+  __shared__ int s_at;
+  SumPiece* sp = reinterpret_cast<SumPiece*>(dyn + kSumBuf);  // behind sbuf
+  constexpr int kTile = 1024;
+  long long pos = sequential_start(a, (long long)first, (long long)last, term, sbuf, s_sum);
+  sequential_range<float, kSumSeg / kOrdThreads>(a, pos, min((long long)last, (long long)first + kSumSeg - 1), term, sbuf, S,
+                                                 s_sum);
+  for (int c0 = 1; c0 < np;) {
+    const int cn = min(np, c0 + kTile);
+    for (int i = tid; i < cn - c0; i += kOrdThreads) {
+      const int4 w = __ldcg(reinterpret_cast<const int4*>(pieces + c0 + i));
+      sp[i] = SumPiece{w.x, {w.y, w.z}, w.w};
+    }
+    __syncthreads();
+    for (int c = c0; c < cn;) {
+      if (tid == 0) {
+        uint32_t u = __float_as_uint(s_sum);
+        int at = c;
+        for (; at < cn; ++at) {
+          const SumPiece& p = sp[at - c0];
+          if (p.eb == 0 || p.eb != (int)(u >> 23)) break;  // not evaluated, or another binade
+          const int A = (int)((u & 0x7fffffu) | 0x800000u) + p.k[u & 1u];
+          if (A > 0xffffff) break;  // leaves the binade
+          u = (u & 0x7f800000u) | ((uint32_t)A & 0x7fffffu);
+        }
+        s_sum = __uint_as_float(u);
+        s_at = at;
+      }
+      __syncthreads();
+      c = s_at;
+      __syncthreads();
+      if (c < cn) {
+        const long long p0 = (long long)first + (long long)c * kSumSeg;
+        sequential_range<float, kSumSeg / kOrdThreads>(a, p0, min((long long)last, p0 + kSumSeg - 1), term, sbuf, S, s_sum);
+        ++c;
+      }
+    }
+    c0 = cn;
+  }
+  if (tid == 0) {
+    const float median = __ldcg(a + sd.mid);
+    const float std_dev = sqrtf(__fdiv_rn(s_sum, (float)n));
     SearchHeader* hdr = sd.hdr;
     hdr->median = median;
     hdr->mean = m;
@@ -1308,54 +1331,14 @@ __global__ void __launch_bounds__(kOrdThreads, 1) order_moments_kernel(const __g
 
 }  // namespace
 
-namespace {
-// Rounds that bring a range of n values to kSmemRange, with slack (a task that needs more
-// finishes in its finisher's own steps).
-int rounds_for(long long n) {
-  int r = 0;
-  while (n > kSmemRange) {
-    n = n / 2 + 1;
-    ++r;
-  }
-  return r + 1;
-}
-}  // namespace
-
-cudaError_t search_stats_exact(const SearchBatch& b, int num_sms, cudaStream_t stream) {
+cudaError_t search_stats_exact(const SearchBatch& b, int min_ties, cudaStream_t stream) {
   if (b.count <= 0) return cudaSuccess;
-  const int smem_sel = (int)(sizeof(float) * kSmemRange + sizeof(int) * 4 * kSmemPairs);
-  const int smem_sum = (int)(sizeof(float) * kSumBuf);
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute(order_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_sel)) !=
-          cudaSuccess ||
-      (e = cudaFuncSetAttribute(order_moments_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_sum)) !=
-          cudaSuccess)
-    return e;
-  const int n = b.count;
-  const long long max_steps = (b.maxN + kStep - 1) / kStep;  // warp steps of the largest range
-  auto grid_x = [&](int tasks) {
-    long long g = (4ll * num_sms + (long long)tasks * n - 1) / ((long long)tasks * n);
-    const long long cap = std::max(1ll, (max_steps + kRoundWarps - 1) / kRoundWarps);
-    return (int)std::max(1ll, std::min(g, cap));
-  };
-  const int min_ties = exact_statistics_always() ? INT_MIN : kExactStatsTies;
-  order_reset_kernel<<<dim3(1, n), 32, 0, stream>>>(b);
-  const int g1 = grid_x(1);
-  order_init_kernel<<<dim3(g1, n), kRoundThreads, 0, stream>>>(b, min_ties);
-  for (int r = rounds_for(b.maxN); r > 0; --r) {
-    round_count_kernel<<<dim3(g1, n), kRoundThreads, 0, stream>>>(b, 0, 1);
-    round_lists_kernel<<<dim3(g1, n), kRoundThreads, 0, stream>>>(b, 0, 1);
-    round_swap_kernel<<<dim3(g1, n), kRoundThreads, 0, stream>>>(b, 0, 1);
-  }
-  order_finish_kernel<<<dim3(1, n), kOrdThreads, smem_sel, stream>>>(b, 0, min_ties);
-  const int g2 = grid_x(2);
-  for (int r = rounds_for(b.maxN / 2 + 1); r > 0; --r) {
-    round_count_kernel<<<dim3(g2, 2 * n), kRoundThreads, 0, stream>>>(b, 1, 2);
-    round_lists_kernel<<<dim3(g2, 2 * n), kRoundThreads, 0, stream>>>(b, 1, 2);
-    round_swap_kernel<<<dim3(g2, 2 * n), kRoundThreads, 0, stream>>>(b, 1, 2);
-  }
-  order_finish_kernel<<<dim3(2, n), kOrdThreads, smem_sel, stream>>>(b, 1, min_ties);
-  order_moments_kernel<<<dim3(1, n), kOrdThreads, smem_sum, stream>>>(b, min_ties);
+  const int smem = (int)(sizeof(float) * kSmemRange + sizeof(int) * 4 * kSmemPairs);
+  static_assert(sizeof(float) * kSumBuf + 1024 * sizeof(SumPiece) <= sizeof(float) * kSmemRange + sizeof(int) * 4 * kSmemPairs,
+                "the sum's buffers fit the selection's");
+  cudaError_t e = cudaFuncSetAttribute(order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  order_kernel<<<dim3(kOrderCluster, b.count), kOrdThreads, smem, stream>>>(b, min_ties);
   return cudaGetLastError();
 }
 
@@ -1366,8 +1349,9 @@ void set_exact_statistics_always(bool always) { g_exact_always.store(always); }
 bool exact_statistics_always() { return g_exact_always.load(); }
 
 cudaError_t search_stats_batch(const SearchBatch& b, int num_sms, cudaStream_t stream) {
-  cudaError_t e = search_stats_emulated(b, num_sms, stream);
-  if (e == cudaSuccess) e = search_stats_exact(b, num_sms, stream);
+  const int min_ties = exact_statistics_always() ? INT_MIN : kExactStatsTies;
+  cudaError_t e = search_stats_emulated(b, num_sms, min_ties, stream);
+  if (e == cudaSuccess) e = search_stats_exact(b, min_ties, stream);
   return e;
 }
 

@@ -67,7 +67,7 @@ struct Planned {
 }  // namespace
 
 struct sc_dd_pool {
-  int device = 0, num_sms = 148, n_partials = 0;
+  int device = 0, num_sms = 148;
   size_t budget = 0;
   char* arena = nullptr;
   size_t arena_bytes = 0;
@@ -331,7 +331,6 @@ int sc_dd_pool_create(size_t scratch_budget_bytes, sc_dd_pool** out) {
     delete p;
     return pcuda(e, "sc_dd_pool_create");
   }
-  p->n_partials = 2 * p->num_sms;
   p->budget = scratch_budget_bytes;
   *out = p;
   return SC_DD_OK;
@@ -379,12 +378,9 @@ size_t sc_dd_request_scratch_bytes(const sc_dd_request* r) {
   if (w < 1) return 0;
   const long long nwin = ((long long)r->num_channels + w - 1) / w;
   const int cap = (int)std::min<long long>(nwin + 1, r->num_channels / 2 + 2);
-  int sms = 148;
-  int dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int elem = r->precision == SC_DD_PRECISION_BF16 ? scb::kElemBF16
                    : r->precision == SC_DD_PRECISION_FP16 ? scb::kElemF16 : scb::kElemF32;
-  return scb::ExecSearch::scratch_bytes(Tr, r->num_channels, cap, 2 * sms, elem);
+  return scb::ExecSearch::scratch_bytes(Tr, r->num_channels, cap, elem);
 }
 
 int sc_dd_pool_search(sc_dd_pool* p, const sc_dd_request* reqs, int count, sc_dd_hit* out, int capacity,
@@ -425,7 +421,7 @@ int sc_dd_pool_search(sc_dd_pool* p, const sc_dd_request* reqs, int count, sc_dd
     pl.min_drift = r.min_drift;
     pl.beam = r.beam;
     pl.coarse = r.coarse_channel;
-    pl.bytes = scb::ExecSearch::scratch_bytes(q.Tr, q.N, q.cand_cap, p->n_partials, q.elem);
+    pl.bytes = scb::ExecSearch::scratch_bytes(q.Tr, q.N, q.cand_cap, q.elem);
   }
   // Admission: consecutive requests while their scratch fits the budget (at least one).
   size_t arena_need = 0, lvl_need = 0;
@@ -458,7 +454,7 @@ int sc_dd_pool_search(sc_dd_pool* p, const sc_dd_request* reqs, int count, sc_dd
     size_t off = 0;
     uint64_t key = 1469598103934665603ull;
     for (Planned& pl : sub) {
-      pl.es.carve(p->arena + off, p->n_partials);
+      pl.es.carve(p->arena + off);
       off += pl.bytes;
       const sc_dd_request& r = reqs[sb.first + (&pl - sub.data())];
       key = fnv(key, &r, sizeof(r));
