@@ -241,6 +241,10 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
       cudaStream_t st = lane ? side->stream[lane - 1] : stream;
       float* la = lane ? side->lvl_a[lane - 1] : lvl_a;
       float* lb = lane ? side->lvl_b[lane - 1] : lvl_b;
+      // Searches that run one after another take every pair, which lie side by side: a search of
+      // many drift blocks then needs a pass per eight of them, not per two (60 x 100003, 36 drift
+      // blocks: levels 0.68 -> 0.46 ms).
+      if (lanes == 1 && side && side->n > 0) lb = la + (lvl_b - lvl_a) * (1 + side->n);
       if (ss[k].elem != kElemF32) {
         if ((e = levels_search(ss[k].norm16, ss[k].N, ss[k].Tr, ss[k].N, ss[k].dmin, ss[k].dmax, la, lb, ss[k].top16,
                                num_sms, st, LevelPlan{}, ss[k].elem, header_status(ss[k]))) != cudaSuccess)

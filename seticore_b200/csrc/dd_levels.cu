@@ -342,11 +342,13 @@ cudaError_t stripes_search(const float* input, long long row_stride, int Tr, int
   const long long budget = l2 > 0 ? std::min(l2, cap) : cap;
   // Drift blocks per pass (J) and stripe length (L).  Whole-row mode: the fewest passes,
   // ceil(ndb / J) x stripes, counting a narrow remainder stripe as a full pass (each pass
-  // costs a launch's fill and drain), the larger J on a tie, and stripes of equal length.
-  // With an L2 budget: the largest J whose stripes span at least four stripe units.
+  // costs a launch's fill and drain), the larger J on a tie, and stripes of equal length.  Every
+  // J is looked at: 36 drift blocks of 64 x 100003 take five whole-row passes of eight (0.46
+  // ms), where halving alone offered only stripes (0.51 ms).
+  // With an L2 budget: the largest J, by halving, whose stripes span at least four stripe units.
   int J = 0;
   long long L = 0, best_passes = -1;
-  for (int j = std::min(ndb, std::min(kMaxBatch, level_max_chunk()));; j = (j + 1) / 2) {
+  for (int j = std::min(ndb, std::min(kMaxBatch, level_max_chunk()));; j = l2 > 0 ? (j + 1) / 2 : j - 1) {
     const long long avail = budget / ((long long)j * Tr) - stripe_row_length(0, j, fr);
     long long lj = 0, stripes = 0;
     if (avail >= Nt) {

@@ -9,8 +9,8 @@
 //      blocks of the chunk: row t covers channels [x0 + d0*t, x0 + d1*t + W + R - 1).
 //      This trapezoid lives in shared memory; each input value is read from HBM/L2 once
 //      per chunk instead of once per drift block.  Float rows arrive by one bulk async copy
-//      per row (the TMA engine's cp.async.bulk, completing on an mbarrier) with the ragged
-//      edges filled by the threads; 16-bit rows arrive raw the same way, in the second half
+//      per row (the TMA engine's cp.async.bulk, completing on an mbarrier; each row from its own
+//      16-byte phase) with the ragged edges filled by the threads; 16-bit rows arrive raw the same way, in the second half
 //      of the tile, and are converted to float in place.
 //   2. Each warp takes (drift block, offset part) units: all offsets of the block for up
 //      to 16 rows, one of two halves for 32 rows, and halves in the short-strip form.
@@ -50,14 +50,6 @@
 #include "dd_internal.h"
 
 namespace scb {
-
-// 16-byte asynchronous global->shared copy (LDGSTS); src_bytes 0 writes zeros and reads
-// nothing.  Both addresses must be 16-byte aligned.
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, int src_bytes) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gsrc), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Bulk (TMA) row copies for float rows: one cp.async.bulk per staged row, completing on a
 // shared-memory mbarrier.  Both addresses must be 16-byte aligned and the size a multiple
@@ -382,21 +374,22 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
         item_tile = tile_i;
       }
       {
-        // Row layout: row t of segment g holds global channels [as, as + wpad), as aligned
-        // down to V elements; the sheared window of job k (in a shared trapezoid) starts k*t
-        // further.  Rows are packed in (segment, row) order: offsets by a warp scan.
+        // Row layout: row t of segment g holds global channels [as, as + wpad), where as is the
+        // window's start moved down to the row's last 16-byte boundary: V elements apart, and
+        // each row has its own phase, so that rows of any stride and base take the bulk copies
+        // (with one phase for all, a row stride that is not a multiple of four floats sent every
+        // row through per-thread loads, a memory latency per row: 60 x 100003 with such rows,
+        // 1163 -> 900 us a search).  The sheared window of job k (in a
+        // shared trapezoid) starts k*t further.  Rows are packed in (segment, row) order:
+        // offsets by a warp scan.
         const int k0w = (local - lt * pg.n_chunks) * pg.jobs_per_chunk;
         const int njw = min(pg.jobs_per_chunk, pg.n_jobs - k0w);
         const bool shared_w = (pg.job_row_stride == 0);
         const int nsegw = shared_w ? 1 : njw;
         const int extra = shared_w ? (njw - 1) * pg.d_step : 0;
         const long long x0w = (long long)tile_i * W;
-        // Float rows whose base, row stride and job stride are 16-byte aligned take bulk
-        // copies for their in-range 16-byte chunks.
-        // 16-bit rows land raw in the second half of the tile and are converted in place.
-        const bool bulk_ok = ((reinterpret_cast<uintptr_t>(pg.rows) & 15) == 0) && ((pg.row_stride % V) == 0) &&
-                             ((pg.job_row_stride % V) == 0);
-        const long long n_full = (long long)(pg.N / V) * V;  // channels in whole 16-byte chunks
+        // The in-range 16-byte chunks of a row take bulk copies; 16-bit rows land raw in the
+        // second half of the tile and are converted in place.
         unsigned tx = 0;
         int off = 0;
         for (int e0 = 0; e0 < nsegw * R; e0 += 32) {
@@ -409,7 +402,10 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
           if (valid) {
             const long long dg = (long long)pg.d_first + (long long)(k0w + gg) * pg.d_step;
             const long long gs = x0w + dg * t;
-            as = floor_div(gs, V) * V;
+            const long long at = (long long)(reinterpret_cast<uintptr_t>(pg.rows) / sizeof(E)) +
+                                 (long long)(k0w + gg) * pg.job_row_stride + (long long)t * pg.row_stride;
+            const int m = (int)(at & (V - 1));  // channel 0's place in its 16-byte chunk
+            as = floor_div(gs + m, V) * V - m;
             a = (int)(gs - as);
             wpad = (a + W + LEAD + extra * t + V - 1) / V * V;
           }
@@ -425,9 +421,11 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
             geo_win[gg][t] = at + a;
             geo_wid[gg][t] = wpad;
             geo_start[gg][t] = as;
-            const long long b_lo = as > -pg.pad ? as : -pg.pad;  // rows hold data from -pad on
-            const long long b_hi = as + wpad < n_full ? as + wpad : n_full;
-            const bool bulk = bulk_ok && b_hi > b_lo;
+            // whole chunks inside [-pad, N) (rows hold data from -pad on)
+            const long long b_lo = as >= -pg.pad ? as : as + (-pg.pad - as + V - 1) / V * V;
+            const long long end = as + wpad < pg.N ? as + wpad : pg.N;
+            const long long b_hi = end > as ? as + (end - as) / V * V : as;
+            const bool bulk = b_hi > b_lo;
             geo_blo[gg][t] = bulk ? (int)(b_lo - as) : 0;
             geo_bhi[gg][t] = bulk ? (int)(b_hi - as) : 0;
             if (bulk) tx += (unsigned)(b_hi - b_lo) * (unsigned)sizeof(E);
@@ -468,8 +466,6 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
     __syncthreads();
     const TreeGroup& p = tb.g[item_group];
     const E* rows = static_cast<const E*>(p.rows);
-    const bool vec_ok = ((reinterpret_cast<uintptr_t>(rows) & 15) == 0) && ((p.row_stride % V) == 0) &&
-                        ((p.job_row_stride % V) == 0);
     const int local = item - p.item_begin;
     const int tile_idx = item_tile;
     const int chunk = local - (local / p.n_chunks) * p.n_chunks;
@@ -493,13 +489,7 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
             const int j = q < n_left ? q * V : bhi + (q - n_left) * V;
             const long long c = as + j;
             float* d = dst + j;
-            if (vec_ok && c >= -p.pad && c + V - 1 < p.N) {
-              cp_async16(d, src + c, 16);  // whole chunk in range
-            } else if (vec_ok && (c + V - 1 < -p.pad || c >= p.N)) {
-              cp_async16(d, src, 0);  // whole chunk out of range: zero fill, nothing read
-            } else {
-              for (int i = 0; i < V; ++i) d[i] = (c + i >= -p.pad && c + i < p.N) ? src[c + i] : 0.0f;
-            }
+            for (int i = 0; i < V; ++i) d[i] = (c + i >= -p.pad && c + i < p.N) ? src[c + i] : 0.0f;
           }
         }
       }
@@ -550,66 +540,22 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
               const int j = q < n_left ? q * V : bhi + (q - n_left) * V;
               const long long c = as + j;
               float* d = dst + j;
-              if (vec_ok && c >= 0 && c + V - 1 < p.N) {
-                const uint4 w = __ldg(reinterpret_cast<const uint4*>(src + c));
-                const E* h = reinterpret_cast<const E*>(&w);
-                reinterpret_cast<float4*>(d)[0] =
-                    make_float4(to_float(h[0]), to_float(h[1]), to_float(h[2]), to_float(h[3]));
-                reinterpret_cast<float4*>(d)[1] =
-                    make_float4(to_float(h[4]), to_float(h[5]), to_float(h[6]), to_float(h[7]));
-              } else {
-                for (int i = 0; i < V; ++i) d[i] = (c + i >= 0 && c + i < p.N) ? to_float(src[c + i]) : 0.0f;
-              }
+              for (int i = 0; i < V; ++i) d[i] = (c + i >= 0 && c + i < p.N) ? to_float(src[c + i]) : 0.0f;
             }
           }
         }
       }
     } else {
-      // 16-bit rows that no bulk copy can take (unaligned), converted to float as they are
-      // staged: a thread loads its 16-byte chunks (eight values) of G rows before converting
-      // any, so those loads are in flight together (two rows at a time for 32 rows, whose tree
-      // already fills the registers).
-      constexpr int G = R >= 32 ? 2 : 4;
-      for (int g = 0; g < nseg; ++g) {
-        const E* seg = rows + (long long)(k0 + g) * p.job_row_stride;
-        for (int t0 = 0; t0 < R; t0 += G) {
-          int maxq = 0;
-          for (int u = 0; u < G && t0 + u < R; ++u) maxq = max(maxq, geo_wid[g][t0 + u] / V);
-          for (int q = threadIdx.x; q < maxq; q += blockDim.x) {
-            uint4 raw[G];
-            bool full[G];
-#pragma unroll
-            for (int u = 0; u < G; ++u) {
-              const int t = t0 + u;
-              full[u] = false;
-              if (t < R && q < geo_wid[g][t] / V) {
-                const long long c = geo_start[g][t] + (long long)q * V;
-                full[u] = vec_ok && c >= 0 && c + V - 1 < p.N;
-                if (full[u]) raw[u] = __ldg(reinterpret_cast<const uint4*>(seg + (long long)t * p.row_stride + c));
-              }
-            }
-#pragma unroll
-            for (int u = 0; u < G; ++u) {
-              const int t = t0 + u;
-              if (t >= R || q >= geo_wid[g][t] / V) continue;
-              const long long c = geo_start[g][t] + (long long)q * V;
-              float* d = tile + geo_base[g][t] + q * V;
-              if (full[u]) {
-                const E* h = reinterpret_cast<const E*>(&raw[u]);
-                reinterpret_cast<float4*>(d)[0] =
-                    make_float4(to_float(h[0]), to_float(h[1]), to_float(h[2]), to_float(h[3]));
-                reinterpret_cast<float4*>(d)[1] =
-                    make_float4(to_float(h[4]), to_float(h[5]), to_float(h[6]), to_float(h[7]));
-              } else {
-                const E* src = seg + (long long)t * p.row_stride;
-                for (int i = 0; i < V; ++i) d[i] = (c + i >= 0 && c + i < p.N) ? to_float(src[c + i]) : 0.0f;
-              }
-            }
-          }
+      // 16-bit rows without a whole chunk in range: zeros and a few ragged values.
+      for (int e = warp; e < nseg * R; e += nwarps) {
+        const int g = e / R, t = e - g * R;
+        const E* src = rows + (long long)(k0 + g) * p.job_row_stride + (long long)t * p.row_stride;
+        for (int i = lane; i < geo_wid[g][t]; i += kWarp) {
+          const long long c = geo_start[g][t] + i;
+          tile[geo_base[g][t] + i] = (c >= 0 && c < p.N) ? to_float(src[c]) : 0.0f;
         }
       }
     }
-    cp_async_wait_all();
     if (item_tx && !stage_waited) {
       if (!mbar_wait(&stage_bar, stage_phase, tb.stage_wait_tries >= 0 ? tb.stage_wait_tries : kStageWaitTries))
         stage_failed = 1;
