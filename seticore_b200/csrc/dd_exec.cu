@@ -225,36 +225,52 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
     // searches are dealt round-robin over the main stream and the side streams, when there are
     // any (two concurrent 16-bit level searches measured slower than one after the other: their
     // first level is bound by L1 throughput, not by latency); the 16-bit searches run it on
-    // their normalised copy, with the default split, on the main stream.
+    // their normalised copy, with the default split, on the main stream.  A search that is alone,
+    // or wide (below), runs on the main stream with every pair, which lie side by side: a search
+    // of many drift blocks then needs a pass per eight of them, not per two (60 x 100003, 36
+    // drift blocks: levels 0.68 -> 0.46 ms).
+    const long long half = lvl_b - lvl_a;
+    const int pairs = side && side->n > 0 ? 1 + side->n : 1;
+    // Wide: its drift blocks do not fit one pass of its own pair, and a pass of all pairs fills
+    // the GPU for long enough (128 MB of planes) that the launches' ends do not matter.  Eight
+    // searches each: 256 x 131072, 4 drift blocks 2195 -> 2007 us; 128 x 131072, 10 drift blocks
+    // 2628 -> 2317; 4 of 64 x 2^20, 8 drift blocks 3948 -> 3482.  But 16 of 64 x 32768, 8 drift
+    // blocks: 573 side by side and 618 one by one; 256 x 131072, 2 drift blocks: 1112 and 1202.
+    auto wide = [&](const ExecSearch& q) {
+      const long long per_db = (long long)q.Tr * (level_row_length(q.N) + kLevelRowSlack), ndb = q.dmax - q.dmin + 1;
+      return pairs > 1 && ndb * per_db > 2 * half &&
+             std::min<long long>(ndb, 2 * half * pairs / per_db) * per_db * (long long)sizeof(float) >= (128ll << 20);
+    };
+    auto level = [&](const ExecSearch& q, float* la, float* lb, cudaStream_t st) {
+      const LevelPlan plan = hooks.level_plan ? hooks.level_plan(hooks.ctx, q, la, lb, st) : q.level_plan;
+      return levels_search(q.input, q.row_stride, q.Tr, q.N, q.dmin, q.dmax, la, lb, q.top, num_sms, st, plan, kElemF32,
+                           header_status(q));
+    };
     int n_level = 0;
-    for (int k = 0; k < m; ++k) n_level += ss[k].Tr > 32 && ss[k].elem == kElemF32;
-    const int lanes = (side && side->n > 0 && n_level >= 2) ? 1 + std::min(side->n, n_level - 1) : 1;
+    for (int k = 0; k < m; ++k) n_level += ss[k].Tr > 32 && ss[k].elem == kElemF32 && !wide(ss[k]);
+    const int lanes = pairs > 1 && n_level >= 2 ? std::min(pairs, n_level) : 1;
+    for (int k = 0; k < m; ++k) {  // the main stream's searches, before the side streams start
+      const ExecSearch& q = ss[k];
+      if (q.Tr <= 32) continue;
+      if (q.elem != kElemF32)
+        e = levels_search(q.norm16, q.N, q.Tr, q.N, q.dmin, q.dmax, lvl_a, lvl_b, q.top16, num_sms, stream, LevelPlan{},
+                          q.elem, header_status(q));
+      else if (lanes == 1 || wide(q))
+        e = level(q, lvl_a, lvl_a + half * pairs, stream);
+      if (e != cudaSuccess) return e;
+    }
     if (lanes > 1) {
       if ((e = cudaEventRecord(side->fork, stream)) != cudaSuccess) return e;
       for (int i = 0; i + 1 < lanes; ++i)
         if ((e = cudaStreamWaitEvent(side->stream[i], side->fork, 0)) != cudaSuccess) return e;
-    }
-    int j = 0;
-    for (int k = 0; k < m; ++k) {
-      if (ss[k].Tr <= 32) continue;
-      const int lane = (lanes > 1 && ss[k].elem == kElemF32) ? (j++ % lanes) : 0;  // 0: the main stream
-      cudaStream_t st = lane ? side->stream[lane - 1] : stream;
-      float* la = lane ? side->lvl_a[lane - 1] : lvl_a;
-      float* lb = lane ? side->lvl_b[lane - 1] : lvl_b;
-      // Searches that run one after another take every pair, which lie side by side: a search of
-      // many drift blocks then needs a pass per eight of them, not per two (60 x 100003, 36 drift
-      // blocks: levels 0.68 -> 0.46 ms).
-      if (lanes == 1 && side && side->n > 0) lb = la + (lvl_b - lvl_a) * (1 + side->n);
-      if (ss[k].elem != kElemF32) {
-        if ((e = levels_search(ss[k].norm16, ss[k].N, ss[k].Tr, ss[k].N, ss[k].dmin, ss[k].dmax, la, lb, ss[k].top16,
-                               num_sms, st, LevelPlan{}, ss[k].elem, header_status(ss[k]))) != cudaSuccess)
+      int j = 0;
+      for (int k = 0; k < m; ++k) {
+        if (ss[k].Tr <= 32 || ss[k].elem != kElemF32 || wide(ss[k])) continue;
+        const int lane = j++ % lanes;  // 0: the main stream
+        if ((e = lane ? level(ss[k], side->lvl_a[lane - 1], side->lvl_b[lane - 1], side->stream[lane - 1])
+                      : level(ss[k], lvl_a, lvl_b, stream)) != cudaSuccess)
           return e;
-        continue;
       }
-      const LevelPlan plan = hooks.level_plan ? hooks.level_plan(hooks.ctx, ss[k], la, lb, st) : ss[k].level_plan;
-      if ((e = levels_search(ss[k].input, ss[k].row_stride, ss[k].Tr, ss[k].N, ss[k].dmin, ss[k].dmax, la, lb,
-                             ss[k].top, num_sms, st, plan, kElemF32, header_status(ss[k]))) != cudaSuccess)
-        return e;
     }
     for (int i = 0; i + 1 < lanes; ++i) {
       if ((e = cudaEventRecord(side->join[i], side->stream[i])) != cudaSuccess ||

@@ -226,11 +226,14 @@ struct FoldPair {
 
 // Runs the generated strip code of offset part `part` (PART offsets each); the parts are
 // unrolled at compile time so that each call site names one generated function.
+constexpr int kPacked = -1;  // as RELOAD: the packed form (both halves of the tree in float2 adds)
 template <int R, int PART, int U, int ITERS, int RELOAD, int P = 0, typename Row, typename Fold>
 __device__ __forceinline__ void strip_part(int part, const Row (&row)[R], float* mrow, const Fold& fold) {
   if constexpr (P * PART < R) {
-    if (part == P) taylor_strip_loop<R, P * PART, P * PART + PART, U, ITERS, RELOAD>(row, mrow, fold);
-    else strip_part<R, PART, U, ITERS, RELOAD, P + 1>(part, row, mrow, fold);
+    if (part == P) {
+      if constexpr (RELOAD == kPacked) taylor_strip_x2<R, P * PART, P * PART + PART, U, ITERS>(row, mrow, fold);
+      else taylor_strip_loop<R, P * PART, P * PART + PART, U, ITERS, RELOAD>(row, mrow, fold);
+    } else strip_part<R, PART, U, ITERS, RELOAD, P + 1>(part, row, mrow, fold);
   }
 }
 
@@ -643,9 +646,9 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
         BufferSink<W> sink{static_cast<unsigned>(__cvta_generic_to_shared(ebuf)) + 4u * (unsigned)(lane * S)};
         if constexpr (NPARTS == 1) {
           taylor_strip_emit<R, 0, R, kU, ITERS>(row, sink);
-        } else {
-          if (part == 0) taylor_strip_emit<R, 0, PART, kU, ITERS>(row, sink);
-          else taylor_strip_emit<R, PART, R, kU, ITERS>(row, sink);
+        } else {  // two halves: the packed form
+          if (part == 0) taylor_strip_emit_x2<R, 0, PART, kU, ITERS>(row, sink);
+          else taylor_strip_emit_x2<R, PART, R, kU, ITERS>(row, sink);
         }
         // Order the buffer's generic-proxy writes before the async-proxy reads of the stores.
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -861,7 +864,9 @@ cudaError_t launch_rows(TreeBatch& b, int R, int num_sms, size_t budget, cudaStr
   switch (R) {
     case 2: return launch_tree<E, 2, 1, S>(b, num_sms, budget, stream);
     case 4: return launch_tree<E, 4, 1, S>(b, num_sms, budget, stream);
-    case 8: return launch_tree<E, 8, 1, S>(b, num_sms, budget, stream);
+    case 8:
+      return launch_tree<E, 8, 1, S, false, 8, 1, (S == kU && std::is_same<E, float>::value ? kPacked : 0)>(
+          b, num_sms, budget, stream);
     case 16:
       // Long strips: all 16 offsets in one warp, which loads most leaves once per drift block
       // (two offset halves load every leaf twice; shared-memory bandwidth bounded that form).
@@ -874,7 +879,15 @@ cudaError_t launch_rows(TreeBatch& b, int R, int num_sms, size_t budget, cudaStr
         return launch_tree<E, 16, 1, S, false, 8, 2, (std::is_same<E, float>::value ? 12 : 8)>(b, num_sms, budget, stream);
       // Short strips (the last level of a tree of more than 32 rows, one job of two offset
       // halves per CTA): capped at 128 registers, eight such CTAs share an SM (six at the
-      // 134 registers the compiler picks unbounded; 5 % slower on 256-row beams).
+      // 134 registers the compiler picks unbounded; 5 % slower on 256-row beams).  Float planes
+      // take the packed form, and so does the first level: fewer instructions per channel where
+      // neither the adds' pipes nor the loads are the limit (32 beams of 256 rows, both levels:
+      // 4.56 -> 4.36 ms; ten or twelve CTAs per SM at 96 or 80 registers: 4.41, 4.45).  The long
+      // strips keep the single-float form: packed, their 16-row tree issues 21 % fewer
+      // instructions but needs 168 registers, so twelve warps per SM (16 searches of 2^20
+      // channels: 3.55 against 3.50 ms; at 128 registers it spills, 3.69).
+      else if constexpr (std::is_same<E, float>::value)
+        return launch_tree<E, 16, 2, S, false, 2, 8, kPacked>(b, num_sms, budget, stream);
       else return launch_tree<E, 16, 2, S, false, 2, 8>(b, num_sms, budget, stream);
     default: return cudaErrorInvalidValue;
   }

@@ -202,6 +202,167 @@ def gen_strip_loop(R, lo, hi, U, ITERS, emit=False, reload=0, h2=False):
             f"    const Row (&row)[{R}], float* __restrict__ mrow, const Fold& fold) {{\n{body_text}\n}}\n")
 
 
+def gen_strip_x2(R, lo, hi, U, ITERS, emit=False):
+    """The strip function with the tree's two halves packed: node (L, b, o) of the upper R/2 rows and
+    the same node of the lower R/2 rows sit in one float2, so one paired add (__fadd2_rn, two
+    IEEE float adds) does both; only the root level adds single floats.
+
+    The two halves of a root meet at different channels, node q of the upper half at s with node q
+    of the lower at s + q and s + q + 1.  The lower half runs K = hi/2 channels ahead of the
+    upper one, so every packed node q is made at the same step s, its upper half is used at once
+    and only its lower half is kept, for K - q steps: sum(K - q) single registers instead of
+    a window for every node of a lagging half.  A pair of 8-row trees with all its windows then
+    takes 124 registers of state and 16 loads per channel where the single-float form of 16 rows
+    takes 208.
+
+    The prologue makes, before step 0, the lower halves of the steps -K .. -1 (single floats: the
+    upper halves would be wasted) and the windows of the packed nodes."""
+    H = R // 2
+    qs = list(range(lo // 2, hi // 2))
+    assert lo % 2 == 0 and hi % 2 == 0 and U >= len(qs)
+    K = hi // 2
+    # packed nodes: positions at which they are consumed, relative to the step
+    pos = {(H, 0, q): {0} for q in qs}
+    L = H
+    while L > 1:
+        for (LL, b, o), P in list(pos.items()):
+            if LL == L:
+                sh = (o + 1) // 2
+                pos.setdefault((L // 2, 2 * b, o // 2), set()).update(P)
+                pos.setdefault((L // 2, 2 * b + 1, o // 2), set()).update(x + sh for x in P)
+        L //= 2
+    win = {k: (min(P), max(P)) for k, P in pos.items()}
+
+    def nm(k):
+        return "_".join(str(x) for x in k)
+
+    def num(j):
+        return str(j).replace("-", "m")
+
+    def leaf(b, j, base=""):
+        return f"make_float2(row[{b}][{base}{j}], row[{b + H}][{base}{j + K}])"
+
+    def kids(k):
+        L, b, o = k
+        return (L // 2, 2 * b, o // 2), (L // 2, 2 * b + 1, o // 2), (o + 1) // 2
+
+    lines = []
+    for k in sorted(win):
+        mn, ld = win[k]
+        if ld > mn:
+            lines.append(f"  float2 s{nm(k)}[{ld - mn}];")
+    for q in qs:
+        lines.append(f"  float h{q}[{K - q}];")
+    # prologue demands: whole pairs (the windows) and lower halves alone
+    full = {k: set(range(*win[k])) for k in win}
+    low = {k: set() for k in win}
+    for q in qs:
+        low[(H, 0, q)] = set(range(q - K, 0))
+    for k in sorted(win, key=lambda k: -k[0]):
+        if k[0] == 1:
+            continue
+        a, c, sh = kids(k)
+        full[a] |= full[k]
+        full[c] |= {j + sh for j in full[k]}
+        low[a] |= low[k]
+        low[c] |= {j + sh for j in low[k]}
+    pro = []
+    for k in sorted(win):
+        mn, ld = win[k]
+        for j in sorted(full[k] | low[k]):
+            if j in full[k]:
+                if k[0] == 1:
+                    e = leaf(k[1], j)
+                else:
+                    a, c, sh = kids(k)
+                    e = f"__fadd2_rn(w{nm(a)}_{num(j)}, w{nm(c)}_{num(j + sh)})"
+                pro.append((j - ld, k[0], f"  const float2 w{nm(k)}_{num(j)} = {e};"))
+            else:
+                if k[0] == 1:
+                    e = f"row[{k[1] + H}][{j + K}]"
+                else:
+                    a, c, sh = kids(k)
+
+                    def half(x, jj):
+                        return f"w{nm(x)}_{num(jj)}.y" if jj in full[x] else f"y{nm(x)}_{num(jj)}"
+                    e = f"{half(a, j)} + {half(c, j + sh)}"
+                pro.append((j - ld, k[0], f"  const float y{nm(k)}_{num(j)} = {e};"))
+    pro.sort(key=lambda x: (x[0], x[1]))
+    lines += [t for _, _, t in pro]
+    for k in sorted(win):
+        mn, ld = win[k]
+        for j in range(mn, ld):
+            lines.append(f"  s{nm(k)}[{j - mn}] = w{nm(k)}_{num(j)};")
+    for q in qs:
+        for j in range(q - K, 0):
+            k = (H, 0, q)
+            lines.append(f"  h{q}[{j - (q - K)}] = " + (f"w{nm(k)}_{num(j)}.y;" if j in full[k] else f"y{nm(k)}_{num(j)};"))
+    lines.append("#pragma unroll 1")
+    lines.append(f"  for (int it = 0; it < {ITERS}; ++it) {{")
+    lines.append(f"    const int base = it * {U};")
+
+    def at(k, j):
+        mn, ld = win[k]
+        return f"s{nm(k)}[{j - mn}]" if j < ld else f"v{nm(k)}_{num(j)}"
+
+    def lower(q, j):
+        return f"v{nm((H, 0, q))}_{j}.y" if j >= 0 else f"h{q}[{j - (q - K)}]"
+
+    body = []
+    for k in sorted(win):
+        mn, ld = win[k]
+        for j in range(ld, U + ld):
+            if k[0] == 1:
+                e = leaf(k[1], j, "base + ")
+            else:
+                a, c, sh = kids(k)
+                e = f"__fadd2_rn({at(a, j)}, {at(c, j + sh)})"
+            body.append((j - ld, k[0], f"    const float2 v{nm(k)}_{num(j)} = {e};"))
+    for st in range(U):
+        if emit:
+            for i, q in enumerate(qs):
+                up = f"v{nm((H, 0, q))}_{st}.x"
+                for d in (0, 1):
+                    body.append((st, R, f"    sink.put({2 * i + d}, base + {st}, {up} + {lower(q, st + q - K + d)});"))
+            continue
+        # Offsets 2q and 2q + 1 share their upper half: their larger sum is upper + max(lower at +q,
+        # lower at +q + 1), exactly (rounding is monotonic, and a NaN sum never counts).
+        for q in qs:
+            up = f"v{nm((H, 0, q))}_{st}.x"
+            body.append((st, R, f"    const float o{st}_{q} = {up} + fmaxf({lower(q, st + q - K)}, {lower(q, st + q - K + 1)});"))
+        acc = "0.0f"
+        for i in range(0, len(qs), 2):
+            if i + 1 < len(qs):
+                e = f"fmax3({acc}, o{st}_{qs[i]}, o{st}_{qs[i + 1]})"
+            else:
+                e = f"fmaxf({acc}, o{st}_{qs[i]})"
+            acc = f"m{st}_{i}"
+            body.append((st, R + 1, f"    const float {acc} = {e};"))
+        body.append((st, R + 2, f"    fold(mrow, base + {st}, {acc});"))
+    body.sort(key=lambda x: (x[0], x[1]))
+    lines += [t for _, _, t in body]
+    for k in sorted(win):
+        mn, ld = win[k]
+        for j in range(ld - mn):
+            lines.append(f"    s{nm(k)}[{j}] = {at(k, U + mn + j)};")
+    for q in qs:
+        for j in range(K - q):
+            lines.append(f"    h{q}[{j}] = {lower(q, U + (q - K) + j)};")
+    lines.append("  }")
+    text = "\n".join(lines)
+    if emit:
+        return (f"template <typename Row, typename Sink>\n__device__ __forceinline__ void "
+                f"{x2_name(R, lo, hi, U, ITERS, True)}(\n"
+                f"    const Row (&row)[{R}], Sink& sink) {{\n{text}\n}}\n")
+    return (f"template <typename Row, typename Fold>\n__device__ __forceinline__ void "
+            f"{x2_name(R, lo, hi, U, ITERS)}(\n"
+            f"    const Row (&row)[{R}], float* __restrict__ mrow, const Fold& fold) {{\n{text}\n}}\n")
+
+
+def x2_name(R, lo, hi, U, ITERS, emit=False):
+    return f"taylor_strip_{'emit_' if emit else ''}x2_{R}_{lo}_{hi}_{U}_{ITERS}"
+
+
 def loop_name(R, lo, hi, U, ITERS, reload=0, h2=False):
     return (f"taylor_strip_loop{'_h2' if h2 else ''}_{R}_{lo}_{hi}_{U}_{ITERS}" +
             (f"_r{reload}" if reload else ""))
@@ -264,6 +425,13 @@ LOOP_CONFIGS = [(2, 1, 11, 3), (4, 1, 11, 3), (8, 1, 11, 3), (16, 1, 11, 3, 12),
                 (2, 1, 11, 1), (4, 1, 11, 1), (8, 1, 11, 1), (16, 2, 11, 1)]
 
 
+# (R, offset parts, U, iterations) of the packed form (both halves of the tree in float2 adds): the
+# last levels of a tree of more than 32 rows.
+X2_CONFIGS = [(16, 2, 11, 1), (8, 1, 11, 1)]
+# (R, offset parts, U, iterations) of its emitting form.
+X2_EMIT_CONFIGS = [(16, 2, 11, 1)]
+
+
 # (R, offset parts, U, iterations, reload) of the paired-FP16 form (two drift blocks per lane,
 # the 16-bit forms' 16- and 32-row trees).
 H2_CONFIGS = [(16, 1, 11, 3, 12), (16, 1, 11, 3, 10), (32, 2, 11, 3, 0)]
@@ -294,6 +462,15 @@ def main(out_path):
         for k in range(nparts):
             parts.append(gen_strip_loop(R, k * step, (k + 1) * step, U, IT, reload=rl, h2=True))
 
+    for R, nparts, U, IT in X2_CONFIGS:
+        step = R // nparts
+        for k in range(nparts):
+            parts.append(gen_strip_x2(R, k * step, (k + 1) * step, U, IT))
+    for R, nparts, U, IT in X2_EMIT_CONFIGS:
+        step = R // nparts
+        for k in range(nparts):
+            parts.append(gen_strip_x2(R, k * step, (k + 1) * step, U, IT, emit=True))
+
     # Dispatcher: taylor_strip_loop<R, LO, HI, U, ITERS, RELOAD>(row, mrow, fold) for any element
     # accessor and fold (which merges a channel's maximum: all channels, or a range of them).
     parts.append("template <int R, int LO, int HI, int U, int ITERS, int RELOAD = 0, typename Row, typename Fold>\n"
@@ -316,6 +493,25 @@ def main(out_path):
             lo, hi = k * step, (k + 1) * step
             parts.append(f"  if constexpr (R == {R} && LO == {lo} && HI == {hi} && U == {U} && ITERS == {IT} && "
                          f"RELOAD == {rel}) {loop_name(R, lo, hi, U, IT, rel, True)}(row, mrow, fold);")
+    parts.append("}")
+    parts.append("template <int R, int LO, int HI, int U, int ITERS, typename Row, typename Fold>\n"
+                 "__device__ __forceinline__ void taylor_strip_x2(const Row (&row)[R], float* __restrict__ mrow, "
+                 "const Fold& fold) {")
+    for R, nparts, U, IT in X2_CONFIGS:
+        step = R // nparts
+        for k in range(nparts):
+            lo, hi = k * step, (k + 1) * step
+            parts.append(f"  if constexpr (R == {R} && LO == {lo} && HI == {hi} && U == {U} && ITERS == {IT}) "
+                         f"{x2_name(R, lo, hi, U, IT)}(row, mrow, fold);")
+    parts.append("}")
+    parts.append("template <int R, int LO, int HI, int U, int ITERS, typename Row, typename Sink>\n"
+                 "__device__ __forceinline__ void taylor_strip_emit_x2(const Row (&row)[R], Sink& sink) {")
+    for R, nparts, U, IT in X2_EMIT_CONFIGS:
+        step = R // nparts
+        for k in range(nparts):
+            lo, hi = k * step, (k + 1) * step
+            parts.append(f"  if constexpr (R == {R} && LO == {lo} && HI == {hi} && U == {U} && ITERS == {IT}) "
+                         f"{x2_name(R, lo, hi, U, IT, True)}(row, sink);")
     parts.append("}")
     parts.append("template <int R, int LO, int HI, int U, int ITERS, typename Row, typename Sink>\n"
                  "__device__ __forceinline__ void taylor_strip_emit(const Row (&row)[R], Sink& sink) {")
