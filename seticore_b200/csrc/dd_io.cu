@@ -42,10 +42,21 @@ __global__ void gather_kernel(const float* __restrict__ in, long long row_stride
   const int k = blockIdx.x;
   const int b = ranges[2 * k], w = ranges[2 * k + 1] - ranges[2 * k];
   float* o = out + offsets[k];
-  const long long n = (long long)T * w;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-    const long long t = i / w;
-    o[i] = __ldg(in + t * row_stride + b + (i - t * w));
+  // A warp per row, four columns per lane in flight.
+  constexpr int K = 4;
+  const int lane = threadIdx.x & 31;
+  for (int t = threadIdx.x >> 5; t < T; t += blockDim.x >> 5) {
+    const float* __restrict__ src = in + t * row_stride + b;
+    float* dst = o + (long long)t * w;
+    for (int c0 = lane; c0 < w; c0 += 32 * K) {
+      float v[K];
+#pragma unroll
+      for (int q = 0; q < K; ++q)
+        if (c0 + 32 * q < w) v[q] = __ldg(src + c0 + 32 * q);
+#pragma unroll
+      for (int q = 0; q < K; ++q)
+        if (c0 + 32 * q < w) dst[c0 + 32 * q] = v[q];
+    }
   }
 }
 
