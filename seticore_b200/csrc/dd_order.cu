@@ -57,7 +57,7 @@ constexpr int kMaxSegs = kOrderMaxSegs;  // counting segments per partition step
 constexpr int kSmemRange = 16384;        // ranges of at most this many values run in shared memory
 constexpr int kSmemPairs = kSmemRange / 2 + 1;
 constexpr int kSerialRange = 256;        // ranges of at most this many values are finished by one thread
-constexpr int kOrderCluster = 8;         // CTAs per search
+constexpr int kOrderCluster = 16;        // CTAs per search, at most
 constexpr int kSumSeg = 4096;            // terms per speculative piece of the float sum
 constexpr int kSeqPrefix = 2048;         // leading terms of a sum added one by one (thread 0)
 constexpr int kTermsPerThreadF = 16;     // terms per thread in one scan chunk of a float sum
@@ -75,7 +75,6 @@ struct SumPiece {
 };
 // Shared memory of the kernel beyond the dynamic shared-memory range buffer.
 struct OrdShared {
-  SumPiece piece[kOrdWarps];
   double warp_d[kOrdWarps], warp_d2[kOrdWarps];
   int seg_ge[kMaxSegs + 1];  // per segment: values >= pivot; then their exclusive prefix
   int seg_le[kMaxSegs + 1];  // per segment: values <= pivot; then their exclusive prefix
@@ -260,6 +259,16 @@ struct VChunk {
   }
   // 4-bit masks of this lane's group q: values >= p (ge) and <= p (le) inside [x0, x1).
   __device__ __forceinline__ void masks(int q, int a0, int x0, int x1, float p, unsigned& mg, unsigned& ml) const {
+    if (a0 >= x0 && a0 + kStep <= x1) {  // a whole step inside: no position tests
+      mg = ml = 0u;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float f = at(q, c);
+        mg |= (!(f < p) ? 1u : 0u) << c;
+        ml |= (!(p < f) ? 1u : 0u) << c;
+      }
+      return;
+    }
     const int base = a0 + 128 * q + 4 * (int)(threadIdx.x & 31);
     mg = ml = 0u;
 #pragma unroll
@@ -336,6 +345,16 @@ __device__ void count_segments(const float* a, const Segs& sg, float p, int w0, 
     for (int a0 = sg.start(g); a0 < x1; a0 += kStep) {
       VChunk<GLOBAL> w;
       w.load(a, a0, x0, x1);
+      if (a0 >= x0 && a0 + kStep <= x1) {
+#pragma unroll
+        for (int q = 0; q < kV4; ++q)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            cge += w.at(q, c) < p ? 0 : 1;
+            cle += p < w.at(q, c) ? 0 : 1;
+          }
+        continue;
+      }
 #pragma unroll
       for (int q = 0; q < kV4; ++q) {
         unsigned mg, ml;
@@ -427,51 +446,51 @@ __device__ int scan_and_cut(const float* a, const Segs& sg, float p, OrdShared& 
   return K == 0 ? S.lk : min(S.lk, S.rk);
 }
 
-// 3. The K pairs: positions and values, listed by rank.  seg_ge, seg_le: the prefixes.
+// 3. The K pairs: positions and values, listed by rank.  seg_ge, seg_le: the prefixes.  A warp takes
+// 32 consecutive positions at a time, so the ranks come from two ballots and neighbouring lanes
+// store to neighbouring places (four positions per lane, with scans and scattered stores, took
+// 2.4 times as long on 2^20 values).
 template <bool GLOBAL>
 __device__ void list_pairs(const float* a, const Segs& sg, float p, int K, int total_le, const int* seg_ge,
                            const int* seg_le, int w0, int nw, int* lpos, float* lval, int* rpos, float* rval) {
   const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
   auto pre = [](const int* s, int g) {
     if constexpr (GLOBAL) return __ldcg(s + g);
     else return s[g];
   };
+  constexpr int B = 16;  // loads in flight per lane
   for (int g = w0; g < sg.nseg; g += nw) {
-    int rge = pre(seg_ge, g), rle = pre(seg_le, g);
+    int rge = pre(seg_ge, g), rle = total_le - 1 - pre(seg_le, g);  // the next ranks (from the right for rle)
     if (rge >= K && total_le - pre(seg_le, g + 1) >= K) continue;  // no pair has a value in this segment
     const int x0 = sg.x0(g), x1 = sg.x1(g);
-    for (int a0 = sg.start(g); a0 < x1; a0 += kStep) {
-      VChunk<GLOBAL> w;
-      w.load(a, a0, x0, x1);
+    for (int b0 = x0; b0 < x1; b0 += 32 * B) {
+      float v[B];
 #pragma unroll
-      for (int q = 0; q < kV4; ++q) {
-        unsigned mg, ml;
-        w.masks(q, a0, x0, x1, p, mg, ml);
-        const int packed = __popc(mg) | (__popc(ml) << 16);
-        const int inc = warp_incl_scan(packed);
-        const int eg = rge + ((inc - packed) & 0xffff), el = rle + ((inc - packed) >> 16);
-        const int base = a0 + 128 * q + 4 * lane;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const unsigned below = (1u << c) - 1u;
-          if ((mg >> c) & 1u) {
-            const int r = eg + __popc(mg & below);
-            if (r < K) {
-              lpos[r] = base + c;
-              lval[r] = w.at(q, c);
-            }
-          }
-          if ((ml >> c) & 1u) {
-            const int rd = total_le - 1 - (el + __popc(ml & below));
-            if (rd < K) {
-              rpos[rd] = base + c;
-              rval[rd] = w.at(q, c);
-            }
-          }
+      for (int k = 0; k < B; ++k) {
+        const int i = b0 + 32 * k + lane;
+        v[k] = 0.0f;
+        if (i < x1) {
+          if constexpr (GLOBAL) v[k] = __ldcg(a + i);
+          else v[k] = a[i];
         }
-        const int tot = __shfl_sync(0xffffffffu, inc, 31);
-        rge += tot & 0xffff;
-        rle += tot >> 16;
+      }
+#pragma unroll
+      for (int k = 0; k < B; ++k) {
+        const int i = b0 + 32 * k + lane;
+        const bool in = i < x1, ge = in && !(v[k] < p), le = in && !(p < v[k]);
+        const unsigned mg = __ballot_sync(0xffffffffu, ge), ml = __ballot_sync(0xffffffffu, le);
+        const int r = rge + __popc(mg & below), rd = rle - __popc(ml & below);
+        if (ge && r < K) {
+          lpos[r] = i;
+          lval[r] = v[k];
+        }
+        if (le && rd < K) {
+          rpos[rd] = i;
+          rval[rd] = v[k];
+        }
+        rge += __popc(mg);
+        rle -= __popc(ml);
       }
     }
   }
@@ -732,7 +751,16 @@ __device__ long long sequential_start(const float* __restrict__ v, long long lo,
   __syncthreads();
   if (threadIdx.x == 0) {
     Acc acc = Acc(0);
-    for (int r = 0; r < (int)(pre_end - lo); ++r) acc = acc + (Acc)sbuf[r + (r >> 4)];
+    const int n = (int)(pre_end - lo);
+    int r = 0;
+    for (; r + 16 <= n; r += 16) {  // one padded run at a time, its loads ahead of its adds
+      float t[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) t[k] = sbuf[r + (r >> 4) + k];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) acc = acc + (Acc)t[k];
+    }
+    for (; r < n; ++r) acc = acc + (Acc)sbuf[r + (r >> 4)];
     s_sum = acc;
   }
   __syncthreads();
@@ -989,24 +1017,38 @@ __device__ __forceinline__ SumPiece then(const SumPiece& f, const SumPiece& g) {
   r.map = (int)map_then((unsigned)f.map, (unsigned)g.map);
   return r;
 }
-// One block: the piece v[pos, end), end - pos <= kSumSeg, on the grid of an accumulator of biased
-// exponent eb.  Every thread gets it.  A term that no such accumulator keeps in its binade
-// saturates the piece.
+// One warp: the piece v[pos, end), end - pos <= kSumSeg, on the grid of an accumulator of biased
+// exponent eb, each lane a run of consecutive terms.  Lane 0 gets it.  A term that no such
+// accumulator keeps in its binade saturates the piece.
 template <typename TermFn>
-__device__ SumPiece sum_piece(const float* v, long long pos, long long end, int eb, TermFn term, OrdShared& S) {
-  using PK = Packed<24>;
-  constexpr int TPT = kSumSeg / kOrdThreads;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+__device__ SumPiece sum_piece(const float* v, long long pos, long long end, int eb, TermFn term) {
+  constexpr int kRun = kSumSeg / 32, kU = 16;
+  const int lane = threadIdx.x & 31;
+  const int n = (int)(end - pos);
+  const float scale = __uint_as_float((uint32_t)(277 - eb) << 23);  // 2^(150 - eb): a term in grid steps, exactly
   SumPiece p{eb, {0, 0}, 2};
+  for (int r0 = lane * kRun; r0 < (lane + 1) * kRun; r0 += kU) {
+    float4 f[kU / 4];
 #pragma unroll
-  for (int j = 0; j < TPT; ++j) {
-    const long long i = pos + tid * TPT + j;
-    const uint32_t w = i < end ? PK::make(term(__ldcg(v + i)), eb - 150) : 0u;
-    SumPiece t;
-    t.k[0] = PK::big(w) || PK::neg(w) ? kPieceSat : (int)min(PK::steps(w, 0), (long long)kPieceSat);
-    t.k[1] = PK::big(w) || PK::neg(w) ? kPieceSat : (int)min(PK::steps(w, 1), (long long)kPieceSat);
-    t.map = (int)PK::pmap(w);
-    p = then(p, t);
+    for (int j = 0; j < kU / 4; ++j)  // pos is a multiple of 4; the array is padded to whole groups
+      f[j] = r0 + 4 * j < n ? __ldcg(reinterpret_cast<const float4*>(v + pos + r0 + 4 * j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < kU; ++j) {
+      const float4 q4 = f[j / 4];
+      const float t = r0 + j < n ? term(j % 4 == 0 ? q4.x : (j % 4 == 1 ? q4.y : (j % 4 == 2 ? q4.z : q4.w))) : 0.0f;
+      // Whole steps and the rest, exactly (a term too small to scale exactly is far below half a
+      // step); a tie goes to the even sum.  Not a number, or 2^25 steps or more: saturated.
+      const float x = t * scale;
+      const float w = floorf(x), rest = x - w;
+      const int q = x < (float)kPieceSat ? (int)w : kPieceSat;
+      const int up = rest > 0.5f ? 1 : 0;
+      const bool tie = rest == 0.5f;
+      SumPiece s;
+      s.k[0] = q + (tie ? (q & 1) : up);
+      s.k[1] = q + (tie ? ((q & 1) ^ 1) : up);
+      s.map = tie ? 0 : ((s.k[0] & 1) ? 1 : 2);
+      p = then(p, s);
+    }
   }
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {  // neighbouring runs, left then right
@@ -1016,11 +1058,6 @@ __device__ SumPiece sum_piece(const float* v, long long pos, long long end, int 
     y.map = __shfl_down_sync(0xffffffffu, p.map, o);
     if ((lane & (2 * o - 1)) == 0) p = then(p, y);
   }
-  __syncthreads();
-  if (lane == 0) S.piece[warp] = p;
-  __syncthreads();
-  p = S.piece[0];
-  for (int w = 1; w < kOrdWarps; ++w) p = then(p, S.piece[w]);
   return p;
 }
 
@@ -1148,8 +1185,10 @@ __device__ void cluster_steps(cg::cluster_group& cl, const SearchDesc& sd, Order
 //
 // As 51 launches (three per partition step, whether a search needed them or not) these cost every
 // call 67 to 165 us and a search of 2^20 whole-number column sums 2.0 ms; the one launch costs
-// 2 to 5 us and 1.6 ms.
-__global__ void __cluster_dims__(kOrderCluster, 1, 1) __launch_bounds__(kOrdThreads, 1)
+// 2 to 5 us and 1.1 ms (partition steps 0.6 ms, bound by their barriers, the lists' scattered
+// stores and the leader's scans; the selections' last steps in shared memory 0.25 ms; the sums
+// 0.2 ms).
+__global__ void __launch_bounds__(kOrdThreads, 1)
     order_kernel(const __grid_constant__ SearchBatch b, int min_ties) {
   const SearchDesc& sd = b.s[blockIdx.y];
   const int N = sd.N;
@@ -1157,14 +1196,15 @@ __global__ void __cluster_dims__(kOrderCluster, 1, 1) __launch_bounds__(kOrdThre
   __shared__ OrdShared S;
   extern __shared__ __align__(16) float dyn[];
   cg::cluster_group cl = cg::this_cluster();
-  const int r = (int)cl.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r = (int)cl.block_rank(), C = (int)cl.num_blocks();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* sdata = dyn;                                      // kSmemRange values
   int* slists = reinterpret_cast<int*>(dyn + kSmemRange);  // 4 * kSmemPairs entries
   OrderTask* tasks = order_tasks(sd);
   float* a = sd.work;
   // The column sums copied to the work array (16-byte words: both start 16-byte aligned).
   const int n4 = N / 4;
-  for (int i = r * kOrdThreads + tid; i < n4; i += kOrderCluster * kOrdThreads)
+  for (int i = r * kOrdThreads + tid; i < n4; i += C * kOrdThreads)
     reinterpret_cast<float4*>(a)[i] = __ldcg(reinterpret_cast<const float4*>(sd.colsum) + i);
   if (r == 0)
     for (int i = 4 * n4 + tid; i < N; i += kOrdThreads) a[i] = __ldcg(sd.colsum + i);
@@ -1174,7 +1214,7 @@ __global__ void __cluster_dims__(kOrderCluster, 1, 1) __launch_bounds__(kOrdThre
     task_init(a, tasks[0], 0, sd.mid, N);
   }
   cl.sync();
-  cluster_steps(cl, sd, tasks, 0, 0, r, kOrderCluster, S);
+  cluster_steps(cl, sd, tasks, 0, 0, r, C, S);
   bool bad = false;
   if (r == 0) {
     __threadfence();
@@ -1195,7 +1235,7 @@ __global__ void __cluster_dims__(kOrderCluster, 1, 1) __launch_bounds__(kOrdThre
     }
   }
   cl.sync();
-  const int half = kOrderCluster / 2, t = r < half ? 1 : 2, cta = r % half;
+  const int half = C / 2, t = r < half ? 1 : 2, cta = r % half;
   cluster_steps(cl, sd, tasks, t, 3 - t, cta, half, S);
   if (cta == 0) {
     __threadfence();
@@ -1213,12 +1253,12 @@ __global__ void __cluster_dims__(kOrderCluster, 1, 1) __launch_bounds__(kOrdThre
   __shared__ double s_dsum;
   float* sbuf = dyn;  // kSumBuf floats
   {
-    const PlainSum p = plain_sum(a, first, last, r, kOrderCluster, S);
-    if (tid < kOrderCluster) cl.map_shared_rank(s_plain, tid)[r] = p;
+    const PlainSum p = plain_sum(a, first, last, r, C, S);
+    if (tid < C) cl.map_shared_rank(s_plain, tid)[r] = p;
   }
   cl.sync();
   PlainSum tot = s_plain[0];
-  for (int q = 1; q < kOrderCluster; ++q) {
+  for (int q = 1; q < C; ++q) {
     tot.abs += s_plain[q].abs;
     tot.sum += s_plain[q].sum;
     tot.g = min(tot.g, s_plain[q].g);
@@ -1228,7 +1268,7 @@ __global__ void __cluster_dims__(kOrderCluster, 1, 1) __launch_bounds__(kOrdThre
       auto same = [](float f) { return f; };
       const long long pos = sequential_start(a, (long long)first, (long long)last, same, sbuf, s_dsum);
       sequential_range<double, kTermsPerThreadD>(a, pos, (long long)last, same, sbuf, S, s_dsum);
-      if (tid < kOrderCluster) *cl.map_shared_rank(&s_dsum, tid) = s_dsum;
+      if (tid < C) *cl.map_shared_rank(&s_dsum, tid) = s_dsum;
     }
     cl.sync();
     tot.sum = s_dsum;
@@ -1241,14 +1281,15 @@ __global__ void __cluster_dims__(kOrderCluster, 1, 1) __launch_bounds__(kOrdThre
     const float d = __fsub_rn(f, m);
     return __fmul_rn(d, d);
   };
-  const int np = (n + kSumSeg - 1) / kSumSeg;
+  const int base = first & ~3;  // pieces start at multiples of 4, so that they take 16-byte loads
+  const int np = (last + 1 - base + kSumSeg - 1) / kSumSeg;
   // In the pair lists' memory (8 bytes per channel): the pieces, then the prefix sums.
   SumPiece* pieces = reinterpret_cast<SumPiece*>(sd.lists);
   double* prefix = reinterpret_cast<double*>(pieces + np);
-  for (int c = r * kOrdWarps + warp; c < np; c += kOrderCluster * kOrdWarps) {
-    const int c1 = min(last + 1, first + (c + 1) * kSumSeg);
+  for (int c = r * kOrdWarps + warp; c < np; c += C * kOrdWarps) {
+    const int c1 = (int)min((long long)last + 1, (long long)base + (c + 1ll) * kSumSeg);
     double acc = 0.0;
-    for (int i = first + c * kSumSeg + lane; i < c1; i += 32) acc += (double)term(__ldcg(a + i));
+    for (int i = max(first, base + c * kSumSeg) + lane; i < c1; i += 32) acc += (double)term(__ldcg(a + i));
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     if (lane == 0) prefix[c] = acc;
   }
@@ -1267,14 +1308,13 @@ __global__ void __cluster_dims__(kOrderCluster, 1, 1) __launch_bounds__(kOrdThre
     }
   }
   cl.sync();
-  for (int c = 1 + r; c < np; c += kOrderCluster) {  // piece 0 starts from zero: term by term
+  for (int c = 1 + r * kOrdWarps + warp; c < np; c += C * kOrdWarps) {  // piece 0 starts from zero: term by term
     const int eb = (int)((__float_as_uint((float)__ldcg(prefix + c)) >> 23) & 0xffu);
     SumPiece p{0, {0, 0}, 2};
     if (eb > 24 && eb < 255)
-      p = sum_piece(a, (long long)first + (long long)c * kSumSeg, min((long long)last + 1, (long long)first + (c + 1ll) * kSumSeg),
-                    eb, term, S);
-    if (tid == 0) pieces[c] = p;
-    __syncthreads();
+      p = sum_piece(a, (long long)base + (long long)c * kSumSeg, min((long long)last + 1, (long long)base + (c + 1ll) * kSumSeg),
+                    eb, term);
+    if (lane == 0) pieces[c] = p;
   }
   cl.sync();
   if (r != 0) return;
@@ -1283,7 +1323,7 @@ __global__ void __cluster_dims__(kOrderCluster, 1, 1) __launch_bounds__(kOrdThre
   SumPiece* sp = reinterpret_cast<SumPiece*>(dyn + kSumBuf);  // behind sbuf
   constexpr int kTile = 1024;
   long long pos = sequential_start(a, (long long)first, (long long)last, term, sbuf, s_sum);
-  sequential_range<float, kSumSeg / kOrdThreads>(a, pos, min((long long)last, (long long)first + kSumSeg - 1), term, sbuf, S,
+  sequential_range<float, kSumSeg / kOrdThreads>(a, pos, min((long long)last, (long long)base + kSumSeg - 1), term, sbuf, S,
                                                  s_sum);
   for (int c0 = 1; c0 < np;) {
     const int cn = min(np, c0 + kTile);
@@ -1310,7 +1350,7 @@ __global__ void __cluster_dims__(kOrderCluster, 1, 1) __launch_bounds__(kOrdThre
       c = s_at;
       __syncthreads();
       if (c < cn) {
-        const long long p0 = (long long)first + (long long)c * kSumSeg;
+        const long long p0 = (long long)base + (long long)c * kSumSeg;
         sequential_range<float, kSumSeg / kOrdThreads>(a, p0, min((long long)last, p0 + kSumSeg - 1), term, sbuf, S, s_sum);
         ++c;
       }
@@ -1338,8 +1378,27 @@ cudaError_t search_stats_exact(const SearchBatch& b, int min_ties, cudaStream_t 
                 "the sum's buffers fit the selection's");
   cudaError_t e = cudaFuncSetAttribute(order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  order_kernel<<<dim3(kOrderCluster, b.count), kOrdThreads, smem, stream>>>(b, min_ties);
-  return cudaGetLastError();
+  if ((e = cudaFuncSetAttribute(order_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
+  // Sixteen CTAs per search where a cluster of that many fits (16 SMs of one GPC) and the batch is
+  // small enough that the searches run side by side, else eight (64 searches that all leave at
+  // once: 8.6 and 5.0 us).
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(kOrdThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  for (int c = b.count <= 8 ? kOrderCluster : kOrderCluster / 2;; c /= 2) {
+    at[0].val.clusterDim.x = c;
+    cfg.gridDim = dim3(c, b.count);
+    int clusters = 0;
+    if (c <= 8 || (cudaOccupancyMaxActiveClusters(&clusters, order_kernel, &cfg) == cudaSuccess && clusters > 0)) break;
+    cudaGetLastError();
+  }
+  return cudaLaunchKernelEx(&cfg, order_kernel, b, min_ties);
 }
 
 namespace {
