@@ -242,7 +242,7 @@ typedef struct sc_dd_pool_stats {
   long long sub_batches;     /* admitted groups of requests that fit the scratch budget */
   long long graph_replays;   /* sub-batches replayed from a captured CUDA graph */
   long long graph_captures;
-  long long tuned_launches;  /* autotuning decisions taken (tree launches, level splits) */
+  long long tuned_launches;  /* autotuning decisions taken (tree launches) */
   float last_call_ms;        /* device time of the last call, CUDA events */
   int pad;
 } sc_dd_pool_stats;
@@ -252,7 +252,7 @@ typedef struct sc_dd_pool sc_dd_pool;
 /* A pool runs lists of requests of any mix of shapes: requests are admitted in order
  * into sub-batches whose scratch fits scratch_budget_bytes (one request always fits:
  * the pool grows its arena for a larger one), every kernel runs once per sub-batch of up
- * to 64 searches, tree launches and level splits are autotuned on first sight, and a
+ * to 64 searches, tree launches are autotuned on first sight, and a
  * sub-batch seen again is replayed from a captured CUDA graph.  No counterpart in the
  * reference (which runs one search at a time). */
 int sc_dd_pool_create(size_t scratch_budget_bytes, sc_dd_pool** out);

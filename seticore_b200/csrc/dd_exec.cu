@@ -242,8 +242,7 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
              std::min<long long>(ndb, 2 * half * pairs / per_db) * per_db * (long long)sizeof(float) >= (128ll << 20);
     };
     auto level = [&](const ExecSearch& q, float* la, float* lb, cudaStream_t st) {
-      const LevelPlan plan = hooks.level_plan ? hooks.level_plan(hooks.ctx, q, la, lb, st) : q.level_plan;
-      return levels_search(q.input, q.row_stride, q.Tr, q.N, q.dmin, q.dmax, la, lb, q.top, num_sms, st, plan, kElemF32,
+      return levels_search(q.input, q.row_stride, q.Tr, q.N, q.dmin, q.dmax, la, lb, q.top, num_sms, st, kElemF32,
                            header_status(q));
     };
     int n_level = 0;
@@ -253,8 +252,8 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
       const ExecSearch& q = ss[k];
       if (q.Tr <= 32) continue;
       if (q.elem != kElemF32)
-        e = levels_search(q.norm16, q.N, q.Tr, q.N, q.dmin, q.dmax, lvl_a, lvl_b, q.top16, num_sms, stream, LevelPlan{},
-                          q.elem, header_status(q));
+        e = levels_search(q.norm16, q.N, q.Tr, q.N, q.dmin, q.dmax, lvl_a, lvl_b, q.top16, num_sms, stream, q.elem,
+                          header_status(q));
       else if (lanes == 1 || wide(q))
         e = level(q, lvl_a, lvl_a + half * pairs, stream);
       if (e != cudaSuccess) return e;

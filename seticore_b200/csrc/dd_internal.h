@@ -292,17 +292,10 @@ cudaError_t search_hits_batch(const SearchBatch& b, int num_sms, cudaStream_t st
 cudaError_t path_values(const float* input, long long row_stride, int Tr, int N, const int* index,
                         const int* drift_steps, float* out, int n, cudaStream_t stream);
 
-// How a tree of more than 32 rows is split: levels of m[0..n) rows each -- 2 or 4
-// (emit_kernel), 8 or 16 (direct_kernel, one thread per channel) or, first only,
-// kStreamEmit16 (the emitting form of the fused tree) -- then a fused max level of
-// final_rows (2, 4, 8 or 16) rows.  n == 0: the default split.
+// First levels of a tree of more than 32 rows: the emitting form of the fused tree with the sixteen
+// offsets in two halves or all in one warp.
 constexpr int kStreamEmit16 = 1016;
-constexpr int kStreamEmit16One = 1017;  // the emitting form with all sixteen offsets in one warp
-struct LevelPlan {
-  int n;
-  int m[12];
-  int final_rows;
-};
+constexpr int kStreamEmit16One = 1017;
 
 // L2 budget of one stripe pass of the one-level split (bytes; negative: the default).
 void set_level_stripe_bytes(long long bytes);
@@ -311,11 +304,11 @@ long long level_stripe_bytes();  // the value set (negative: none)
 // Multi-level tree for Tr > 32 (one search): level kernels write the partial planes of
 // every sub-problem, then the fused max kernel finishes them (see dd_levels.cu).
 // scratch_a / scratch_b: level_buffer_floats(Tr, N) floats each, in one allocation.
-// `input` holds elements of type `elem` (float, or the precision form's 16-bit copy, which
-// only the default plan reads: its first level converts on load).
+// `input` holds elements of type `elem` (float, or the precision form's 16-bit copy, whose first
+// level converts on load).
 cudaError_t levels_search(const void* input, long long row_stride, int Tr, int N, int dmin, int dmax,
                           float* scratch_a, float* scratch_b, float* top, int num_sms,
-                          cudaStream_t stream, const LevelPlan& plan = LevelPlan{}, int elem = kElemF32,
+                          cudaStream_t stream, int elem = kElemF32,
                           int* status = nullptr);
 
 // A fully planned search for exec_queue: the request, its drift plan and its scratch.
@@ -326,7 +319,6 @@ struct ExecSearch {
   int dmin, dmax, window_size;
   double snr_threshold;
   int elem;  // kElemF32, or the 16-bit storage of the precision form
-  LevelPlan level_plan;
   int cand_cap;
   // scratch (carve() lays it out from one base pointer)
   float* top;
@@ -352,8 +344,6 @@ struct ExecHooks {
   void* ctx = nullptr;
   TreeLaunch (*tree_launch)(void* ctx, const TreeBatch& tb, int R, int elem) = [](void*, const TreeBatch&, int,
                                                                                    int) { return TreeLaunch{}; };
-  // The level split of a search with more than 32 rows (may time alternatives first).
-  LevelPlan (*level_plan)(void* ctx, const ExecSearch& s, float* lvl_a, float* lvl_b, cudaStream_t st) = nullptr;
   void (*before_tree)(void* ctx, cudaStream_t s) = nullptr;
   void (*after_tree)(void* ctx, cudaStream_t s) = nullptr;
 };

@@ -18,8 +18,7 @@
 //    the last level reads in that row (each block row has its own channel origin).
 //  * 16-bit rows and Tr > 256: direct16x4_kernel (four channels per thread from global
 //    memory), then emit_kernel's 4- and 2-row levels while more than 16 rows remain.
-// The pool's autotuner times these against the other splits per shape class.  The pairing
-// of the adds is the tree's own at every level, so every path sum is bit-identical to the
+// The pairing of the adds is the tree's own at every level, so every path sum is bit-identical to the
 // reference's twoStageTaylorTree (taylor.cu:298-327).
 #include <algorithm>
 #include <atomic>
@@ -84,41 +83,8 @@ __global__ void emit_kernel(const float* __restrict__ src, long long src_stride,
   for (int o = 0; o < M; ++o) dst[(((long long)p * M + o) * nb + q) * dst_stride + c] = out[o];
 }
 
-// One level of M in {8, 16} rows, one thread per channel: all M in-block offsets of the
-// M-row subtree at channel c from its 136 (M = 16) or 36 (M = 8) leaves, in the tree's
-// pairing (taylor_direct_M, generated).  Loads of neighbouring threads overlap, so most
-// come from L1; the level reads its input from HBM once and writes the planes once.
-// Problem p reads rows from src + p * src_problem_rows rows (0: every problem reads the same
-// rows, as the first level does for a chunk of drift blocks) with drift D0 + p.
-template <int M, typename E>
-__global__ void __launch_bounds__(128, 6) direct_kernel(const E* __restrict__ src, long long src_stride,
-                                                        long long src_problem_rows, int Tp, int D0,
-                                                        float* __restrict__ dst, long long dst_stride, int N) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= N) return;
-  const int nb = Tp / M;
-  const int p = blockIdx.y / nb;
-  const int q = blockIdx.y - p * nb;
-  const long long D = (long long)D0 + p;
-  const E* r0 = src + ((long long)p * src_problem_rows + (long long)q * M) * src_stride;
-  float out[M];
-  // Leaves lie in [c + min(0, (M-1)D), c + (M-1) + max(0, (M-1)D)]: inside the row for
-  // most channels, which then load without bounds checks.
-  static_assert(M == 8, "16 rows use direct16x4_kernel");
-  const long long span = (long long)(M - 1) * D;
-  const bool inside = c + (span < 0 ? span : 0) >= 0 && c + (M - 1) + (span > 0 ? span : 0) < N;
-  if (inside) {
-    auto ld = [&](int t, int pos) { return as_float(r0[t * src_stride + c + D * t + pos]); };
-    taylor_direct_8(ld, out);
-  } else {
-    auto ld = [&](int t, int pos) { return ld_or_zero(r0 + t * src_stride, c + pos + D * t, N); };
-    taylor_direct_8(ld, out);
-  }
-#pragma unroll
-  for (int o = 0; o < M; ++o) dst[(((long long)p * M + o) * nb + q) * dst_stride + c] = out[o];
-}
-
-// The 16-row level with four consecutive channels per thread: neighbouring channels share
+// One level of 16 rows, four consecutive channels per thread: all 16 in-block offsets of the subtree
+// at each channel, in the tree's pairing (taylor_direct_16x4, generated).  Neighbouring channels share
 // leaves and nodes (46 leaf loads and 86 adds per channel instead of 136 and 152), and the
 // four results of each offset leave as one 16-byte store.  Plane rows are padded to whole
 // tiles (a multiple of 4 channels), so the last thread of a row stores inside its plane.
@@ -172,34 +138,6 @@ TreeGroup final_group(const float* src, long long Np, int N, int final_rows, int
   tp.elig_T1 = Tr - 1;
   tp.top = top;
   return tp;
-}
-
-// The emitting 16-row tree for drift blocks db0 .. db0 + nj - 1 of the input's Tr rows
-// (whole rows, the plane layout of the other level kernels): group q reads rows
-// 16q .. 16q + 15 (one trapezoid for the nj drift blocks) and writes plane r*(Tr/16) + q of
-// drift block j to out + j*job_stride.
-cudaError_t emit16(const float* input, long long row_stride, int Tr, int N, long long Np, int db0, int nj,
-                   float* out, long long job_stride, int num_sms, cudaStream_t stream, int* status) {
-  const int nb = Tr / 16;
-  TreeBatch eb;
-  eb.count = nb;
-  eb.n_items = 0;
-  for (int q = 0; q < nb; ++q) {
-    TreeGroup& g = eb.g[q];
-    g = TreeGroup{};
-    g.rows = input + (long long)16 * q * row_stride;
-    g.row_stride = row_stride;
-    g.job_row_stride = 0;
-    g.N = N;
-    g.d_first = db0;
-    g.d_step = 1;
-    g.n_jobs = nj;
-    g.emit_out = out + (long long)q * Np;
-    g.emit_job_stride = job_stride;
-    g.emit_plane_stride = (long long)nb * Np;
-    g.status = status;
-  }
-  return tree_emit_batch(eb, num_sms, stream);
 }
 
 constexpr int kEmitTile = 352;     // channels per work item of the emitting tree
@@ -422,38 +360,25 @@ long long level_stripe_bytes() { return g_stripe_bytes.load(); }
 
 cudaError_t levels_search(const void* input_v, long long row_stride, int Tr, int N, int dmin, int dmax,
                           float* scratch_a, float* scratch_b, float* top, int num_sms,
-                          cudaStream_t stream, const LevelPlan& plan, int elem, int* status) {
+                          cudaStream_t stream, int elem, int* status) {
   int sizes[12];
   int nlev = 0;
-  int final_rows = 16;
   const float* input = static_cast<const float*>(input_v);
-  if (elem != kElemF32 && plan.n > 0) return cudaErrorInvalidValue;  // 16-bit input: default split only
-  if (plan.n > 0) {
-    int prod = plan.final_rows;
-    for (int l = 0; l < plan.n; ++l) {
-      const int M = plan.m[l];
-      const bool emit = (M == kStreamEmit16 || M == kStreamEmit16One) && l == 0;
-      if (M != 2 && M != 4 && M != 8 && M != 16 && !emit) return cudaErrorInvalidValue;
-      sizes[nlev++] = M;
-      prod *= emit ? 16 : M;
-    }
-    final_rows = plan.final_rows;
-    if (prod != Tr || (final_rows != 2 && final_rows != 4 && final_rows != 8 && final_rows != 16))
-      return cudaErrorInvalidValue;
-  } else {
-    // Default: the 16-row level, then 4s and 2s down to at most 16 rows.  A single 16-row
-    // level (Tr <= 256) of float rows takes the emitting tree in stripe passes; 16-bit rows
-    // and deeper splits the four-channels-per-thread level kernel (the emitting tree
-    // converts 16-bit rows with per-thread loads as it stages them: 0.79x on 256-row beams).
-    int tp = Tr / 16;
-    sizes[nlev++] = (tp <= 16 && elem == kElemF32) ? default_first_level() : 16;
-    while (tp > 16) {
-      const int M = (tp / 4 >= 16) ? 4 : 2;
-      sizes[nlev++] = M;
-      tp /= M;
-    }
-    final_rows = tp;
+  // The 16-row level, then 4s and 2s down to at most 16 rows.  A single 16-row level (Tr <= 256) of
+  // float rows takes the emitting tree in stripe passes; 16-bit rows and deeper splits the
+  // four-channels-per-thread level kernel (the emitting tree converts 16-bit rows with per-thread
+  // loads as it stages them: 0.79x on 256-row beams).  Chains of 4- and 2-row levels, an 8-row
+  // first level and the per-thread 16-row one were timed against this on 57 shapes of 64 to 1024
+  // rows, 16384 to 2^20 channels and 2 to 34 drift blocks: none was faster by more than 0.4 %, and
+  // timing them took three quarters of a pool's first call (24 uneven searches: 105 ms, 27 without).
+  int tp = Tr / 16;
+  sizes[nlev++] = (tp <= 16 && elem == kElemF32) ? default_first_level() : 16;
+  while (tp > 16) {
+    const int M = (tp / 4 >= 16) ? 4 : 2;
+    sizes[nlev++] = M;
+    tp /= M;
   }
+  const int final_rows = tp;
   // scratch_b lies in the same allocation as scratch_a, which holds 2 * (scratch_b -
   // scratch_a) floats: one level buffer for the ping-pong of multi-level plans, or room for
   // the planes of several drift blocks at once.
@@ -502,12 +427,9 @@ cudaError_t levels_search(const void* input_v, long long row_stride, int Tr, int
     int P = 1, Tp = Tr;
     long long dscale = 1;  // product of the level sizes so far
     for (int l = 0; l < nlev; ++l) {
-      int M = sizes[l];
+      const int M = sizes[l];
       const int D0 = (int)(dscale * db);
-      if (M == kStreamEmit16 || M == kStreamEmit16One) {
-        M = 16;
-        if ((err = emit16(src, stride, Tp, N, Np, db, 1, dst, per_db, num_sms, stream, status)) != cudaSuccess) return err;
-      } else if (M == 16) {
+      if (M == 16) {
         dim3 grid((N + 511) / 512, (unsigned)(P * (Tp / M)));
         if (l == 0 && elem == kElemBF16) {
           direct16x4_kernel<<<grid, 128, 0, stream>>>(static_cast<const __nv_bfloat16*>(input_v), stride, Tp, Tp, D0,
@@ -518,9 +440,6 @@ cudaError_t levels_search(const void* input_v, long long row_stride, int Tr, int
         } else {
           direct16x4_kernel<<<grid, 128, 0, stream>>>(src, stride, Tp, Tp, D0, dst, Np, N);
         }
-      } else if (M == 8) {
-        dim3 grid((N + 127) / 128, (unsigned)(P * (Tp / M)));
-        direct_kernel<8><<<grid, 128, 0, stream>>>(src, stride, Tp, Tp, D0, dst, Np, N);
       } else {
         dim3 grid((N + 255) / 256, (unsigned)(P * (Tp / M)));
         if (M == 4) emit_kernel<4><<<grid, 256, 0, stream>>>(src, stride, Tp, D0, dst, Np, N);

@@ -11,13 +11,11 @@
 // power-of-two buckets of its largest drift-block count and total channels) is seen, it is
 // timed with each candidate launch shape -- tile width (1056 or 352 channels) and
 // shared-memory budget (which sets how many drift blocks share a staged trapezoid and how
-// many CTAs share an SM) -- and the fastest is kept; likewise, each
-// class of more than 32 rows (rows, buckets of channels and drift blocks) times the
-// candidate level splits (stage-fusion depth).  Timing reruns are harmless: the tree
+// many CTAs share an SM) -- and the fastest is kept.  Timing reruns are harmless: the tree
 // kernel only raises per-channel maxima, so repeating it is idempotent.
 //
 // CUDA graphs: a sub-batch seen before (same requests, same arena layout) is replayed
-// from a captured graph that also holds the copies of the results to pinned host memory.
+// from a captured graph, whose last kernels write the results to pinned host memory.
 #include <algorithm>
 #include <cstddef>
 #include <cmath>
@@ -87,7 +85,6 @@ struct sc_dd_pool {
   std::vector<Graph> graphs;
   std::unordered_map<uint64_t, int> seen;  // sub-batch key -> times seen
   std::unordered_map<uint64_t, scb::TreeLaunch> tuned_launch;
-  std::unordered_map<uint64_t, scb::LevelPlan> tuned_plan;
   uint64_t clock = 0;
   int tuning = 1, use_graphs = 1;
   bool tuning_now = false;
@@ -149,86 +146,6 @@ scb::TreeLaunch pool_tree_launch(void* ctx, const scb::TreeBatch& tb, int R, int
   return best;
 }
 
-std::vector<scb::LevelPlan> level_candidates(int Tr) {
-  std::vector<scb::LevelPlan> out;
-  // a 16-row first level (one thread per channel, or the emitting fused tree with two
-  // drift blocks per staged read), then 4s / 2s down to at most 16 rows
-  if (Tr >= 32) {
-    for (int first : {16, scb::kStreamEmit16}) {
-      scb::LevelPlan pl{};
-      pl.m[pl.n++] = first;
-      int rem = Tr / 16;
-      while (rem > 16 && pl.n < 12) {
-        const int m = (rem / 4 >= 16) ? 4 : 2;
-        pl.m[pl.n++] = m;
-        rem /= m;
-      }
-      pl.final_rows = rem;
-      out.push_back(pl);
-    }
-    // the one-thread-per-channel 8-row level first, finishing in 16 or fewer rows
-    if (Tr / 8 <= 16) {
-      scb::LevelPlan pl{};
-      pl.m[pl.n++] = 8;
-      pl.final_rows = Tr / 8;
-      out.push_back(pl);
-    }
-  }
-  // emit levels of 4s then 2s (or 2s then 4s) down to a final of 16 or 8 rows
-  for (int fin : {16, 8}) {
-    for (int order = 0; order < 2; ++order) {
-      scb::LevelPlan pl{};
-      pl.final_rows = fin;
-      int rem = Tr / fin;
-      if (rem < 2) continue;
-      std::vector<int> ms;
-      while (rem > 1) {
-        const int m = (rem % 4 == 0) ? 4 : 2;
-        ms.push_back(m);
-        rem /= m;
-      }
-      if (order == 1) std::reverse(ms.begin(), ms.end());
-      if ((int)ms.size() > 12) continue;
-      pl.n = (int)ms.size();
-      for (int i = 0; i < pl.n; ++i) pl.m[i] = ms[i];
-      bool dup = false;
-      for (auto& q : out)
-        if (q.n == pl.n && q.final_rows == pl.final_rows && std::equal(q.m, q.m + q.n, pl.m)) dup = true;
-      if (!dup) out.push_back(pl);
-    }
-  }
-  return out;
-}
-
-scb::LevelPlan pool_level_plan(void* ctx, const scb::ExecSearch& s, float* la, float* lb, cudaStream_t st) {
-  sc_dd_pool* p = static_cast<sc_dd_pool*>(ctx);
-  const int v[3] = {s.Tr, bucket(s.N), bucket(s.dmax - s.dmin + 1)};
-  const uint64_t key = fnv(1469598103934665603ull, v, sizeof(v));
-  auto it = p->tuned_plan.find(key);
-  if (it != p->tuned_plan.end()) return it->second;
-  if (!p->tuning || !p->tuning_now) return scb::LevelPlan{};
-  scb::LevelPlan best{};
-  float best_ms = 1e30f;
-  for (const scb::LevelPlan& pl : level_candidates(s.Tr)) {
-    cudaEventRecord(p->t0, st);
-    int* status = reinterpret_cast<int*>(reinterpret_cast<char*>(s.hdr) + offsetof(scb::SearchHeader, error));
-    if (scb::levels_search(s.input, s.row_stride, s.Tr, s.N, s.dmin, s.dmax, la, lb, s.top, p->num_sms, st, pl,
-                           scb::kElemF32, status) != cudaSuccess)
-      continue;
-    cudaEventRecord(p->t1, st);
-    cudaEventSynchronize(p->t1);
-    float ms = 0;
-    cudaEventElapsedTime(&ms, p->t0, p->t1);
-    if (ms < best_ms) {
-      best_ms = ms;
-      best = pl;
-    }
-  }
-  p->tuned_plan[key] = best;
-  p->st.tuned_launches++;
-  return best;
-}
-
 // Grows the arena and the level buffers in stream order on `stream` (cudaFreeAsync /
 // cudaMallocAsync): every earlier call of this pool has finished with them (a call
 // synchronises its stream before it returns), and work of other streams -- another pool's,
@@ -285,10 +202,8 @@ cudaError_t queue_sub(sc_dd_pool* p, std::vector<Planned>& sub, cudaStream_t s) 
   scb::ExecHooks hooks;
   hooks.ctx = p;
   hooks.tree_launch = pool_tree_launch;
-  hooks.level_plan = pool_level_plan;
-  // The tuner times one level search at a time on its own stream: no side stream then.
   cudaError_t e = scb::exec_queue(es.data(), (int)es.size(), p->lvl_a, p->lvl_b, p->num_sms, s, hooks,
-                                  p->tuning_now || p->side.n == 0 ? nullptr : &p->side);
+                                  p->side.n == 0 ? nullptr : &p->side);
   return e;
 }
 
@@ -499,7 +414,7 @@ int sc_dd_pool_search(sc_dd_pool* p, const sc_dd_request* reqs, int count, sc_dd
         p->st.graph_captures++;
         if ((e = cudaGraphLaunch(ex, stream)) != cudaSuccess) return pcuda(e, "graph launch");
       } else {
-        // First sight: run directly; tree launches and level splits not seen before are tuned.
+        // First sight: run directly; tree launches not seen before are tuned.
         p->tuning_now = true;
         std::swap(p->cap_stream, stream);  // the tuning hooks time on p->cap_stream
         e = queue_sub(p, sub, p->cap_stream);
