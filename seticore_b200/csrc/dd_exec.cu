@@ -3,9 +3,9 @@
 // Used by the engine (dd_api.cu, one shape) and by the pool (dd_pool.cu, mixed shapes).
 // The searches travel in batches of up to kMaxBatch as kernel parameters, so a call is a
 // fixed sequence of launches (capturable in a CUDA graph) whatever the mix:
-//   clear -> [normalise] -> column sums (searches whose tree does not compute them) ->
-//   tree launches grouped by (rows, element type), the float32 ones adding the column
-//   sums -> levels for more than 32 rows, one search at a time -> statistics ->
+//   clear -> [normalise] -> tree launches grouped by (rows, element type), the float32 ones
+//   adding the column sums -> levels for more than 32 rows, one search at a time -> column
+//   sums (searches whose trees did not compute them) -> statistics ->
 //   [flag + FP32 recompute of the flagged channels] -> hits
 #include <algorithm>
 #include <cstddef>
@@ -175,20 +175,6 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
         }
       if (q.count && (e = normalize_batch(q, num_sms, stream)) != cudaSuccess) return e;
     }
-    // Column sums: the float32 trees over up to 32 rows compute their own from the staged
-    // rows and the 16-bit forms in their normalising pass; the level path reads the input
-    // once here.
-    {
-      SearchBatch cb;
-      cb.count = 0;
-      cb.maxN = 0;
-      for (int k = 0; k < m; ++k)
-        if (!fused_colsum(ss[k])) {
-          cb.s[cb.count++] = b.s[k];
-          cb.maxN = std::max(cb.maxN, ss[k].N);
-        }
-      if ((e = column_sums_batch(cb, stream)) != cudaSuccess) return e;
-    }
     if (hooks.before_tree) hooks.before_tree(hooks.ctx, stream);
     // Trees over up to 32 rows: one launch per (rows, element type).
     for (int R : {2, 4, 8, 16, 32}) {
@@ -241,9 +227,20 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
       return pairs > 1 && ndb * per_db > 2 * half &&
              std::min<long long>(ndb, 2 * half * pairs / per_db) * per_db * (long long)sizeof(float) >= (128ll << 20);
     };
-    auto level = [&](const ExecSearch& q, float* la, float* lb, cudaStream_t st) {
-      return levels_search(q.input, q.row_stride, q.Tr, q.N, q.dmin, q.dmax, la, lb, q.top, num_sms, st, kElemF32,
-                           header_status(q));
+    bool summed[kMaxBatch];
+    for (int k = 0; k < m; ++k) summed[k] = fused_colsum(ss[k]);
+    auto level = [&](int k, bool alone, float* la, float* lb, cudaStream_t st) {
+      const ExecSearch& q = ss[k];
+      // Column sums on the way cost the first level its spread: a tile's row groups then run one
+      // after another on one CTA.  That pays where tiles are many -- a dozen per SM for a search
+      // alone, two per SM beside others, whose launches fill the gaps.  32 beams of 256 x 131072:
+      // 5.13 -> 4.95 ms (0.60 ms of their own launch before, 0.43 ms more in the levels); 4 of 64 x
+      // 2^20: 0.16 of 3.65 ms saved; but one by one, 256 x 131072 with 4 drift blocks 2.00 -> 2.27
+      // ms of levels for 0.17 ms of sums.
+      const long long tiles = q.N / 352;
+      float* colsum = tiles >= (alone ? 12ll : 2ll) * num_sms ? q.colsum : nullptr;
+      return levels_search(q.input, q.row_stride, q.Tr, q.N, q.dmin, q.dmax, la, lb, q.top, num_sms, st, colsum, &summed[k],
+                           kElemF32, header_status(q));
     };
     int n_level = 0;
     for (int k = 0; k < m; ++k) n_level += ss[k].Tr > 32 && ss[k].elem == kElemF32 && !wide(ss[k]);
@@ -252,10 +249,10 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
       const ExecSearch& q = ss[k];
       if (q.Tr <= 32) continue;
       if (q.elem != kElemF32)
-        e = levels_search(q.norm16, q.N, q.Tr, q.N, q.dmin, q.dmax, lvl_a, lvl_b, q.top16, num_sms, stream, q.elem,
-                          header_status(q));
+        e = levels_search(q.norm16, q.N, q.Tr, q.N, q.dmin, q.dmax, lvl_a, lvl_b, q.top16, num_sms, stream, nullptr,
+                          nullptr, q.elem, header_status(q));
       else if (lanes == 1 || wide(q))
-        e = level(q, lvl_a, lvl_a + half * pairs, stream);
+        e = level(k, true, lvl_a, lvl_a + half * pairs, stream);
       if (e != cudaSuccess) return e;
     }
     if (lanes > 1) {
@@ -266,8 +263,8 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
       for (int k = 0; k < m; ++k) {
         if (ss[k].Tr <= 32 || ss[k].elem != kElemF32 || wide(ss[k])) continue;
         const int lane = j++ % lanes;  // 0: the main stream
-        if ((e = lane ? level(ss[k], side->lvl_a[lane - 1], side->lvl_b[lane - 1], side->stream[lane - 1])
-                      : level(ss[k], lvl_a, lvl_b, stream)) != cudaSuccess)
+        if ((e = lane ? level(k, false, side->lvl_a[lane - 1], side->lvl_b[lane - 1], side->stream[lane - 1])
+                      : level(k, false, lvl_a, lvl_b, stream)) != cudaSuccess)
           return e;
       }
     }
@@ -277,6 +274,20 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
         return e;
     }
     if (hooks.after_tree) hooks.after_tree(hooks.ctx, stream);
+    // Column sums: the float32 trees over up to 32 rows compute their own from the staged rows, the
+    // 16-bit forms in their normalising pass and the levels where they can; the rest read the
+    // input once more here.
+    {
+      SearchBatch cb;
+      cb.count = 0;
+      cb.maxN = 0;
+      for (int k = 0; k < m; ++k)
+        if (!summed[k]) {
+          cb.s[cb.count++] = b.s[k];
+          cb.maxN = std::max(cb.maxN, ss[k].N);
+        }
+      if ((e = column_sums_batch(cb, stream)) != cudaSuccess) return e;
+    }
     if ((e = search_stats_batch(b, num_sms, stream)) != cudaSuccess) return e;
     // The 16-bit searches: list the channels near the threshold, recompute them exactly
     // in FP32 from the original power.

@@ -139,6 +139,10 @@ struct TreeBatch {
   // paired-FP16 tree (two drift blocks per unit, FP16 sums; the precision form's flag bound
   // then takes FP16 adds).
   int pair16 = 0;
+  // Emitting launches: 1 runs all groups of a tile one after another on one CTA (group 0 first),
+  // so that the groups' column sums -- rows 16q .. 16q + 15 of group q -- add up in row order and
+  // the input needs no other read for them.  Every group has the same tiles and one chunk.
+  int tile_major = 0;
   TreeGroup g[kMaxBatch];
 };
 
@@ -305,10 +309,11 @@ long long level_stripe_bytes();  // the value set (negative: none)
 // every sub-problem, then the fused max kernel finishes them (see dd_levels.cu).
 // scratch_a / scratch_b: level_buffer_floats(Tr, N) floats each, in one allocation.
 // `input` holds elements of type `elem` (float, or the precision form's 16-bit copy, whose first
-// level converts on load).
+// level converts on load).  colsum (may be null): where the levels may form the column sums of
+// float rows on the way; *colsum_done says whether they do.
 cudaError_t levels_search(const void* input, long long row_stride, int Tr, int N, int dmin, int dmax,
                           float* scratch_a, float* scratch_b, float* top, int num_sms,
-                          cudaStream_t stream, int elem = kElemF32,
+                          cudaStream_t stream, float* colsum, bool* colsum_done, int elem = kElemF32,
                           int* status = nullptr);
 
 // A fully planned search for exec_queue: the request, its drift plan and its scratch.

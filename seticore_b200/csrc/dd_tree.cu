@@ -357,19 +357,23 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
   // Emitting form: lanes 0..PART-1 of each warp issue the bulk stores of its buffer.
   float* const ebuf = smem + warp * PART * W;
   bool stores_pending = false;
-  for (int item = blockIdx.x; item < tb.n_items; item += gridDim.x) {
+  __shared__ float csum[EMIT ? W : 1];  // tile-major launches: the tile's column sums so far
+  const int run = EMIT && tb.tile_major ? tb.count : 1;  // consecutive items a CTA takes
+  for (int item = blockIdx.x * run; item < tb.n_items;
+       item += item % run == run - 1 ? (int)(gridDim.x - 1) * run + 1 : 1) {
     __syncthreads();  // the previous item is finished with the tile, the layout and item_group
     // Warp 0 decodes the item and lays out the staged rows, one row per lane.
     if (warp == 0) {
       constexpr unsigned kAll = 0xffffffffu;
       int gi = 0;  // the last group whose first item is <= item
-      for (int base = 0; base < tb.count; base += 32) {
+      if (run > 1) gi = item % run;
+      for (int base = 0; base < (run > 1 ? 0 : tb.count); base += 32) {
         const int i = base + lane;
         const unsigned m = __ballot_sync(kAll, i < tb.count && tb.g[i].item_begin <= item);
         if (m) gi = base + 31 - __clz(m);
       }
       const TreeGroup& pg = tb.g[gi];
-      const int local = item - pg.item_begin;
+      const int local = run > 1 ? item / run : item - pg.item_begin;
       const int lt = local / pg.n_chunks;
       const int tile_i = lt + pg.tile_first;
       if (lane == 0) {
@@ -469,7 +473,7 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
     __syncthreads();
     const TreeGroup& p = tb.g[item_group];
     const E* rows = static_cast<const E*>(p.rows);
-    const int local = item - p.item_begin;
+    const int local = run > 1 ? item / run : item - p.item_begin;
     const int tile_idx = item_tile;
     const int chunk = local - (local / p.n_chunks) * p.n_chunks;
     const long long x0 = (long long)tile_idx * W;
@@ -572,6 +576,20 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
       return;
     }
 
+    if constexpr (EMIT) {
+      // Column sums across the groups of the tile, in row order: the zero-shear job's window of row
+      // t starts at channel x0.
+      if (run > 1 && p.colsum) {
+        const int gi = item_group;
+        for (int i = threadIdx.x; i < W; i += blockDim.x) {
+          float acc = gi == 0 ? 0.0f : csum[i];
+#pragma unroll
+          for (int t = 0; t < R; ++t) acc += tile[geo_win[0][t] + p.colsum_job * p.d_step * t + i];
+          csum[i] = acc;
+          if (gi == run - 1 && x0 + i < p.N) p.colsum[x0 + i] = acc;
+        }
+      }
+    }
     if constexpr (!EMIT && !PAIR) {
       // Column sums from the staged rows, in row order (bit-identical to sumColumns).
       // The zero-shear job's window of row t starts at channel x0, kz*d_step*t past the
@@ -835,7 +853,16 @@ cudaError_t launch_tree(TreeBatch& b, int num_sms, size_t smem_budget, cudaStrea
   b.stage_wait_tries = stage_wait_tries();
   // Enough warps for every (job, offset part) unit of a chunk, at most MAXW.
   const int warps = max_warps > MAXW ? MAXW : max_warps;
-  const int grid = (int)(n_items < slots ? n_items : slots);
+  long long runs = n_items;
+  if constexpr (EMIT) {
+    if (b.tile_major) {
+      for (int k = 0; k < b.count; ++k)  // the same tiles, whole chunks
+        if (b.g[k].n_tiles != b.g[0].n_tiles || b.g[k].tile_first != b.g[0].tile_first || b.g[k].n_chunks != 1)
+          return cudaErrorInvalidValue;
+      runs = n_items / b.count;
+    }
+  }
+  const int grid = (int)(runs < slots ? runs : slots);
   kern<<<grid, warps * kWarp, smem, stream>>>(b);
   return cudaGetLastError();
 }
