@@ -30,7 +30,7 @@
 // but the launches and last-block hand-overs between them: nine kernels took 92 us at 2^20
 // channels and 54 us at 32768, besides the gaps between them; the one takes 66 and 21 us (16
 // SMs; at 2^20 channels it is bound by instruction issue and by the cluster's 24 bytes per
-// clock and SM from L2).  64 searches of 2^20: 624 -> 453 us, the later reads served by L2.
+// clock and SM from L2).  64 searches of 2^20: 624 -> 402 us, the later reads served by L2.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -254,7 +254,11 @@ __device__ void pick_candidate(StatsShared& S, int j, int n, long long target_ra
 // [r, r + 1) * 16 * wl, its warp w the wl channels from (16 r + w) * wl.  C is at least 4 (the
 // three targets' candidates live in CTAs 0 to 2).  min_ties: a search whose most repeated order
 // statistic value has at least that many copies leaves the deviation to dd_order.cu.
-__global__ void __launch_bounds__(kSelThreads) stats_kernel(const __grid_constant__ SearchBatch b, int min_ties) {
+// MINB: CTAs per SM at least.  A few searches run fastest with all the registers (one CTA per SM:
+// 2^20 channels 76 us, 91 at 64 registers); more hide one another's barriers (64 searches 402 us
+// with two CTAs per SM, 451 with one; 8 of 999424 channels 107 and 131).
+template <int MINB>
+__global__ void __launch_bounds__(kSelThreads, MINB) stats_kernel(const __grid_constant__ SearchBatch b, int min_ties) {
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   StatsShared& S = *reinterpret_cast<StatsShared*>(dyn_smem);
   cg::cluster_group cl = cg::this_cluster();
@@ -687,8 +691,9 @@ cudaError_t column_sums_batch(const SearchBatch& b, cudaStream_t stream) {
 cudaError_t search_stats_emulated(const SearchBatch& b, int num_sms, int min_ties, cudaStream_t stream) {
   if (b.count <= 0) return cudaSuccess;
   const int smem = (int)sizeof(StatsShared);
-  cudaError_t e = cudaFuncSetAttribute(stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(stats_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  auto kern = b.count <= 4 ? stats_kernel<1> : stats_kernel<2>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   // Sixteen CTAs per search while they fit the SMs side by side, eight for larger batches, and
   // fewer for short rows, whose time is the barriers.
@@ -707,10 +712,10 @@ cudaError_t search_stats_emulated(const SearchBatch& b, int num_sms, int min_tie
     at[0].val.clusterDim.x = c;
     cfg.gridDim = dim3(c, b.count);
     int clusters = 0;
-    if (c <= 8 || (cudaOccupancyMaxActiveClusters(&clusters, stats_kernel, &cfg) == cudaSuccess && clusters > 0)) break;
+    if (c <= 8 || (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters > 0)) break;
     cudaGetLastError();  // sixteen CTAs do not fit one cluster here
   }
-  return cudaLaunchKernelEx(&cfg, stats_kernel, b, min_ties);
+  return cudaLaunchKernelEx(&cfg, kern, b, min_ties);
 }
 
 }  // namespace scb
