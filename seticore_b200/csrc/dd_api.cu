@@ -231,9 +231,7 @@ int ensure_prec(sc_dd* d, int slots) {
 }
 
 void free_inc(sc_dd* d) {
-  if (d->inc_index) cudaFreeHost(d->inc_index);
-  if (d->inc_steps) cudaFreeHost(d->inc_steps);
-  if (d->inc_vals) cudaFreeHost(d->inc_vals);
+  if (d->inc_index) cudaFreeHost(d->inc_index);  // one block holds the three arrays
   d->inc_index = d->inc_steps = nullptr;
   d->inc_vals = nullptr;
   d->inc_cap = 0;
@@ -293,12 +291,12 @@ int ensure_inc(sc_dd* d, int n) {
   free_inc(d);
   const int cap = std::max(n, 4096);
   cudaError_t e;
-  if ((e = cudaMallocHost(&d->inc_index, sizeof(int) * cap)) != cudaSuccess ||
-      (e = cudaMallocHost(&d->inc_steps, sizeof(int) * cap)) != cudaSuccess ||
-      (e = cudaMallocHost(&d->inc_vals, sizeof(float) * cap)) != cudaSuccess) {
-    free_inc(d);
+  if ((e = cudaMallocHost(&d->inc_index, (2 * sizeof(int) + sizeof(float)) * (size_t)cap)) != cudaSuccess) {
+    d->inc_index = nullptr;
     return cuda_fail(e, "incoherent staging allocation");
   }
+  d->inc_steps = d->inc_index + cap;
+  d->inc_vals = reinterpret_cast<float*>(d->inc_steps + cap);
   d->inc_cap = cap;
   return SC_DD_OK;
 }

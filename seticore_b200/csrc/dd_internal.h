@@ -208,8 +208,13 @@ inline size_t norm_buffer_bytes(int Tr, int N) {
   return dense > paired ? dense : paired;
 }
 
+// Small searches get at least kLevelMinFloats (32 MB) per buffer, so that one pass holds more of their
+// drift blocks (16 searches of 64 x 32768 on four pairs: 4 drift blocks 293 -> 263 us of levels,
+// 8 drift blocks 579 -> 489).
+constexpr size_t kLevelMinFloats = (size_t)8 << 20;
 inline size_t level_buffer_floats(int Tr, int N) {
-  return (size_t)Tr * (size_t)(level_row_length(N) + kLevelRowSlack);
+  const size_t n = (size_t)Tr * (size_t)(level_row_length(N) + kLevelRowSlack);
+  return n < kLevelMinFloats ? kLevelMinFloats : n;
 }
 
 // Precision form (dd_precision.cu), per search of a batch:
