@@ -48,18 +48,17 @@ UNIT = "Gsamples/s"
 # covering k coarse channels moves k times this.
 TREE_DRAM_BYTES = 78400384
 # Warp instructions the tree kernel executes per coarse channel of the node (ncu
-# smsp__inst_executed.sum of the same capture: 748.2 M for 4 coarse channels).
-TREE_WARP_INSTR = 748.2e6 / 4
+# smsp__inst_executed.sum of a launch over 4 coarse channels: 738.4 M).
+TREE_WARP_INSTR = 738.4e6 / 4
 # Level path of the beams workload, DRAM bytes per beam of 256 x 131072 (2 drift blocks, one
-# whole-row pass): the emitting first level 134.3 + 213.1 MB and the last level 269.5 + 3.9 MB
-# (ncu, one launch each, summarised with the level kernels' profile).
-BEAMS_DRAM_BYTES = 620.7e6
-# Kernels of one FP32 batch of up to 64 searches of 2^20 channels and at most 32 rows (the
-# launch list of one node step under ncu): clear, tree, range, three
-# histogram passes, compaction, order-statistic finish, two variance kernels, window, drift
-# recovery, and the exact statistics' launches, which exit at once when no search needs them
-# (reset, init, 15 partition rounds of three launches, two finishers, moments).
-LAUNCHES_PER_BATCH = 62
+# whole-row pass): the emitting first level, which also forms the column sums, 134.3 + 211.3 MB
+# and the last level 253.3 + 58.7 MB (ncu without cache control, beams searched one after
+# another, summarised with the level kernels' profile).
+BEAMS_DRAM_BYTES = 657.6e6
+# Kernels of one FP32 batch of up to 64 searches of 2^20 channels and at most 16 rows (the
+# launch list of one node step under ncu): clear, tree, statistics, exact statistics (which
+# exits at once when no search needs it), windows, drift recovery.
+LAUNCHES_PER_BATCH = 6
 
 
 def dist_setup():

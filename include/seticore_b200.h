@@ -187,8 +187,8 @@ int sc_dd_set_level_stripe_bytes(long long bytes);
  * variance sum moves the deviation by up to a few 1e-4 -- gets its statistics in the
  * reference's own std::nth_element order, bit-identical; the others emulate the float sum in
  * channel order (measured 2e-5 to 4e-5 relative on distinct-valued column sums, up to 3e-4
- * on heavy-tailed ones).  mode 1: every search takes the exact order (about 4 ms per batch of
- * 64 searches of 2^20 channels).  Process-wide; launches queued after the call follow it (a
+ * on heavy-tailed ones).  mode 1: every search takes the exact order (about 4.7 ms more per
+ * batch of 64 searches of 2^20 channels, 0.9 ms for one).  Process-wide; launches queued after the call follow it (a
  * CUDA graph keeps the mode it was captured with).  Other modes: SC_DD_EINVAL. */
 int sc_dd_set_exact_statistics(int mode);
 
@@ -282,7 +282,7 @@ const char* sc_dd_pool_last_error(void);
  * Same inputs, results and ordering as sc_dd_search, plus the shape (unrounded
  * num_timesteps, num_channels, foff in MHz, tsamp in s) that sc_dd_create would take.
  * It calls no cudaMalloc, cudaFree, cudaMallocHost or other allocating routine: its scratch
- * is one fixed device array inside the library (22.8 MB, held by every GPU that loads
+ * is one fixed device array inside the library (22.6 MB, held by every GPU that loads
  * the library until the process exits) and its host side uses the stack and `out`.
  * Limits (SC_DD_ELIMIT beyond them): num_channels <= SC_DD_STATIC_MAX_CHANNELS, rounded
  * timesteps <= 16, at most 65536 windows (num_channels / window_size).  A max_drift that is
