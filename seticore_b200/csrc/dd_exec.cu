@@ -183,8 +183,10 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
         tb.count = 0;
         tb.n_items = 0;
         tb.pair16 = (elem != kElemF32 && pair_rows(R) && pair_on) ? 1 : 0;
+        SearchHeader* first = nullptr;
         for (int k = 0; k < m; ++k) {
           if (ss[k].Tr != R || ss[k].elem != elem) continue;
+          if (!tb.count) first = b.s[k].hdr;
           if (elem == kElemF32) {
             TreeGroup g = tree_group(ss[k], ss[k].input, ss[k].row_stride, ss[k].top);
             if (tree_colsum(ss[k])) {
@@ -202,6 +204,7 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
             tb.g[tb.count++] = tree_group(ss[k], ss[k].norm16, ss[k].N, ss[k].top16);
           }
         }
+        if (tb.count && R <= 16) tb.next_item = &first->next_item;
         if (tb.count && (e = tree_max_batch(tb, R, num_sms, stream, elem, hooks.tree_launch(hooks.ctx, tb, R, elem))) !=
                             cudaSuccess)
           return e;

@@ -39,7 +39,7 @@ struct SearchHeader {
   int ties;         // most copies of one value among the three order statistics' values
   float median, std_dev, mean, threshold;
   unsigned ticket;  // CTAs of the drift recovery that are done (the last one writes the report)
-  int pad;
+  unsigned next_item;  // work counter of the tree launch whose first search this is
 };
 
 // Where the last kernel of a search leaves its results: host memory that the device can write
@@ -143,6 +143,9 @@ struct TreeBatch {
   // so that the groups' column sums -- rows 16q .. 16q + 15 of group q -- add up in row order and
   // the input needs no other read for them.  Every group has the same tiles and one chunk.
   int tile_major = 0;
+  // Device counter, zero before the launch and after it: CTAs take the items in order, one at a
+  // time, as they finish the last one.  Null: CTA c takes items c, c + grid, ...
+  unsigned* next_item = nullptr;
   TreeGroup g[kMaxBatch];
 };
 

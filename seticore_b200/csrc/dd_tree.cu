@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
   // (job_row_stride == 0) share one trapezoid segment; otherwise each job has its own.
   __shared__ int geo_base[kMaxSeg][R], geo_win[kMaxSeg][R], geo_wid[kMaxSeg][R];
   __shared__ long long geo_start[kMaxSeg][R];
-  __shared__ int item_group, item_tile;
+  __shared__ int item_group, item_tile, item_next;
   // Bulk-copied part of each staged row, as offsets [blo, bhi) from the row's start (float
   // rows only); the threads fill the rest.
   __shared__ int geo_blo[kMaxSeg][R], geo_bhi[kMaxSeg][R];
@@ -359,9 +359,19 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
   bool stores_pending = false;
   __shared__ float csum[EMIT ? W : 1];  // tile-major launches: the tile's column sums so far
   const int run = EMIT && tb.tile_major ? tb.count : 1;  // consecutive items a CTA takes
-  for (int item = blockIdx.x * run; item < tb.n_items;
-       item += item % run == run - 1 ? (int)(gridDim.x - 1) * run + 1 : 1) {
+  // Items are taken as CTAs finish: the SMs of a long launch drift apart by a few per cent (64
+  // searches of 16 x 2^20: 14.29 -> 13.69 ms; BF16, 32 of them: 5.02 -> 4.57).  Not for 32 rows, one
+  // CTA per SM (8 x 32 x 2^20: 3410 and 3425 us), nor for short strips, whose items are too short.
+  constexpr bool kTakes = !EMIT && R <= 16 && S == kStrip;
+  int item = blockIdx.x * run;
+  while (item < tb.n_items) {
     __syncthreads();  // the previous item is finished with the tile, the layout and item_group
+    // The item after this one, asked for by the last warp while warp 0 lays this one out.
+    if (kTakes && tb.next_item && threadIdx.x == blockDim.x - 1) {
+      const unsigned taken = atomicAdd(tb.next_item, 1u);
+      item_next = (int)(gridDim.x + taken);
+      if (taken == (unsigned)(tb.n_items - 1)) *tb.next_item = 0;  // one request an item: this is the launch's last
+    }
     // Warp 0 decodes the item and lays out the staged rows, one row per lane.
     if (warp == 0) {
       constexpr unsigned kAll = 0xffffffffu;
@@ -703,6 +713,8 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
         topS[i] = 0.0f;
       }
     }
+    if (kTakes && tb.next_item) item = item_next;
+    else item += item % run == run - 1 ? (int)(gridDim.x - 1) * run + 1 : 1;
   }
   if (EMIT && stores_pending) bulk_wait_all();  // the buffers stay valid until read
 }
@@ -739,6 +751,8 @@ cudaError_t launch_tree(TreeBatch& b, int num_sms, size_t smem_budget, cudaStrea
   // caller: host threads launching with different budgets cannot lower it under each other.
   err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn);
   if (err != cudaSuccess) return err;
+  // The items that take longest first, so that the last ones to be taken are short.
+  if (b.next_item) std::stable_sort(b.g, b.g + b.count, [](const TreeGroup& x, const TreeGroup& y) { return x.n_jobs > y.n_jobs; });
   size_t smem = 0;
   int max_warps = 1;
   long long n_items = 0;
