@@ -3,9 +3,10 @@
 // Used by the engine (dd_api.cu, one shape) and by the pool (dd_pool.cu, mixed shapes).
 // The searches travel in batches of up to kMaxBatch as kernel parameters, so a call is a
 // fixed sequence of launches (capturable in a CUDA graph) whatever the mix:
-//   clear -> [normalise] -> tree launches grouped by (rows, element type), the float32 ones
+//   clear -> [normalise] -> [one or two searches: column sums, statistics beside what follows] ->
+//   tree launches grouped by (rows, element type), the float32 ones
 //   adding the column sums -> levels for more than 32 rows, one search at a time -> column
-//   sums (searches whose trees did not compute them) -> statistics ->
+//   sums (searches whose trees did not compute them) -> statistics -> exact statistics ->
 //   [flag + FP32 recompute of the flagged channels] -> hits
 #include <algorithm>
 #include <cstddef>
@@ -95,6 +96,35 @@ PrecisionDesc to_pdesc(const ExecSearch& e, const SearchHeader* hdr, bool pair_o
 bool tree_colsum(const ExecSearch& e) { return e.elem == kElemF32 && e.Tr <= 32 && e.dmin <= 0 && e.dmax >= 0; }
 bool fused_colsum(const ExecSearch& e) { return tree_colsum(e) || e.elem != kElemF32; }
 
+// Whether the first level of a search of more than 32 float rows forms the column sums on the way.
+// They cost it its spread: a tile's row groups then run one after another on one CTA.  That pays
+// where tiles are many -- a dozen per SM for a search alone, two per SM beside others, whose launches
+// fill the gaps.  32 beams of 256 x 131072: 5.13 -> 4.95 ms (0.60 ms of their own launch before, 0.43
+// ms more in the levels); 4 of 64 x 2^20: 0.16 of 3.65 ms saved; but one by one, 256 x 131072 with 4
+// drift blocks 2.00 -> 2.27 ms of levels for 0.17 ms of sums.
+bool levels_sum_columns(const ExecSearch& q, bool alone, int num_sms) {
+  return q.N / 352 >= (alone ? 12ll : 2ll) * num_sms;
+}
+
+// Whether the column sums and the statistics of a batch run before its tree, which then starts while
+// the statistics are under way.  The statistics of a search are a chain of barriers on 16 SMs (20 us
+// at 32768 channels, 77 at 2^20) that leaves the others idle; beside the tree they cost it those SMs
+// for that long, and one more read of the input for the sums (12 us at 16 x 2^20, which the tree then
+// finds in L2).  Device time, after and before the tree: 16 x 2^20, 54 drift blocks 310 -> 268 us,
+// 14 drift blocks 167 -> 130; 16 x 32768 71 -> 52; 16 x 4096 63 -> 49; 32 x 2^20 546 -> 503; 64 x
+// 100003 272 -> 248; 256 x 131072, 2 drift blocks 702 -> 670.  Two searches gain as much (2 of
+// 16 x 2^20 555 -> 526); four, whose statistics take 64 SMs, no more than 2 % and lose as much at
+// some sizes (4 of 16 x 32768, 14 drift blocks 74 -> 75).  Not where the levels form the sums on the
+// way, nor for the 16-bit forms, whose sums come with the normalisation.
+bool statistics_first(const ExecSearch* s, int m, int num_sms) {
+  if (m > 2) return false;
+  if (s[0].Tr > 32)
+    return m == 1 && s[0].elem == kElemF32 && s[0].Tr <= 256 && !levels_sum_columns(s[0], true, num_sms);
+  for (int k = 0; k < m; ++k)
+    if (!tree_colsum(s[k]) || s[k].Tr != s[0].Tr) return false;
+  return true;
+}
+
 // The search's header word that a kernel sets when it gives up a wait.
 int* header_status(const ExecSearch& e) {
   return reinterpret_cast<int*>(reinterpret_cast<char*>(e.hdr) + offsetof(SearchHeader, error));
@@ -176,6 +206,11 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
       if (q.count && (e = normalize_batch(q, num_sms, stream)) != cudaSuccess) return e;
     }
     if (hooks.before_tree) hooks.before_tree(hooks.ctx, stream);
+    const bool stats_first = statistics_first(ss, m, num_sms);
+    const int min_ties = exact_statistics_ties();
+    if (stats_first && ((e = column_sums_batch(b, stream)) != cudaSuccess ||
+                        (e = search_stats_emulated(b, num_sms, min_ties, stream)) != cudaSuccess))
+      return e;
     // Trees over up to 32 rows: one launch per (rows, element type).
     for (int R : {2, 4, 8, 16, 32}) {
       for (int elem : {kElemF32, kElemBF16, kElemF16}) {
@@ -184,12 +219,13 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
         tb.n_items = 0;
         tb.pair16 = (elem != kElemF32 && pair_rows(R) && pair_on) ? 1 : 0;
         SearchHeader* first = nullptr;
+        tb.beside_previous = stats_first ? 1 : 0;
         for (int k = 0; k < m; ++k) {
           if (ss[k].Tr != R || ss[k].elem != elem) continue;
           if (!tb.count) first = b.s[k].hdr;
           if (elem == kElemF32) {
             TreeGroup g = tree_group(ss[k], ss[k].input, ss[k].row_stride, ss[k].top);
-            if (tree_colsum(ss[k])) {
+            if (tree_colsum(ss[k]) && !stats_first) {
               g.colsum = ss[k].colsum;
               g.colsum_job = -ss[k].dmin;
             }
@@ -231,19 +267,12 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
              std::min<long long>(ndb, 2 * half * pairs / per_db) * per_db * (long long)sizeof(float) >= (128ll << 20);
     };
     bool summed[kMaxBatch];
-    for (int k = 0; k < m; ++k) summed[k] = fused_colsum(ss[k]);
+    for (int k = 0; k < m; ++k) summed[k] = stats_first || fused_colsum(ss[k]);
     auto level = [&](int k, bool alone, float* la, float* lb, cudaStream_t st) {
       const ExecSearch& q = ss[k];
-      // Column sums on the way cost the first level its spread: a tile's row groups then run one
-      // after another on one CTA.  That pays where tiles are many -- a dozen per SM for a search
-      // alone, two per SM beside others, whose launches fill the gaps.  32 beams of 256 x 131072:
-      // 5.13 -> 4.95 ms (0.60 ms of their own launch before, 0.43 ms more in the levels); 4 of 64 x
-      // 2^20: 0.16 of 3.65 ms saved; but one by one, 256 x 131072 with 4 drift blocks 2.00 -> 2.27
-      // ms of levels for 0.17 ms of sums.
-      const long long tiles = q.N / 352;
-      float* colsum = tiles >= (alone ? 12ll : 2ll) * num_sms ? q.colsum : nullptr;
+      float* colsum = levels_sum_columns(q, alone, num_sms) ? q.colsum : nullptr;
       return levels_search(q.input, q.row_stride, q.Tr, q.N, q.dmin, q.dmax, la, lb, q.top, num_sms, st, colsum, &summed[k],
-                           kElemF32, header_status(q));
+                           kElemF32, header_status(q), &b.s[k].hdr->next_item, stats_first);
     };
     int n_level = 0;
     for (int k = 0; k < m; ++k) n_level += ss[k].Tr > 32 && ss[k].elem == kElemF32 && !wide(ss[k]);
@@ -277,9 +306,9 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
         return e;
     }
     if (hooks.after_tree) hooks.after_tree(hooks.ctx, stream);
-    // Column sums: the float32 trees over up to 32 rows compute their own from the staged rows, the
-    // 16-bit forms in their normalising pass and the levels where they can; the rest read the
-    // input once more here.
+    // Column sums where the statistics did not come first: the float32 trees over up to 32 rows compute
+    // their own from the staged rows, the 16-bit forms in their normalising pass and the levels where
+    // they can; the rest read the input once more here.
     {
       SearchBatch cb;
       cb.count = 0;
@@ -291,7 +320,8 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
         }
       if ((e = column_sums_batch(cb, stream)) != cudaSuccess) return e;
     }
-    if ((e = search_stats_batch(b, num_sms, stream)) != cudaSuccess) return e;
+    if (!stats_first && (e = search_stats_emulated(b, num_sms, min_ties, stream)) != cudaSuccess) return e;
+    if ((e = search_stats_exact(b, min_ties, stream)) != cudaSuccess) return e;
     // The 16-bit searches: list the channels near the threshold, recompute them exactly
     // in FP32 from the original power.
     {

@@ -146,6 +146,9 @@ struct TreeBatch {
   // Device counter, zero before the launch and after it: CTAs take the items in order, one at a
   // time, as they finish the last one.  Null: CTA c takes items c, c + grid, ...
   unsigned* next_item = nullptr;
+  // 1: the launch may start as soon as every CTA of the kernel before it runs (the statistics of a
+  // search whose column sums came first); it ends after that kernel.
+  int beside_previous = 0;
   TreeGroup g[kMaxBatch];
 };
 
@@ -261,6 +264,7 @@ cudaError_t column_sums_batch(const SearchBatch& b, cudaStream_t stream);
 // but, for the searches whose order statistics sit on repeated values (min_ties copies or
 // more), the deviation in the reference's own nth_element order, bit-identical (dd_order.cu).
 cudaError_t search_stats_batch(const SearchBatch& b, int num_sms, cudaStream_t stream);
+int exact_statistics_ties();  // min_ties of the two halves below
 cudaError_t search_stats_emulated(const SearchBatch& b, int num_sms, int min_ties, cudaStream_t stream);
 cudaError_t search_stats_exact(const SearchBatch& b, int min_ties, cudaStream_t stream);
 // The exact statistics run for a search whose three order statistics' values include one
@@ -318,11 +322,12 @@ long long level_stripe_bytes();  // the value set (negative: none)
 // scratch_a / scratch_b: level_buffer_floats(Tr, N) floats each, in one allocation.
 // `input` holds elements of type `elem` (float, or the precision form's 16-bit copy, whose first
 // level converts on load).  colsum (may be null): where the levels may form the column sums of
-// float rows on the way; *colsum_done says whether they do.
+// float rows on the way; *colsum_done says whether they do.  next_item, beside: TreeBatch's, for the
+// emitting first level (beside: its first pass).
 cudaError_t levels_search(const void* input, long long row_stride, int Tr, int N, int dmin, int dmax,
                           float* scratch_a, float* scratch_b, float* top, int num_sms,
                           cudaStream_t stream, float* colsum, bool* colsum_done, int elem = kElemF32,
-                          int* status = nullptr);
+                          int* status = nullptr, unsigned* next_item = nullptr, bool beside = false);
 
 // A fully planned search for exec_queue: the request, its drift plan and its scratch.
 struct ExecSearch {

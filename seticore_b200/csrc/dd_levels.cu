@@ -198,7 +198,7 @@ long long stripe_row_length(long long L, int nj, int fr) {
 // L2 budget, so the last level reads them from L2 and the next pass rewrites the same lines.
 cudaError_t stripe_pass(const float* input, long long row_stride, int Tr, int N, int d0, int nj,
                         long long x_b, long long x_e, long long Lp, float* buf, float* top, int nparts, int num_sms,
-                        cudaStream_t stream, float* colsum, int* status) {
+                        cudaStream_t stream, float* colsum, int* status, unsigned* next_item, bool beside) {
   const int fr = Tr / 16;
   const long long etile = kEmitTile;
   float* G = buf + 704 - x_b;
@@ -242,6 +242,8 @@ cudaError_t stripe_pass(const float* input, long long row_stride, int Tr, int N,
     g.colsum_job = -d0;
   }
   eb.tile_major = colsum ? 1 : 0;
+  eb.next_item = colsum ? nullptr : next_item;
+  eb.beside_previous = beside ? 1 : 0;
   cudaError_t err = tree_emit_batch(eb, num_sms, stream, 0, nparts);
   if (err != cudaSuccess) return err;
   TreeBatch tb;
@@ -275,7 +277,7 @@ cudaError_t stripe_pass(const float* input, long long row_stride, int Tr, int N,
 // the level buffers (`cap` floats).
 cudaError_t stripes_search(const float* input, long long row_stride, int Tr, int N, int dmin, int dmax,
                            float* buf, long long cap, float* top, int nparts, int num_sms, cudaStream_t stream,
-                           float* colsum, bool* colsum_done, int* status) {
+                           float* colsum, bool* colsum_done, int* status, unsigned* next_item, bool beside) {
   const int fr = Tr / 16;
   const int ndb = dmax - dmin + 1;
   // The whole row as one stripe (x_b = 0 suits every tile width, so any tile multiple will do).
@@ -343,7 +345,8 @@ cudaError_t stripes_search(const float* input, long long row_stride, int Tr, int
       // drift blocks are one chunk.
       const bool sums = colsum && L >= Nt && d0 <= 0 && d0 + nj > 0 && nj <= kColsumJobs;
       if ((err = stripe_pass(input, row_stride, Tr, N, d0, nj, x_b, x_e, Lp, buf, top, nparts, num_sms, stream,
-                             sums ? colsum : nullptr, status)) != cudaSuccess)
+                             sums ? colsum : nullptr, status, next_item, beside && d0 == dmin && x_b == 0)) !=
+          cudaSuccess)
         return err;
       if (sums) *colsum_done = true;
     }
@@ -369,7 +372,8 @@ long long level_stripe_bytes() { return g_stripe_bytes.load(); }
 
 cudaError_t levels_search(const void* input_v, long long row_stride, int Tr, int N, int dmin, int dmax,
                           float* scratch_a, float* scratch_b, float* top, int num_sms,
-                          cudaStream_t stream, float* colsum, bool* colsum_done, int elem, int* status) {
+                          cudaStream_t stream, float* colsum, bool* colsum_done, int elem, int* status, unsigned* next_item,
+                          bool beside) {
   int sizes[12];
   int nlev = 0;
   const float* input = static_cast<const float*>(input_v);
@@ -397,7 +401,7 @@ cudaError_t levels_search(const void* input_v, long long row_stride, int Tr, int
   cudaError_t err;
   if (nlev == 1 && (sizes[0] == kStreamEmit16 || sizes[0] == kStreamEmit16One))  // float rows (checked above)
     return stripes_search(input, row_stride, Tr, N, dmin, dmax, scratch_a, 2 * half, top,
-                          sizes[0] == kStreamEmit16One ? 1 : 2, num_sms, stream, colsum, colsum_done, status);
+                          sizes[0] == kStreamEmit16One ? 1 : 2, num_sms, stream, colsum, colsum_done, status, next_item, beside);
   if (nlev == 1 && (sizes[0] == 16 || sizes[0] == kStreamEmit16)) {
     // One level, then the last: the planes of up to J drift blocks per pair of launches.
     long long J = 2 * half / per_db;

@@ -1407,8 +1407,10 @@ std::atomic<bool> g_exact_always{false};
 void set_exact_statistics_always(bool always) { g_exact_always.store(always); }
 bool exact_statistics_always() { return g_exact_always.load(); }
 
+int exact_statistics_ties() { return exact_statistics_always() ? INT_MIN : kExactStatsTies; }
+
 cudaError_t search_stats_batch(const SearchBatch& b, int num_sms, cudaStream_t stream) {
-  const int min_ties = exact_statistics_always() ? INT_MIN : kExactStatsTies;
+  const int min_ties = exact_statistics_ties();
   cudaError_t e = search_stats_emulated(b, num_sms, min_ties, stream);
   if (e == cudaSuccess) e = search_stats_exact(b, min_ties, stream);
   return e;

@@ -270,6 +270,8 @@ __global__ void __launch_bounds__(kSelThreads, MINB) stats_kernel(const __grid_c
   const int wl = (int)((((long long)N + C * kSelWarps - 1) / (C * kSelWarps) + 7) & ~7ll);
   const int c0 = (int)min((long long)N, (long long)r * kSelWarps * wl);
   const int c1 = (int)min((long long)N, (long long)(r + 1) * kSelWarps * wl);
+  // The tree of a search whose column sums came first may run beside this (dd_exec.cu).
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   cl.sync();  // every CTA of the cluster runs: its shared memory may be written from here on
 
   // The key range.

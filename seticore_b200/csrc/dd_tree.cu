@@ -308,6 +308,9 @@ __device__ __forceinline__ void strip_part_h2(int part, const Row (&row)[R], flo
   }
 }
 
+// A launch that started beside the kernel before it (TreeBatch::beside_previous) ends after it.
+__device__ __forceinline__ void wait_previous_kernel() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // MAXW: warps per CTA at most; 8 / MAXW CTAs share an SM.
 // PAIR: the paired-FP16 tree over the paired copy (the rows are 32-bit words, staged like
 // float rows: word j of row t holds the FP16 pair (y[t][j], y[t][j + t]), the leaves of drift
@@ -362,7 +365,7 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
   // Items are taken as CTAs finish: the SMs of a long launch drift apart by a few per cent (64
   // searches of 16 x 2^20: 14.29 -> 13.69 ms; BF16, 32 of them: 5.02 -> 4.57).  Not for 32 rows, one
   // CTA per SM (8 x 32 x 2^20: 3410 and 3425 us), nor for short strips, whose items are too short.
-  constexpr bool kTakes = !EMIT && R <= 16 && S == kStrip;
+  constexpr bool kTakes = EMIT || (R <= 16 && S == kStrip);
   int item = blockIdx.x * run;
   while (item < tb.n_items) {
     __syncthreads();  // the previous item is finished with the tile, the layout and item_group
@@ -583,6 +586,7 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
       if (threadIdx.x == 0 && p.status) atomicExch(p.status, 1);
       if (item_tx) mbar_wait(&stage_bar, stage_phase ^ 1u);  // the copies may still be landing (full limit)
       if (EMIT && stores_pending) bulk_wait_all();
+      wait_previous_kernel();
       return;
     }
 
@@ -717,6 +721,7 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
     else item += item % run == run - 1 ? (int)(gridDim.x - 1) * run + 1 : 1;
   }
   if (EMIT && stores_pending) bulk_wait_all();  // the buffers stay valid until read
+  wait_previous_kernel();
 }
 
 template <typename E, int R, int NPARTS, int S, bool EMIT = false, int MAXW = 8>
@@ -877,6 +882,19 @@ cudaError_t launch_tree(TreeBatch& b, int num_sms, size_t smem_budget, cudaStrea
     }
   }
   const int grid = (int)(runs < slots ? runs : slots);
+  if (b.beside_previous) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(warps * kWarp);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, b);
+  }
   kern<<<grid, warps * kWarp, smem, stream>>>(b);
   return cudaGetLastError();
 }
