@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) tree_max_kernel(const __grid_
   __shared__ float csum[EMIT ? W : 1];  // tile-major launches: the tile's column sums so far
   const int run = EMIT && tb.tile_major ? tb.count : 1;  // consecutive items a CTA takes
   // Items are taken as CTAs finish: the SMs of a long launch drift apart by a few per cent (64
-  // searches of 16 x 2^20: 14.29 -> 13.69 ms; BF16, 32 of them: 5.02 -> 4.57).  Not for 32 rows, one
+  // searches of 16 x 2^20: 14.29 -> 13.69 ms; in the BF16 form, 32 of them, 4.89 -> 4.56).  Not for 32 rows, one
   // CTA per SM (8 x 32 x 2^20: 3410 and 3425 us), nor for short strips, whose items are too short.
   constexpr bool kTakes = EMIT || (R <= 16 && S == kStrip);
   int item = blockIdx.x * run;
