@@ -809,15 +809,17 @@ cudaError_t launch_tree(TreeBatch& b, int num_sms, size_t smem_budget, cudaStrea
   // (kStage, in strips of this row count), and one strip per round of its units over the CTA's
   // warps; the cut with the smallest estimate is taken.  16 rows, 54 drift blocks: 32768
   // channels (32 tiles) 148 -> 45 us, 2^20 channels (993 tiles on 296 slots) 324 -> 258 us;
-  // beyond a dozen rounds the last one is small change and whole chunks stage least (8 searches
-  // of 2^20 channels, 27 rounds: 1887 us either way).
+  // a launch of a dozen rounds or more whose CTAs take their items as they finish cuts its last round
+  // into quarters instead, so that it ends within a short item: 8 searches of 15 x 1033216, 27
+  // rounds, 2740 -> 2701 us a call.  With fixed shares whole chunks stage least.
   if constexpr (!EMIT) {
-    bool shared = n_items > 0 && n_items < 12 * slots;
+    const bool many = n_items >= 12 * slots;
+    bool shared = n_items > 0 && (!many || (b.next_item && R <= 16 && S == kStrip));  // kTakes
     for (int k = 0; k < b.count; ++k) shared = shared && b.g[k].job_row_stride == 0;
     if (shared) {
       constexpr int kLevels = R >= 32 ? 5 : R >= 16 ? 4 : R >= 8 ? 3 : R >= 4 ? 2 : 1;
       constexpr double kStage = 0.4 * 64.0 / (R * kLevels / NPARTS);
-      const long long rem = n_items % slots;
+      const long long rem = many ? slots : n_items % slots;
       // Tail groups: whole groups inside the last round, and the split rest of the one that
       // reaches into it.
       int first_tail = b.count;
@@ -847,7 +849,7 @@ cudaError_t launch_tree(TreeBatch& b, int num_sms, size_t smem_budget, cudaStrea
       int best = 0, max_jobs = 0;
       double best_time = 0.0;
       for (int k = first_tail; k < b.count; ++k) max_jobs = std::max(max_jobs, b.g[k].jobs_per_chunk);
-      for (int j = max_jobs; j >= 1; --j) {
+      for (int j = many ? 0 : max_jobs; j >= 1; --j) {
         long long items = 0;
         for (int k = first_tail; k < b.count; ++k) {
           const int jk = std::min(j, b.g[k].jobs_per_chunk);
@@ -860,6 +862,7 @@ cudaError_t launch_tree(TreeBatch& b, int num_sms, size_t smem_budget, cudaStrea
           best_time = t;
         }
       }
+      if (many) best = std::max(1, (max_jobs / 4 + MAXW - 1) / MAXW * MAXW);
       for (int k = first_tail; k < b.count; ++k)
         b.g[k].jobs_per_chunk = std::min(best, b.g[k].jobs_per_chunk);
       lay_out();

@@ -31,3 +31,24 @@ def test_counter_is_left_at_zero(port_oracle, case):
         np.testing.assert_array_equal(dd.channel_array("colsum").cpu().numpy(), arrays["colsum"])
         np.testing.assert_array_equal(dd.channel_array("top").cpu().numpy(), arrays["top"])
     dd.close()
+
+
+def test_last_round_in_quarters(port_oracle):
+    """A dozen rounds and more: the last round's drift blocks run in smaller chunks."""
+    if not has_gpu():
+        pytest.skip("no CUDA device")
+    import torch
+    from seticore_b200 import Dedopplerer
+    T, N, n, foff, tsamp, md = 16, 280 * 1056 + 5, 13, -2.7939677e-6, 18.253611, 4.0
+    dd = Dedopplerer(T, N, foff, tsamp)
+    x = np.random.default_rng(5).exponential(1.0, (T, N)).astype(np.float32)
+    _, _, arrays = port_oracle.search(x, foff, tsamp, md, 0.0, 5.0, arrays=True)
+    xt = torch.from_numpy(x).cuda()
+    key = lambda hits: [(h.index, h.drift_steps, h.power) for h in hits]
+    alone = key(dd.search_batch_raw([xt], [-1], [0], md, 0.0, 5.0)[0])
+    np.testing.assert_array_equal(dd.channel_array("top").cpu().numpy(), arrays["top"])
+    assert alone
+    for hits in dd.search_batch_raw([xt] * n, [-1] * n, list(range(n)), md, 0.0, 5.0):
+        assert key(hits) == alone
+    np.testing.assert_array_equal(dd.channel_array("top").cpu().numpy(), arrays["top"])
+    dd.close()
