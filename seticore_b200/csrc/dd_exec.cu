@@ -261,9 +261,17 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
     // searches each: 256 x 131072, 4 drift blocks 2195 -> 2007 us; 128 x 131072, 10 drift blocks
     // 2628 -> 2317; 4 of 64 x 2^20, 8 drift blocks 3948 -> 3482.  But 16 of 64 x 32768, 8 drift
     // blocks: 573 side by side and 618 one by one; 256 x 131072, 2 drift blocks: 1112 and 1202.
+    // More than 256 rows take one drift block at a time whatever the buffers hold, so there the
+    // planes of one drift block decide: from 48 MB on, the planes of searches side by side push one
+    // another's out of L2 between the levels.  Eight searches, 10 drift blocks, side by side and one by
+    // one: 2048 x 1024 (10 MB) 1.69 and 2.52 ms; 1024 x 8192 (35 MB) 3.99 and 4.30; 512 x 20480
+    // (43 MB) 5.06 and 4.86; 512 x 24576 (52 MB) 5.99 and 5.59; 512 x 131072 (277 MB) 31.2 and 25.8.  Not
+    // with two drift blocks: 1024 x 12288 1.30 and 1.35.
     auto wide = [&](const ExecSearch& q) {
-      const long long per_db = (long long)q.Tr * (level_row_length(q.N) + kLevelRowSlack), ndb = q.dmax - q.dmin + 1;
-      return pairs > 1 && ndb * per_db > 2 * half &&
+      const long long np = level_row_length(q.N), per_db = q.Tr * (np + kLevelRowSlack), ndb = q.dmax - q.dmin + 1;
+      if (pairs == 1) return false;
+      if (q.Tr > 256) return ndb > 2 && q.Tr * np * (long long)sizeof(float) >= (48ll << 20);
+      return ndb * per_db > 2 * half &&
              std::min<long long>(ndb, 2 * half * pairs / per_db) * per_db * (long long)sizeof(float) >= (128ll << 20);
     };
     bool summed[kMaxBatch];
