@@ -102,8 +102,11 @@ struct sc_dd {
   scb::SearchHeader* hdrs = nullptr;
   scb::Candidate* cands = nullptr;
   float* scratch_a = nullptr;  // Tr > 32 level buffers (one search at a time), one allocation
-  float* scratch_b = nullptr;  // = scratch_a + level_buffer_floats(Tr, N)
-  // The side streams' pairs (scratch_a + 2 + 2i and 3 + 2i level_buffer_floats, the same
+  float* scratch_b = nullptr;  // = scratch_a + level_floats
+  size_t level_floats = 0;     // per level buffer
+  size_t level_tried = 0;      // the largest size asked for so far
+  int level_asked = 0;         // calls that could use larger ones
+  // The side streams' pairs (scratch_a + 2 + 2i and 3 + 2i level_floats, the same
   // allocation) with their streams and events: a batch deals its level searches over them.
   scb::LevelSide side;
   int level_pairs = 1;  // pairs of level buffers in scratch_a
@@ -237,6 +240,41 @@ void free_inc(sc_dd* d) {
   d->inc_cap = 0;
 }
 
+// All pairs of level buffers lie in one allocation: the emitting level addresses a pair as one
+// array; pair 0 serves the main stream, pair 1 + i side stream i.
+size_t level_bytes(const sc_dd* d, size_t floats) { return 2 * (size_t)d->level_pairs * sizeof(float) * floats; }
+
+void set_levels(sc_dd* d, float* base, size_t floats) {
+  d->scratch_a = base;
+  d->scratch_b = base + floats;
+  d->level_floats = floats;
+  for (int i = 0; i + 1 < d->level_pairs; ++i) {
+    d->side.lvl_a[i] = base + (2 + 2 * i) * floats;
+    d->side.lvl_b[i] = base + (3 + 2 * i) * floats;
+  }
+}
+
+// Larger level buffers for calls of ndb drift blocks that can use them, from the sixteenth such call on:
+// the allocation, the release and a new graph cost about 1 ms, and a call gains 32 us (one search of
+// 64 x 1024, 20 drift blocks) to 90 us (16 of 64 x 32768, 8 drift blocks).  Where the memory is not there the search runs with what it
+// has, and the same size is not asked for again.
+constexpr int kLevelGrowCalls = 16;
+void grow_levels(sc_dd* d, int ndb) {
+  if (!d->scratch_a) return;
+  const size_t want = scb::level_buffer_want(d->Tr, d->N, ndb);
+  if (want <= d->level_floats || want <= d->level_tried || ++d->level_asked < kLevelGrowCalls) return;
+  d->level_tried = want;
+  float* base = nullptr;
+  if (dalloc(d, &base, level_bytes(d, want)) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  cudaDeviceSynchronize();  // the old buffers may still be in use by queued work
+  drop_graphs(d);
+  dfree(d, &d->scratch_a, level_bytes(d, d->level_floats));
+  set_levels(d, base, want);
+}
+
 void free_all(sc_dd* d) {
   drop_graphs(d);
   if (d->cap_stream) cudaStreamDestroy(d->cap_stream);
@@ -246,7 +284,7 @@ void free_all(sc_dd* d) {
   free_slots(d);
   free_prec(d);
   d->scratch_b = nullptr;  // inside scratch_a's allocation
-  dfree(d, &d->scratch_a, 2 * (size_t)d->level_pairs * sizeof(float) * scb::level_buffer_floats(d->Tr, d->N));
+  dfree(d, &d->scratch_a, level_bytes(d, d->level_floats));
   for (int i = 0; i < scb::kLevelSides; ++i) {
     if (d->side.stream[i]) cudaStreamDestroy(d->side.stream[i]);
     if (d->side.join[i]) cudaEventDestroy(d->side.join[i]);
@@ -447,6 +485,7 @@ int run_searches(sc_dd* dd, int count, const float* const* inputs, const long lo
   if (rc != SC_DD_OK) return rc;
   const bool prec = dd->precision != SC_DD_PRECISION_FP32;
   if (prec && (rc = ensure_prec(dd, std::min(count, scb::kMaxBatch))) != SC_DD_OK) return rc;
+  grow_levels(dd, p.dmax - p.dmin + 1);
   cudaError_t e;
   if ((e = cudaEventRecord(dd->ev[0], stream)) != cudaSuccess) return cuda_fail(e, "event");
   int total = 0;
@@ -595,21 +634,17 @@ int sc_dd_create(int num_timesteps, int num_channels, double foff_mhz, double ts
   // One slot; candidates for windows of 16 channels or more (grown when a call needs more).
   int rc = ensure_slots(d, 1, std::min(num_channels / 2 + 2, num_channels / 16 + 2));
   if (rc == SC_DD_OK && d->Tr > 32) {
-    // All pairs of level buffers in one allocation: the emitting level addresses a pair as
-    // one array; pair 0 serves the main stream, pair 1 + i side stream i.
     const size_t L = scb::level_buffer_floats(d->Tr, num_channels);
     const int sides = scb::level_sides(true);
     d->level_pairs = 1 + sides;
-    if ((e = dalloc(d, &d->scratch_a, 2 * (size_t)d->level_pairs * sizeof(float) * L)) != cudaSuccess) {
-      d->level_pairs = 1;
+    float* base = nullptr;
+    if ((e = dalloc(d, &base, level_bytes(d, L))) != cudaSuccess) {
       rc = fail(e == cudaErrorMemoryAllocation ? SC_DD_ENOMEM : SC_DD_ECUDA, "sc_dd_create: level buffers");
     } else {
-      d->scratch_b = d->scratch_a + L;
+      set_levels(d, base, L);
       if (sides > 0 && (e = cudaEventCreateWithFlags(&d->side.fork, cudaEventDisableTiming)) != cudaSuccess)
         rc = cuda_fail(e, "sc_dd_create: level stream");
       for (int i = 0; i < sides && rc == SC_DD_OK; ++i) {
-        d->side.lvl_a[i] = d->scratch_a + (2 + 2 * i) * L;
-        d->side.lvl_b[i] = d->scratch_a + (3 + 2 * i) * L;
         if ((e = cudaStreamCreateWithFlags(&d->side.stream[i], cudaStreamNonBlocking)) != cudaSuccess ||
             (e = cudaEventCreateWithFlags(&d->side.join[i], cudaEventDisableTiming)) != cudaSuccess)
           rc = cuda_fail(e, "sc_dd_create: level stream");

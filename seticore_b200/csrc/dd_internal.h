@@ -190,7 +190,7 @@ int tree_tile_width();
 
 // Row length of the level planes (N rounded up to whole tiles) and the floats one level
 // buffer holds for a search of Tr rounded timesteps: levels_search needs two such buffers
-// in one allocation (scratch_b = scratch_a + level_buffer_floats).
+// in one allocation (scratch_b = scratch_a + that many floats or more).
 inline long long level_row_length(int N) {
   const long long w = tree_tile_width();
   return (N + w - 1) / w * w;
@@ -214,14 +214,14 @@ inline size_t norm_buffer_bytes(int Tr, int N) {
   return dense > paired ? dense : paired;
 }
 
-// Small searches get at least kLevelMinFloats (32 MB) per buffer, so that one pass holds more of their
-// drift blocks (16 searches of 64 x 32768 on four pairs: 4 drift blocks 293 -> 263 us of levels,
-// 8 drift blocks 579 -> 489).
-constexpr size_t kLevelMinFloats = (size_t)8 << 20;
-inline size_t level_buffer_floats(int Tr, int N) {
-  const size_t n = (size_t)Tr * (size_t)(level_row_length(N) + kLevelRowSlack);
-  return n < kLevelMinFloats ? kLevelMinFloats : n;
-}
+inline size_t level_buffer_floats(int Tr, int N) { return (size_t)Tr * (size_t)(level_row_length(N) + kLevelRowSlack); }
+// The floats per level buffer that a search of ndb drift blocks can use: small searches of up to 256
+// rows take buffers of up to kLevelGrowFloats (32 MB), so that one pass holds more of their drift
+// blocks (16 searches of 64 x 32768 on four pairs: 4 drift blocks 293 -> 263 us of levels, 8 drift
+// blocks 579 -> 489).  Pools grow to it at the first call whose drift range can use it and engines
+// at the sixteenth, where the memory is there; any size from level_buffer_floats on serves every search.
+constexpr size_t kLevelGrowFloats = (size_t)8 << 20;
+size_t level_buffer_want(int Tr, int N, int ndb);
 
 // Precision form (dd_precision.cu), per search of a batch:
 struct PrecisionDesc {
@@ -319,7 +319,7 @@ long long level_stripe_bytes();  // the value set (negative: none)
 
 // Multi-level tree for Tr > 32 (one search): level kernels write the partial planes of
 // every sub-problem, then the fused max kernel finishes them (see dd_levels.cu).
-// scratch_a / scratch_b: level_buffer_floats(Tr, N) floats each, in one allocation.
+// scratch_a / scratch_b: level_buffer_floats(Tr, N) floats each or more, in one allocation.
 // `input` holds elements of type `elem` (float, or the precision form's 16-bit copy, whose first
 // level converts on load).  colsum (may be null): where the levels may form the column sums of
 // float rows on the way; *colsum_done says whether they do.  next_item, beside: TreeBatch's, for the
@@ -386,7 +386,7 @@ struct LevelSide {
 int level_sides(bool engine);
 
 // Queues every kernel of n searches (any mix) on `stream`; no synchronisation.
-// lvl_a / lvl_b: level buffers of level_buffer_floats(Tr, N) floats for every search with
+// lvl_a / lvl_b: level buffers of at least level_buffer_floats(Tr, N) floats for every search with
 // Tr > 32, in one allocation.  side: optional side streams for the level path.
 cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, int num_sms, cudaStream_t stream,
                        const ExecHooks& hooks, const LevelSide* side = nullptr);

@@ -367,6 +367,16 @@ int default_first_level() {
 
 }  // namespace
 
+size_t level_buffer_want(int Tr, int N, int ndb) {
+  const size_t n = level_buffer_floats(Tr, N);
+  if (Tr <= 32 || Tr > 256 || n >= kLevelGrowFloats) return n;  // more rows: one drift block at a time
+  // Half of what one whole-row pass of every drift block takes (a pass holds kMaxBatch at most).
+  const long long j = std::min(ndb, kMaxBatch), Nt = ((long long)N + 1055) / 1056 * 1056;
+  const long long row = std::max(Nt + stripe_row_length(0, (int)j, Tr / 16), level_row_length(N) + kLevelRowSlack);
+  const size_t half = ((size_t)(j * Tr * row) / 2 + 64) / 64 * 64;  // whole 256-byte lines
+  return std::max(n, std::min(half, kLevelGrowFloats));
+}
+
 void set_level_stripe_bytes(long long bytes) { g_stripe_bytes.store(bytes < 0 ? -1 : bytes); }
 long long level_stripe_bytes() { return g_stripe_bytes.load(); }
 

@@ -72,6 +72,7 @@ struct sc_dd_pool {
   float* lvl_a = nullptr;
   float* lvl_b = nullptr;
   size_t lvl_floats = 0;
+  size_t lvl_tried = 0;  // the largest size asked for so far
   scb::LevelSide side;  // side stream i's buffers: lvl_a + 2 + 2i and 3 + 2i lvl_floats
   char* host = nullptr;  // pinned: headers + candidate heads of the largest sub-batch
   size_t host_bytes = 0;
@@ -150,10 +151,12 @@ scb::TreeLaunch pool_tree_launch(void* ctx, const scb::TreeBatch& tb, int R, int
 // cudaMallocAsync): every earlier call of this pool has finished with them (a call
 // synchronises its stream before it returns), and work of other streams -- another pool's,
 // another server worker's -- is not waited for, as a device-wide synchronisation or a plain
-// cudaFree would.  Graphs captured over the old buffers are dropped.
-int ensure_device(sc_dd_pool* p, size_t arena, size_t lvl, cudaStream_t stream) {
+// cudaFree would.  Graphs captured over the old buffers are dropped.  lvl_min: floats per level
+// buffer that the searches need; lvl_want: that they can use, given where the memory is there.
+int ensure_device(sc_dd_pool* p, size_t arena, size_t lvl_min, size_t lvl_want, cudaStream_t stream) {
   cudaError_t e;
-  if (arena > p->arena_bytes || lvl > p->lvl_floats) {
+  const bool levels = lvl_min > p->lvl_floats || lvl_want > std::max(p->lvl_floats, p->lvl_tried);
+  if (arena > p->arena_bytes || levels) {
     for (auto& g : p->graphs) cudaGraphExecDestroy(g.exec);
     p->graphs.clear();
     p->seen.clear();
@@ -167,7 +170,9 @@ int ensure_device(sc_dd_pool* p, size_t arena, size_t lvl, cudaStream_t stream) 
     if ((e = cudaMemsetAsync(p->arena, 0, arena, stream)) != cudaSuccess) return pcuda(e, "pool arena memset");
     p->arena_bytes = arena;
   }
-  if (lvl > p->lvl_floats) {
+  if (levels) {
+    const size_t least = std::max(lvl_min, p->lvl_floats);
+    p->lvl_tried = std::max(p->lvl_tried, lvl_want);
     if (p->lvl_a) cudaFreeAsync(p->lvl_a, stream);
     p->lvl_a = p->lvl_b = nullptr;
     for (int i = 0; i < scb::kLevelSides; ++i) p->side.lvl_a[i] = p->side.lvl_b[i] = nullptr;
@@ -175,9 +180,14 @@ int ensure_device(sc_dd_pool* p, size_t arena, size_t lvl, cudaStream_t stream) 
     // All pairs of level buffers in one allocation: the emitting level addresses a pair as
     // one array; pair 0 serves the pool's stream, pair 1 + i side stream i.
     const size_t pairs = 1 + (size_t)p->side.n;
-    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&p->lvl_a), 2 * pairs * lvl * sizeof(float), stream)) !=
-        cudaSuccess)
-      return pfail(SC_DD_ENOMEM, std::string("pool level buffers: ") + cudaGetErrorString(e));
+    size_t lvl = std::max(least, lvl_want);
+    e = cudaMallocAsync(reinterpret_cast<void**>(&p->lvl_a), 2 * pairs * lvl * sizeof(float), stream);
+    if (e != cudaSuccess && lvl > least) {
+      cudaGetLastError();
+      lvl = least;
+      e = cudaMallocAsync(reinterpret_cast<void**>(&p->lvl_a), 2 * pairs * lvl * sizeof(float), stream);
+    }
+    if (e != cudaSuccess) return pfail(SC_DD_ENOMEM, std::string("pool level buffers: ") + cudaGetErrorString(e));
     p->lvl_b = p->lvl_a + lvl;
     for (int i = 0; i < p->side.n; ++i) {
       p->side.lvl_a[i] = p->lvl_a + (2 + 2 * i) * lvl;
@@ -339,7 +349,7 @@ int sc_dd_pool_search(sc_dd_pool* p, const sc_dd_request* reqs, int count, sc_dd
     pl.bytes = scb::ExecSearch::scratch_bytes(q.Tr, q.N, q.cand_cap, q.elem);
   }
   // Admission: consecutive requests while their scratch fits the budget (at least one).
-  size_t arena_need = 0, lvl_need = 0;
+  size_t arena_need = 0, lvl_min = 0, lvl_want = 0;
   std::vector<std::pair<int, int>> subs;
   {
     int i = 0;
@@ -355,9 +365,12 @@ int sc_dd_pool_search(sc_dd_pool* p, const sc_dd_request* reqs, int count, sc_dd
       i = j;
     }
     for (const Planned& pl : plans)
-      if (pl.es.Tr > 32) lvl_need = std::max(lvl_need, scb::level_buffer_floats(pl.es.Tr, pl.es.N));
+      if (pl.es.Tr > 32) {
+        lvl_min = std::max(lvl_min, scb::level_buffer_floats(pl.es.Tr, pl.es.N));
+        lvl_want = std::max(lvl_want, scb::level_buffer_want(pl.es.Tr, pl.es.N, pl.es.dmax - pl.es.dmin + 1));
+      }
   }
-  int rc = ensure_device(p, arena_need, lvl_need, stream);
+  int rc = ensure_device(p, arena_need, lvl_min, lvl_want, stream);
   if (rc != SC_DD_OK) return rc;
 
   cudaError_t e;
