@@ -258,7 +258,7 @@ def gather_hit_slices(input, num_timesteps: int, num_channels: int, bounds, stre
     n = len(bounds)
     if n == 0:
         return []
-    widths = [max(0, e - b) for b, e in bounds]
+    widths = [max(0, int(e) - int(b)) for b, e in bounds]  # Python's integers: T times the widths may pass 2^31
     total = num_timesteps * sum(widths)
     meta = torch.empty(2 * n, dtype=torch.int64, pin_memory=True)
     offs = meta[:n].numpy()
