@@ -60,7 +60,7 @@ typedef struct sc_dd_stats {
   int max_drift_block;
   int num_candidates; /* window maxima above threshold, before the min_drift filter */
   float tree_ms;      /* device time of the Taylor-tree kernel(s), CUDA events on the stream; of a call
-                           * with one or two searches also of the statistics that run beside them */
+                       * with one or two searches until the statistics that run beside them are done */
   float search_ms;    /* device time of the whole search, first memset to last kernel */
   int precision;          /* SC_DD_PRECISION_* of the search */
   int recomputed_channels; /* precision form: channels whose top was recomputed in FP32 */

@@ -205,12 +205,11 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
         }
       if (q.count && (e = normalize_batch(q, num_sms, stream)) != cudaSuccess) return e;
     }
-    if (hooks.before_tree) hooks.before_tree(hooks.ctx, stream);
     const bool stats_first = statistics_first(ss, m, num_sms);
     const int min_ties = exact_statistics_ties();
-    if (stats_first && ((e = column_sums_batch(b, stream)) != cudaSuccess ||
-                        (e = search_stats_emulated(b, num_sms, min_ties, stream)) != cudaSuccess))
-      return e;
+    if (stats_first && (e = column_sums_batch(b, stream)) != cudaSuccess) return e;
+    if (hooks.before_tree) hooks.before_tree(hooks.ctx, stream);
+    if (stats_first && (e = search_stats_emulated(b, num_sms, min_ties, stream)) != cudaSuccess) return e;
     // Trees over up to 32 rows: one launch per (rows, element type).
     for (int R : {2, 4, 8, 16, 32}) {
       for (int elem : {kElemF32, kElemBF16, kElemF16}) {
