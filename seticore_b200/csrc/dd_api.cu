@@ -634,7 +634,7 @@ int sc_dd_create(int num_timesteps, int num_channels, double foff_mhz, double ts
   // One slot; candidates for windows of 16 channels or more (grown when a call needs more).
   int rc = ensure_slots(d, 1, std::min(num_channels / 2 + 2, num_channels / 16 + 2));
   if (rc == SC_DD_OK && d->Tr > 32) {
-    const size_t L = scb::level_buffer_floats(d->Tr, num_channels);
+    const size_t L = scb::level_buffer_start(d->Tr, num_channels);
     const int sides = scb::level_sides(true);
     d->level_pairs = 1 + sides;
     float* base = nullptr;

@@ -215,12 +215,18 @@ inline size_t norm_buffer_bytes(int Tr, int N) {
 }
 
 inline size_t level_buffer_floats(int Tr, int N) { return (size_t)Tr * (size_t)(level_row_length(N) + kLevelRowSlack); }
-// The floats per level buffer that a search of ndb drift blocks can use: small searches of up to 256
-// rows take buffers of up to kLevelGrowFloats (32 MB), so that one pass holds more of their drift
-// blocks (16 searches of 64 x 32768 on four pairs: 4 drift blocks 293 -> 263 us of levels, 8 drift
-// blocks 579 -> 489).  Pools grow to it at the first call whose drift range can use it and engines
-// at the sixteenth, where the memory is there; any size from level_buffer_floats on serves every search.
+// Small searches of up to 256 rows take buffers of up to kLevelGrowFloats (32 MB), so that one pass
+// holds more of their drift blocks (16 searches of 64 x 32768 on four pairs: 4 drift blocks 293 -> 263
+// us of levels, 8 drift blocks 579 -> 489); any size from level_buffer_floats on serves every search.
+// An engine starts with room for four drift blocks a pass and grows to what its calls can use, a pool
+// asks for that at the call, where the memory is there.
 constexpr size_t kLevelGrowFloats = (size_t)8 << 20;
+inline size_t level_buffer_start(int Tr, int N) {
+  const size_t n = level_buffer_floats(Tr, N);
+  if (Tr > 256 || n >= kLevelGrowFloats) return n;
+  return 2 * n < kLevelGrowFloats ? 2 * n : kLevelGrowFloats;
+}
+// The floats per level buffer that a search of ndb drift blocks can use.
 size_t level_buffer_want(int Tr, int N, int ndb);
 
 // Precision form (dd_precision.cu), per search of a batch:

@@ -373,7 +373,7 @@ size_t level_buffer_want(int Tr, int N, int ndb) {
   // Half of what one whole-row pass of every drift block takes (a pass holds kMaxBatch at most).
   const long long j = std::min(ndb, kMaxBatch), Nt = ((long long)N + 1055) / 1056 * 1056;
   const long long row = std::max(Nt + stripe_row_length(0, (int)j, Tr / 16), level_row_length(N) + kLevelRowSlack);
-  const size_t half = ((size_t)(j * Tr * row) / 2 + 64) / 64 * 64;  // whole 256-byte lines
+  const size_t half = ((size_t)(j * Tr * row) / 2 + 63) / 64 * 64;  // whole 256-byte lines
   return std::max(n, std::min(half, kLevelGrowFloats));
 }
 

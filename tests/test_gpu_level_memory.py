@@ -24,8 +24,9 @@ def test_buffers_grow_with_the_drift_range(port_oracle, T, N):
     dd = Dedopplerer(T, N, foff * 1e-6, tsamp)
     row = (N + 1055) // 1056 * 1056 + 2048
     created = dd.memoryUsage()
-    # four pairs of Tr plane rows each, and less than a megabyte and a half of other scratch
-    assert created < 4 * 8 * Tr * row + (3 << 19)
+    # four pairs, each buffer of two drift blocks' plane rows (one above 256 rows), and less than a
+    # megabyte and a half of other scratch
+    assert created < 4 * 8 * (2 if Tr <= 256 else 1) * Tr * row + (3 << 19)
     used = []
     for nmax in (0.5, 9.5, 0.5):  # 2, 20 and 2 drift blocks
         md = nmax * foff / tsamp
