@@ -107,15 +107,16 @@ bool levels_sum_columns(const ExecSearch& q, bool alone, int num_sms) {
 }
 
 // Whether the column sums and the statistics of a batch run before its tree, which then starts while
-// the statistics are under way.  The statistics of a search are a chain of barriers on 16 SMs (20 us
-// at 32768 channels, 77 at 2^20) that leaves the others idle; beside the tree they cost it those SMs
+// the statistics are under way.  The statistics of a search are a chain of barriers on 16 SMs (25 us
+// at 32768 channels, 70 at 2^20) that leaves the others idle; beside the tree they cost it those SMs
 // for that long, and one more read of the input for the sums (12 us at 16 x 2^20, which the tree then
 // finds in L2).  Device time, after and before the tree: 16 x 2^20, 54 drift blocks 310 -> 268 us,
 // 14 drift blocks 167 -> 130; 16 x 32768 71 -> 52; 16 x 4096 63 -> 49; 32 x 2^20 546 -> 503; 64 x
 // 100003 272 -> 248; 256 x 131072, 2 drift blocks 702 -> 670.  Two searches gain as much (2 of
 // 16 x 2^20 555 -> 526); four, whose statistics take 64 SMs, no more than 2 % and lose as much at
 // some sizes (4 of 16 x 32768, 14 drift blocks 74 -> 75).  Not where the levels form the sums on the
-// way, nor for the 16-bit forms, whose sums come with the normalisation.
+// way.  The 16-bit forms, whose sums the normalising pass forms before the tree, have not been measured
+// this way.
 bool statistics_first(const ExecSearch* s, int m, int num_sms) {
   if (m > 2) return false;
   if (s[0].Tr > 32)
@@ -249,7 +250,9 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
     // searches are dealt round-robin over the main stream and the side streams, when there are
     // any (two concurrent 16-bit level searches measured slower than one after the other: their
     // first level is bound by L1 throughput, not by latency); the 16-bit searches run it on
-    // their normalised copy, with the default split, on the main stream.  A search that is alone,
+    // their normalised copy, with the default split, on the main stream, before the side streams
+    // start: beside the float searches there they were never faster (pools of 2 to 16 searches of 64
+    // to 2048 rows: -0.5 to 6 % slower).  A search that is alone,
     // or wide (below), runs on the main stream with every pair, which lie side by side: a search
     // of many drift blocks then needs a pass per eight of them, not per two (60 x 100003, 36
     // drift blocks: levels 0.68 -> 0.46 ms).

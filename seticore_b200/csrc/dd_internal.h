@@ -263,7 +263,8 @@ cudaError_t flag_channels_batch(const PrecisionBatch& b, int num_sms, cudaStream
 // original power in the tree's pairing, the maximum floored at 0.
 cudaError_t recompute_batch(const PrecisionBatch& b, int num_sms, cudaStream_t stream);
 
-// Column sums of each search (searches whose tree computes them skip this).
+// Column sums of each search, for those whose trees do not form them (searches of one or two, whose
+// statistics come first; levels of few tiles).
 cudaError_t column_sums_batch(const SearchBatch& b, cudaStream_t stream);
 // Order statistics, mean, standard deviation and threshold of each search, from its column
 // sums: the order statistics exactly and the float variance emulated in channel order (dd_stats.cu),

@@ -142,7 +142,7 @@ TreeGroup final_group(const float* src, long long Np, int N, int final_rows, int
 
 constexpr int kColsumJobs = 16;    // drift blocks of a tile that the emitting tree stages as one chunk, at most
 constexpr int kEmitTile = 352;     // channels per work item of the emitting tree
-constexpr int kStripeUnit = 5280;  // stripes start at multiples of every tree tile width (160, 352, 1056)
+constexpr int kStripeUnit = 5280;  // stripes start at multiples of both tree tile widths (352, 1056)
 
 // Bytes of planes one stripe pass may write: set_level_stripe_bytes, else
 // SETICORE_B200_LEVEL_L2_MB, else 0, which keeps whole rows (as many drift blocks per pass
@@ -412,7 +412,7 @@ cudaError_t levels_search(const void* input_v, long long row_stride, int Tr, int
   if (nlev == 1 && (sizes[0] == kStreamEmit16 || sizes[0] == kStreamEmit16One))  // float rows (checked above)
     return stripes_search(input, row_stride, Tr, N, dmin, dmax, scratch_a, 2 * half, top,
                           sizes[0] == kStreamEmit16One ? 1 : 2, num_sms, stream, colsum, colsum_done, status, next_item, beside);
-  if (nlev == 1 && (sizes[0] == 16 || sizes[0] == kStreamEmit16)) {
+  if (nlev == 1) {  // the four-channels-per-thread level
     // One level, then the last: the planes of up to J drift blocks per pair of launches.
     long long J = 2 * half / per_db;
     if (J > kMaxBatch) J = kMaxBatch;

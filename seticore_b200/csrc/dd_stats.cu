@@ -28,9 +28,9 @@
 //         leaves).
 // One launch, because what bounds the statistics of one search is not its four reads of 4 MB
 // but the launches and last-block hand-overs between them: nine kernels took 92 us at 2^20
-// channels and 54 us at 32768, besides the gaps between them; the one takes 66 and 21 us (16
+// channels and 54 us at 32768, besides the gaps between them; the one takes 70 and 25 us (16
 // SMs; at 2^20 channels it is bound by instruction issue and by the cluster's 24 bytes per
-// clock and SM from L2).  64 searches of 2^20: 624 -> 402 us, the later reads served by L2.
+// clock and SM from L2).  64 searches of 2^20: 624 -> 395 us, the later reads served by L2.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -255,8 +255,8 @@ __device__ void pick_candidate(StatsShared& S, int j, int n, long long target_ra
 // three targets' candidates live in CTAs 0 to 2).  min_ties: a search whose most repeated order
 // statistic value has at least that many copies leaves the deviation to dd_order.cu.
 // MINB: CTAs per SM at least.  A few searches run fastest with all the registers (one CTA per SM:
-// 2^20 channels 76 us, 91 at 64 registers); more hide one another's barriers (64 searches 402 us
-// with two CTAs per SM, 451 with one; 8 of 999424 channels 107 and 131).
+// 2^20 channels 91 us at 64 registers and 76 with all when the two were compared); more hide one
+// another's barriers (64 searches 402 us with two CTAs per SM, 451 with one; 8 of 999424 channels 107 and 131).
 template <int MINB>
 __global__ void __launch_bounds__(kSelThreads, MINB) stats_kernel(const __grid_constant__ SearchBatch b, int min_ties) {
   extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -445,8 +445,8 @@ __global__ void __launch_bounds__(kSelThreads, MINB) stats_kernel(const __grid_c
   double acc = 0.0, acc4[4] = {0.0, 0.0, 0.0, 0.0};
   // Targets with the same range share a list.  Nearly every warp read of 128 values holds a
   // candidate (about one value in a hundred is one), so the listing is branch-free: a predicated
-  // atomic per value whose result is waited for only by the predicated store.  As branches
-  // around atomics the pass took 44 thousand cycles for 65536 values per CTA, @@ this way.
+  // atomic per value whose result is waited for only by the predicated store, where branches
+  // around the atomics would wait for each in turn.
   const int list_of[3] = {0, t[1].lo == t[0].lo ? 0 : 1, t[2].lo == t[0].lo ? 0 : (t[2].lo == t[1].lo ? 1 : 2)};
   const uint32_t w1 = list_of[1] == 1 ? w[1] : 0u, w2 = list_of[2] == 2 ? w[2] : 0u;
   const unsigned count_a = static_cast<unsigned>(__cvta_generic_to_shared(&S.ncand[0]));
