@@ -58,6 +58,7 @@ constexpr int kSmemRange = 16384;        // ranges of at most this many values r
 constexpr int kSmemPairs = kSmemRange / 2 + 1;
 constexpr int kSerialRange = 256;        // ranges of at most this many values are finished by one thread
 constexpr int kOrderCluster = 16;        // CTAs per search, at most
+constexpr int kSideBySide16 = 7, kSideBySide8 = 15, kSideBySide4 = 33;  // clusters that run at once, by CTAs
 constexpr int kSumSeg = 4096;            // terms per speculative piece of the float sum
 constexpr int kSeqPrefix = 2048;         // leading terms of a sum added one by one (thread 0)
 constexpr int kTermsPerThreadF = 16;     // terms per thread in one scan chunk of a float sum
@@ -1188,11 +1189,8 @@ __device__ void cluster_steps(cg::cluster_group& cl, const SearchDesc& sd, Order
 // 2 to 5 us and 1.1 ms (partition steps 0.6 ms, bound by their barriers, the lists' scattered
 // stores and the leader's scans; the selections' last steps in shared memory 0.25 ms; the sums
 // 0.2 ms).
-__global__ void __launch_bounds__(kOrdThreads, 1)
-    order_kernel(const __grid_constant__ SearchBatch b, int min_ties) {
-  const SearchDesc& sd = b.s[blockIdx.y];
+__device__ __forceinline__ void order_search(const SearchDesc& sd) {
   const int N = sd.N;
-  if (N <= 0 || sd.hdr->ties < min_ties || *(volatile int*)&sd.hdr->error) return;  // every CTA of the cluster alike
   __shared__ OrdShared S;
   extern __shared__ __align__(16) float dyn[];
   cg::cluster_group cl = cg::this_cluster();
@@ -1369,6 +1367,20 @@ __global__ void __launch_bounds__(kOrdThreads, 1)
   }
 }
 
+// min_tied, max_tied: the launch acts where that many searches of the batch take the reference's order.
+// A second launch, which acts where this one does not, may start beside it and ends after it (its first
+// CTA waits; the others leave the SMs to the first launch and to other streams).
+__global__ void __launch_bounds__(kOrdThreads, 1)
+    order_kernel(const __grid_constant__ SearchBatch b, int min_ties, int min_tied, int max_tied) {
+  const SearchDesc& sd = b.s[blockIdx.y];
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  if (sd.N > 0 && sd.hdr->ties >= min_ties) {  // every CTA of the cluster alike, as the tests below
+    const int tied = __syncthreads_count((int)threadIdx.x < b.count && b.s[min((int)threadIdx.x, b.count - 1)].hdr->ties >= min_ties);
+    if (tied >= min_tied && tied <= max_tied && !*(volatile int*)&sd.hdr->error) order_search(sd);
+  }
+  if (blockIdx.x == 0 && blockIdx.y == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
 }  // namespace
 
 cudaError_t search_stats_exact(const SearchBatch& b, int min_ties, cudaStream_t stream) {
@@ -1379,26 +1391,45 @@ cudaError_t search_stats_exact(const SearchBatch& b, int min_ties, cudaStream_t 
   cudaError_t e = cudaFuncSetAttribute(order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(order_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
-  // Sixteen CTAs per search where a cluster of that many fits (16 SMs of one GPC) and the batch is
-  // small enough that the searches run side by side, else eight (64 searches that all leave at
-  // once: 8.6 and 5.0 us).
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
   cfg.blockDim = dim3(kOrdThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  for (int c = b.count <= 8 ? kOrderCluster : kOrderCluster / 2;; c /= 2) {
+  // A CTA fills an SM: 7 clusters of sixteen, 15 of eight, 33 of four and 74 of two run side by side.
+  // Sixteen CTAs per search while the batch fits so, and eight while it runs in two turns (64 searches
+  // that all leave at once: 8.6 and 5.0 us).  More searches of eight run in turns, most of whose SMs
+  // idle in the steps that one CTA does alone, so they take four or two CTAs each (64 searches of
+  // whole-number sums: N = 16384 1279 -> 439 us, 131072 2784 -> 1170, 2^20 7363 -> 5906; 33: 773 ->
+  // 379, 1680 -> 906, 4091 -> 3288).  Where only a few of a large batch take the order, eight are the
+  // faster from 131072 channels on (one of 64 searches of 2^20: 3.4 ms, with two 4.4): two launches then,
+  // of which the number that take it picks one; the other costs 1 to 3 us.
+  const bool all = min_ties == INT_MIN;  // every search takes the order
+  const int small = b.count <= kSideBySide4 ? 4 : 2;
+  int c = b.count <= kSideBySide16 ? 16 : 8, wide = kMaxBatch;
+  if (b.count > (all ? 1 : 2) * kSideBySide8) {
+    if (all || b.maxN <= 65536) c = small;
+    else wide = b.maxN >= (1 << 19) && small == 2 ? 2 * kSideBySide8 : kSideBySide8;
+  }
+  for (;; c /= 2) {
     at[0].val.clusterDim.x = c;
     cfg.gridDim = dim3(c, b.count);
     int clusters = 0;
     if (c <= 8 || (cudaOccupancyMaxActiveClusters(&clusters, order_kernel, &cfg) == cudaSuccess && clusters > 0)) break;
     cudaGetLastError();
   }
-  return cudaLaunchKernelEx(&cfg, order_kernel, b, min_ties);
+  e = cudaLaunchKernelEx(&cfg, order_kernel, b, min_ties, 1, wide);
+  if (e != cudaSuccess || wide == kMaxBatch) return e;
+  cfg.numAttrs = 2;
+  at[0].val.clusterDim.x = small;
+  cfg.gridDim = dim3(small, b.count);
+  return cudaLaunchKernelEx(&cfg, order_kernel, b, min_ties, wide + 1, kMaxBatch);
 }
 
 namespace {

@@ -1,0 +1,35 @@
+"""The statistics of a large batch of small searches run side by side: clusters small enough that one round
+of CTAs holds them.  Device times of a batch against a smaller one that fits a round whatever the cluster."""
+import statistics
+
+import pytest
+
+from tests.conftest import has_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def _search_ms(n, whole):
+    import torch
+    from seticore_b200 import Dedopplerer
+    T, N, foff = 8, 16384, 2.7939677
+    g = torch.Generator("cuda").manual_seed(n)
+    x = torch.empty((n, T, N), device="cuda").exponential_(generator=g)
+    if whole:  # many equal column sums: the statistics take the reference's own order
+        x = (x * 4).floor()
+    dd = Dedopplerer(T, N, foff * 1e-6, 18.25)
+    ms = []
+    for _ in range(30):
+        dd.search_batch_raw(list(x), [-1] * n, list(range(n)), 0.2, 0.0, 200.0)
+        ms.append(dd.last_stats().search_ms)
+    assert dd.last_stats().order_exact == int(whole)
+    dd.close()
+    return statistics.median(ms[10:])
+
+
+def test_exact_statistics_of_a_large_batch():
+    if not has_gpu():
+        pytest.skip("no CUDA device")
+    # 15 searches fill one round of clusters of eight.  64 take 1.2 times as long with clusters of two,
+    # and 3.4 times with eight.
+    assert _search_ms(64, True) < 2 * _search_ms(15, True)
