@@ -1367,18 +1367,26 @@ __device__ __forceinline__ void order_search(const SearchDesc& sd) {
   }
 }
 
-// min_tied, max_tied: the launch acts where that many searches of the batch take the reference's order.
-// A second launch, which acts where this one does not, may start beside it and ends after it (its first
-// CTA waits; the others leave the SMs to the first launch and to other streams).
+// CHOSEN: the launch acts only where min_tied to max_tied searches of the batch take the reference's
+// order.  A second launch, which acts where the first does not, may start beside it and ends after it
+// (its first CTA waits; the others leave the SMs to the first launch and to other streams).
+template <bool CHOSEN>
 __global__ void __launch_bounds__(kOrdThreads, 1)
     order_kernel(const __grid_constant__ SearchBatch b, int min_ties, int min_tied, int max_tied) {
   const SearchDesc& sd = b.s[blockIdx.y];
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  if (sd.N > 0 && sd.hdr->ties >= min_ties) {  // every CTA of the cluster alike, as the tests below
-    const int tied = __syncthreads_count((int)threadIdx.x < b.count && b.s[min((int)threadIdx.x, b.count - 1)].hdr->ties >= min_ties);
-    if (tied >= min_tied && tied <= max_tied && !*(volatile int*)&sd.hdr->error) order_search(sd);
+  if constexpr (CHOSEN) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  if (sd.N > 0 && sd.hdr->ties >= min_ties && !*(volatile int*)&sd.hdr->error) {  // every CTA of the cluster alike
+    bool act = true;
+    if constexpr (CHOSEN) {
+      const int k = min((int)threadIdx.x, b.count - 1);
+      const int tied = __syncthreads_count((int)threadIdx.x < b.count && b.s[k].hdr->ties >= min_ties);
+      act = tied >= min_tied && tied <= max_tied;
+    }
+    if (act) order_search(sd);
   }
-  if (blockIdx.x == 0 && blockIdx.y == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  if constexpr (CHOSEN) {
+    if (blockIdx.x == 0 && blockIdx.y == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  }
 }
 
 }  // namespace
@@ -1388,9 +1396,6 @@ cudaError_t search_stats_exact(const SearchBatch& b, int min_ties, cudaStream_t 
   const int smem = (int)(sizeof(float) * kSmemRange + sizeof(int) * 4 * kSmemPairs);
   static_assert(sizeof(float) * kSumBuf + 1024 * sizeof(SumPiece) <= sizeof(float) * kSmemRange + sizeof(int) * 4 * kSmemPairs,
                 "the sum's buffers fit the selection's");
-  cudaError_t e = cudaFuncSetAttribute(order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  if ((e = cudaFuncSetAttribute(order_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
@@ -1417,19 +1422,23 @@ cudaError_t search_stats_exact(const SearchBatch& b, int min_ties, cudaStream_t 
     if (all || b.maxN <= 65536) c = small;
     else wide = b.maxN >= (1 << 19) && small == 2 ? 2 * kSideBySide8 : kSideBySide8;
   }
+  auto kern = wide == kMaxBatch ? order_kernel<false> : order_kernel<true>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
   for (;; c /= 2) {
     at[0].val.clusterDim.x = c;
     cfg.gridDim = dim3(c, b.count);
     int clusters = 0;
-    if (c <= 8 || (cudaOccupancyMaxActiveClusters(&clusters, order_kernel, &cfg) == cudaSuccess && clusters > 0)) break;
+    if (c <= 8 || (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters > 0)) break;
     cudaGetLastError();
   }
-  e = cudaLaunchKernelEx(&cfg, order_kernel, b, min_ties, 1, wide);
+  e = cudaLaunchKernelEx(&cfg, kern, b, min_ties, 1, wide);
   if (e != cudaSuccess || wide == kMaxBatch) return e;
   cfg.numAttrs = 2;
   at[0].val.clusterDim.x = small;
   cfg.gridDim = dim3(small, b.count);
-  return cudaLaunchKernelEx(&cfg, order_kernel, b, min_ties, wide + 1, kMaxBatch);
+  return cudaLaunchKernelEx(&cfg, kern, b, min_ties, wide + 1, kMaxBatch);
 }
 
 namespace {

@@ -33,3 +33,30 @@ def test_exact_statistics_of_a_large_batch():
     # 15 searches fill one round of clusters of eight.  64 take 1.2 times as long with clusters of two,
     # and 3.4 times with eight.
     assert _search_ms(64, True) < 2 * _search_ms(15, True)
+
+
+@pytest.mark.parametrize("n,tied", [(33, 2), (33, 15), (33, 16), (40, 33), (64, 64), (64, 0), (20, 20)])
+def test_tied_searches_of_a_large_batch(n, tied):
+    """Few and many tied searches of a batch, by either launch: every search's hits, whose SNR holds the
+    deviation, are those of the search alone, launched, captured and replayed."""
+    if not has_gpu():
+        pytest.skip("no CUDA device")
+    import torch
+    from seticore_b200 import Dedopplerer
+    T, N, foff = 4, 70001, 2.7939677
+    g = torch.Generator("cuda").manual_seed(n + tied)
+    x = torch.empty((n, T, N), device="cuda").exponential_(generator=g)
+    pick = [k for k in range(n) if (k * 7) % n < tied]
+    assert len(pick) == tied
+    x[pick] = (x[pick] * 4).floor()
+    one, dd = (Dedopplerer(T, N, foff * 1e-6, 18.25) for _ in range(2))
+    key = lambda hits: [(h.index, h.drift_steps, h.power, h.snr) for h in hits]
+    want = []
+    for k in range(n):
+        want.append(key(one.search_raw(x[k], -1, 0, 0.4, 0.0, 3.0)))
+        assert one.last_stats().order_exact == int(k in pick)
+    assert all(want)
+    for _ in range(4):
+        assert [key(h) for h in dd.search_batch_raw(list(x), [-1] * n, list(range(n)), 0.4, 0.0, 3.0)] == want
+    one.close()
+    dd.close()
