@@ -698,8 +698,11 @@ cudaError_t search_stats_emulated(const SearchBatch& b, int num_sms, int min_tie
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   // Sixteen CTAs per search while they fit the SMs side by side, eight for larger batches, and
-  // fewer for short rows, whose time is the barriers.
-  int c = b.count * 16 <= num_sms ? 16 : 8;
+  // fewer for short rows, whose time is the barriers.  33 clusters of eight run at once (two CTAs per
+  // SM): more take four CTAs each instead of a second round, up to 65536 channels (37 searches of 16384
+  // 121 -> 88 us, 64 of 65536 256 -> 218, the tree included).  Beyond, a search of many equal values,
+  // whose histogram adds queue, holds the others up (one among 48 of 524288: 1.81 ms, with four 1.92).
+  int c = b.count * 16 <= num_sms ? 16 : (b.count <= 33 || b.maxN > 65536 ? 8 : 4);
   while (c > 4 && b.maxN <= c * 1024) c /= 2;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;

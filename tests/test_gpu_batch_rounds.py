@@ -35,6 +35,14 @@ def test_exact_statistics_of_a_large_batch():
     assert _search_ms(64, True) < 2 * _search_ms(15, True)
 
 
+def test_statistics_of_a_large_batch():
+    if not has_gpu():
+        pytest.skip("no CUDA device")
+    # 33 searches fill one round of clusters of eight.  37 take as long with clusters of four, and 1.38
+    # times as long with eight.
+    assert _search_ms(37, False) < 1.2 * _search_ms(33, False)
+
+
 @pytest.mark.parametrize("n,tied", [(33, 2), (33, 15), (33, 16), (40, 33), (64, 64), (64, 0), (20, 20)])
 def test_tied_searches_of_a_large_batch(n, tied):
     """Few and many tied searches of a batch, by either launch: every search's hits, whose SNR holds the
