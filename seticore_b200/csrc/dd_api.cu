@@ -106,7 +106,7 @@ struct sc_dd {
   float* scratch_b = nullptr;  // = scratch_a + level_floats
   size_t level_floats = 0;     // per level buffer
   size_t level_tried = 0;      // the largest size asked for so far
-  int level_asked = 0;         // calls that could use larger ones
+  double level_lost_us = 0;    // time that larger ones would have saved so far
   // The side streams' pairs (scratch_a + 2 + 2i and 3 + 2i level_floats, the same
   // allocation) with their streams and events: a batch deals its level searches over them.
   scb::LevelSide side;
@@ -255,15 +255,24 @@ void set_levels(sc_dd* d, float* base, size_t floats) {
   }
 }
 
-// Larger level buffers for calls of ndb drift blocks that can use them, from the sixteenth such call on:
-// the allocation, the release and a new graph cost about 1 ms, and a call gains 32 us (one search of
-// 64 x 1024, 20 drift blocks) to 90 us (16 of 64 x 32768, 8 drift blocks).  Where the memory is not there the search runs with what it
-// has, and the same size is not asked for again.
-constexpr int kLevelGrowCalls = 16;
-void grow_levels(sc_dd* d, int ndb) {
+// Larger level buffers for calls of n searches of ndb drift blocks that can use them, once the passes that
+// they would have saved (13 to 18 us each, one after another on a stream) cost 150 us: an engine that is
+// used that often is used on, and growing, about 1 ms for the allocation, the release and a new graph, is
+// more than a few searches gain.  40 searches of 64 x 1984 with 53 drift blocks in 16 bits grow at
+// the first call (4.96 -> 1.17 ms), one of 64 x 1024 with 20 at the tenth.  Where the memory is not there
+// the search runs with what it has, and the same size is not asked for again.
+constexpr double kLevelPassUs = 15.0, kLevelGrowUs = 150.0;
+void grow_levels(sc_dd* d, int n, int ndb) {
   if (!d->scratch_a) return;
   const size_t want = scb::level_buffer_want(d->Tr, d->N, ndb);
-  if (want <= d->level_floats || want <= d->level_tried || ++d->level_asked < kLevelGrowCalls) return;
+  if (want <= d->level_floats || want <= d->level_tried) return;
+  const bool f32 = d->precision == SC_DD_PRECISION_FP32;
+  const size_t room = 2 * (n == 1 && f32 ? (size_t)d->level_pairs : 1);  // buffers a pass has
+  const int elem = f32 ? scb::kElemF32 : scb::kElemBF16;
+  const int saved = scb::level_passes(d->Tr, d->N, ndb, room * d->level_floats, elem) -
+                    scb::level_passes(d->Tr, d->N, ndb, room * want, elem);
+  d->level_lost_us += kLevelPassUs * saved * (f32 ? (n + d->level_pairs - 1) / d->level_pairs : n);
+  if (d->level_lost_us < kLevelGrowUs) return;
   d->level_tried = want;
   float* base = nullptr;
   if (dalloc(d, &base, level_bytes(d, want)) != cudaSuccess) {
@@ -486,7 +495,7 @@ int run_searches(sc_dd* dd, int count, const float* const* inputs, const long lo
   if (rc != SC_DD_OK) return rc;
   const bool prec = dd->precision != SC_DD_PRECISION_FP32;
   if (prec && (rc = ensure_prec(dd, std::min(count, scb::kMaxBatch))) != SC_DD_OK) return rc;
-  grow_levels(dd, p.dmax - p.dmin + 1);
+  grow_levels(dd, count, p.dmax - p.dmin + 1);
   cudaError_t e;
   if ((e = cudaEventRecord(dd->ev[0], stream)) != cudaSuccess) return cuda_fail(e, "event");
   int total = 0;

@@ -226,8 +226,10 @@ inline size_t level_buffer_start(int Tr, int N) {
   if (Tr > 256 || n >= kLevelGrowFloats) return n;
   return 2 * n < kLevelGrowFloats ? 2 * n : kLevelGrowFloats;
 }
-// The floats per level buffer that a search of ndb drift blocks can use.
+// The floats per level buffer that a search of ndb drift blocks can use, and the whole-row passes that it
+// takes with `floats` of buffers (up to 256 rows).
 size_t level_buffer_want(int Tr, int N, int ndb);
+int level_passes(int Tr, int N, int ndb, size_t floats, int elem);
 
 // Precision form (dd_precision.cu), per search of a batch:
 struct PrecisionDesc {

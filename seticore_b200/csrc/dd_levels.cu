@@ -377,6 +377,13 @@ size_t level_buffer_want(int Tr, int N, int ndb) {
   return std::max(n, std::min(half, kLevelGrowFloats));
 }
 
+int level_passes(int Tr, int N, int ndb, size_t floats, int elem) {
+  const long long Nt = ((long long)N + 1055) / 1056 * 1056;
+  int j = std::min(ndb, kMaxBatch);
+  while (j > 1 && (size_t)(j * Tr * (elem == kElemF32 ? Nt + stripe_row_length(0, j, Tr / 16) : level_row_length(N))) > floats) --j;
+  return (ndb + j - 1) / j;
+}
+
 void set_level_stripe_bytes(long long bytes) { g_stripe_bytes.store(bytes < 0 ? -1 : bytes); }
 long long level_stripe_bytes() { return g_stripe_bytes.load(); }
 

@@ -1,5 +1,5 @@
 """Level buffers: an engine of more than 32 rows holds what its shape needs when it is created, and grows
-once sixteen calls had a drift range that can use more.  Tops and column sums are the oracle's bit for bit
+once calls whose drift range can use more keep coming.  Tops and column sums are the oracle's bit for bit
 before and after."""
 import numpy as np
 import pytest
@@ -28,7 +28,7 @@ def test_buffers_grow_with_the_drift_range(port_oracle, T, N):
     # megabyte and a half of other scratch
     assert created < 4 * 8 * (2 if Tr <= 256 else 1) * Tr * row + (3 << 19)
     used = []
-    for nmax in (0.5, 9.5, 0.5):  # 2, 20 and 2 drift blocks
+    for nmax in (0.5, 60.5, 0.5):  # 2, 122 and 2 drift blocks
         md = nmax * foff / tsamp
         _, _, want = port_oracle.search(x, foff * 1e-6, tsamp, md, 0.0, 5.0, arrays=True)
         for _ in range(19 if nmax > 1 else 3):  # launched, captured, replayed, and so again once the buffers grew
