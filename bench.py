@@ -56,9 +56,9 @@ TREE_WARP_INSTR = 738.4e6 / 4
 # another, summarised with the level kernels' profile).
 BEAMS_DRAM_BYTES = 657.6e6
 # Kernels of one FP32 batch of up to 64 searches of 2^20 channels and at most 16 rows (the
-# launch list of one node step under ncu): clear, tree, statistics, exact statistics (which
-# exits at once when no search needs it), windows, drift recovery.
-LAUNCHES_PER_BATCH = 6
+# launch list of one node step under ncu): clear, tree, statistics, exact statistics (two forms,
+# which exit at once when no search needs them), windows, drift recovery.
+LAUNCHES_PER_BATCH = 7
 
 
 def dist_setup():

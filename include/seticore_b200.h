@@ -188,7 +188,7 @@ int sc_dd_set_level_stripe_bytes(long long bytes);
  * variance sum moves the deviation by up to a few 1e-4 -- gets its statistics in the
  * reference's own std::nth_element order, bit-identical; the others emulate the float sum in
  * channel order (measured 2e-5 to 4e-5 relative on distinct-valued column sums, up to 3e-4
- * on heavy-tailed ones).  mode 1: every search takes the exact order (about 4.7 ms more per
+ * on heavy-tailed ones).  mode 1: every search takes the exact order (about 3.3 ms more per
  * batch of 64 searches of 2^20 channels, 0.9 ms for one).  Process-wide; launches queued after the call follow it (a
  * CUDA graph keeps the mode it was captured with).  Other modes: SC_DD_EINVAL. */
 int sc_dd_set_exact_statistics(int mode);
