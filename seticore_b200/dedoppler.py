@@ -241,7 +241,8 @@ def prepare_coarse_channels(buffers, num_timesteps: int, has_dc_spike: bool, str
 
 
 # Slices of up to this many floats together are written by the kernel straight into pinned host memory.
-_GATHER_PINNED_FLOATS = 1 << 20
+# Beyond, the copy engine is the faster way (100 slices of 2 x 5000: 414 us, pinned 460 to 640).
+_GATHER_PINNED_FLOATS = 1 << 18
 
 
 def gather_hit_slices(input, num_timesteps: int, num_channels: int, bounds, stream=None):
@@ -258,12 +259,12 @@ def gather_hit_slices(input, num_timesteps: int, num_channels: int, bounds, stre
     n = len(bounds)
     if n == 0:
         return []
-    widths = [max(0, int(e) - int(b)) for b, e in bounds]  # Python's integers: T times the widths may pass 2^31
-    total = num_timesteps * sum(widths)
+    widths = [max(0, e - b) for b, e in bounds]
     meta = torch.empty(2 * n, dtype=torch.int64, pin_memory=True)
     offs = meta[:n].numpy()
     offs[0] = 0
     np.cumsum([num_timesteps * w for w in widths[:-1]], out=offs[1:])
+    total = int(offs[-1]) + num_timesteps * int(widths[-1])  # in 64 bits whatever integers the bounds are
     meta[n:].numpy().view(np.int32)[:] = [v for b, e in bounds for v in (b, max(b, e))]
     pinned = total <= _GATHER_PINNED_FLOATS
     out = (torch.empty(max(1, total), dtype=torch.float32, pin_memory=True) if pinned
