@@ -74,14 +74,15 @@ __device__ __forceinline__ void gather_rows(const float* __restrict__ in, long l
   }
 }
 
-// A slice of 8 rows and 32 columns or more goes by rows, without the flat form's divisions (one slice of 8 x 100000: 422 us a call, flat 773).  Narrower slices and
-// fewer rows would leave lanes or warps idle and go to the host a few bytes at a time: flat (400
+// A slice of 8 rows and 32 columns or more goes by rows, without the flat form's divisions (one slice
+// of 8 x 100000: 422 us a call, flat 773).  Narrower slices and fewer rows would leave lanes or warps idle and go to the host a few bytes at a time: flat (400
 // slices of 256 x 1: 303 us, by rows 445; 100 of 8 x 1: 104 and 134).
 __global__ void gather_kernel(const float* __restrict__ in, long long row_stride, int T, const int* __restrict__ ranges,
                               const long long* __restrict__ offsets, float* __restrict__ out) {
   const int k = blockIdx.x;
   const int b = ranges[2 * k], w = ranges[2 * k + 1] - ranges[2 * k];
   float* o = out + offsets[k];
+  if (w <= 0) return;
   if (__builtin_expect(T < 8 || w < 32, 0)) {
     if ((long long)T * w < (1ll << 31) - 4096) gather_flat<unsigned>(in + b, row_stride, T, w, o);
     else gather_flat<unsigned long long>(in + b, row_stride, T, w, o);
