@@ -106,6 +106,28 @@ bool levels_sum_columns(const ExecSearch& q, bool alone, int num_sms) {
   return q.N / 352 >= (alone ? 12ll : 2ll) * num_sms;
 }
 
+// Whether a batch is one or two searches so long that the whole GPU forms their statistics (after the
+// tree) faster than a cluster each: from 2^22 channels on (one of 2^24, whose statistics a cluster forms in
+// 0.82 ms and the GPU in 0.18; at 3 * 2^20 the two are even).
+bool long_searches(const ExecSearch* s, int m) {
+  if (m > kWideStatsSearches) return false;
+  for (int k = 0; k < m; ++k)
+    if (s[k].N < kWideStatsChannels) return false;
+  return true;
+}
+
+// Whether the trees of long searches of up to 32 rows take long enough to hide a cluster's statistics beside
+// them: their work per channel, about Tr (log2 Tr + 3/4) for each drift block, against 50 us per 2^20
+// channels. One of 2^22 channels, statistics beside the tree and by the GPU after it: 16 x 6 drift
+// blocks 387 and 350 us, 16 x 10 393 and 436, 8 x 12 353 and 345, 8 x 26 404 and 451, 4 x 54 336 and 374.
+// The 32-row tree, one CTA per SM, gives up more for the cluster's SMs: 32 x 26 1745 and 1649, 54 3212
+// and 3186, two searches of 54 6143 and 6252.
+bool tree_hides_statistics(const ExecSearch* s, int m) {
+  long long work = 0;
+  for (int k = 0; k < m; ++k) work += (long long)(s[k].dmax - s[k].dmin + 1) * s[k].Tr * (4 * (31 - __builtin_clz(s[k].Tr)) + 3);
+  return work >= (s[0].Tr == 32 ? 73600 : 2360);  // 100 drift blocks of 32 rows; 7.8 of 16
+}
+
 // Whether the column sums and the statistics of a batch run before its tree, which then starts while
 // the statistics are under way.  The statistics of a search are a chain of barriers on 16 SMs (25 us
 // at 32768 channels, 70 at 2^20) that leaves the others idle; beside the tree they cost it those SMs
@@ -119,6 +141,7 @@ bool levels_sum_columns(const ExecSearch& q, bool alone, int num_sms) {
 // this way.
 bool statistics_first(const ExecSearch* s, int m, int num_sms) {
   if (m > 2) return false;
+  if (long_searches(s, m) && !tree_hides_statistics(s, m)) return false;
   if (s[0].Tr > 32)
     return m == 1 && s[0].elem == kElemF32 && s[0].Tr <= 256 && !levels_sum_columns(s[0], true, num_sms);
   for (int k = 0; k < m; ++k)
@@ -330,7 +353,9 @@ cudaError_t exec_queue(const ExecSearch* s, int n, float* lvl_a, float* lvl_b, i
         }
       if ((e = column_sums_batch(cb, stream)) != cudaSuccess) return e;
     }
-    if (!stats_first && (e = search_stats_emulated(b, num_sms, min_ties, stream)) != cudaSuccess) return e;
+    if (!stats_first && (e = long_searches(ss, m) ? search_stats_wide(b, num_sms, min_ties, stream)
+                                                   : search_stats_emulated(b, num_sms, min_ties, stream)) != cudaSuccess)
+      return e;
     if ((e = search_stats_exact(b, min_ties, stream)) != cudaSuccess) return e;
     // The 16-bit searches: list the channels near the threshold, recompute them exactly
     // in FP32 from the original power.

@@ -275,6 +275,10 @@ cudaError_t column_sums_batch(const SearchBatch& b, cudaStream_t stream);
 cudaError_t search_stats_batch(const SearchBatch& b, int num_sms, cudaStream_t stream);
 int exact_statistics_ties();  // min_ties of the two halves below
 cudaError_t search_stats_emulated(const SearchBatch& b, int num_sms, int min_ties, cudaStream_t stream);
+// The same by the whole GPU (dd_stats_wide.cu), for one or two searches of kWideStatsChannels or more.
+constexpr int kWideStatsChannels = 1 << 22;
+constexpr int kWideStatsSearches = 2;
+cudaError_t search_stats_wide(const SearchBatch& b, int num_sms, int min_ties, cudaStream_t stream);
 cudaError_t search_stats_exact(const SearchBatch& b, int min_ties, cudaStream_t stream);
 // The exact statistics run for a search whose three order statistics' values include one
 // held by at least this many column sums (automatic mode), or for every search.
